@@ -27,6 +27,7 @@
 
 #include "ptl_bpipe.h"
 #include "ptl_kernels.cuh"
+#include "ptl_steps.cuh"
 
 namespace ptl {
 namespace {
@@ -136,6 +137,7 @@ public:
     DBuf nt, rt, nd1, nd, par, ci, dep, loc0, loc, pos, decl, fflag, regs;
     DBuf fn_id, fn_start, fn_size, fn_end, fn_start0, fn_size0, ra_order, lifetime;
     DBuf instr, rd, rs1, rs2, jt, used_instrs, symreg, symswp, stamp, spill, roffs, owner, used, smark, defpos;
+    DBuf tmask, trow, tany;
     DBuf trig_min, trig_max, ra_chunks;
     DBuf ni, nrd, nr1, nr2, njt, joffs, out;
     DBuf errw, flags, meta, progs, tabs, lists, changed, sort_err, a_off, dirty, ra_sync;
@@ -169,7 +171,7 @@ public:
         return {&tab, &in_type, &in_rtype, &in_parent, &in_depth, &in_child, &in_data, &nt, &rt, &nd1, &nd, &par,
                 &ci, &dep, &loc0, &loc, &pos, &decl, &fflag, &regs, &fn_id, &fn_start, &fn_size,
                 &fn_end, &fn_start0, &fn_size0, &ra_order, &lifetime, &instr, &rd, &rs1, &rs2, &jt, &used_instrs, &symreg,
-                &symswp, &stamp, &spill, &roffs, &owner, &used, &smark, &defpos, &trig_min, &trig_max, &ra_chunks, &ni, &nrd,
+                &symswp, &stamp, &spill, &roffs, &owner, &used, &smark, &defpos, &tmask, &trow, &tany, &trig_min, &trig_max, &ra_chunks, &ni, &nrd,
                 &nr1, &nr2, &njt, &joffs, &out, &errw, &flags, &meta, &progs, &tabs, &lists, &changed,
                 &sort_err, &a_off, &dirty, &ra_sync, &sa, &sapos, &sbpos, &seg0, &seg1, &tile_seg, &tile_l, &tile_r,
                 &sort_stops, &leaf, &heap, &counters, &scan_status, &scan_counter, &sort_local, &sort_equal,
@@ -402,7 +404,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
     for (auto& x : hns) x = 0;
 
     // ---- small per-program state and the pinned small area
-    constexpr int kTables = 23, kLists = 4;  // table slots 0..22 are used
+    constexpr int kTables = 25, kLists = 5;  // table slots 0..24 are used
     small_progs_off = static_cast<size_t>(kTables) * (B + 1) * 4;
     small_meta_off = small_progs_off + B * sizeof(Prog);
     small_err_off = small_meta_off + B * 16;
@@ -700,6 +702,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
             P.spill = spill.at<uint32_t>(e);
             P.roffs = roffs.at<uint32_t>(e);
             P.owner = owner.at<unsigned long long>(e);
+            P.rec = P.owner;  // done with after isn_gen
             P.used = used.at<uint8_t>(e);
             P.smark = smark.at<uint8_t>(e);
             P.defpos = defpos.at<uint8_t>(e);
@@ -872,78 +875,140 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
         } else {
         const uint32_t t_f = tiles(6, F, elem_tile);
         batch_stage(BatchStage::InitLifetime, bl(6), t_f, nullptr);
-        Layout Lt, Lc;
-        Lt.build(trig, active);
-        std::vector<uint64_t> chunk_words(B);
-        for (size_t p = 0; p < B; ++p) chunk_words[p] = 2 * (S[p] / 32 + 2);
-        Lc.build(chunk_words, active);
-        BP_CU(trig_min.ensure(Lt.total * 4));
-        BP_CU(trig_max.ensure(Lt.total * 4));
-        BP_CU(cudaMemsetAsync(trig_min.p, 0xFF, Lt.total * 4, s));
-        BP_CU(cudaMemsetAsync(trig_max.p, 0, Lt.total * 4, s));
-        BP_CU(family(Lc, {&ra_chunks}, 4));
-        for (size_t p = 0; p < B; ++p) {
-            hp[p].trig_min = trig_min.at<uint32_t>(Lt.elem(p));
-            hp[p].trig_max = trig_max.at<uint32_t>(Lt.elem(p));
-            hp[p].ra_chunks = ra_chunks.at<uint32_t>(Lc.elem(p));
-        }
-        upload_progs();
         const uint32_t t_w = tiles(7, W, elem_tile);
-        batch_stage(BatchStage::Cross, bl(7), t_w, nullptr);
+        batch_stage(BatchStage::Records, bl(7), t_w, nullptr);
         BP_CU(cudaMemcpyAsync(hfl, flags.p, B * 16, cudaMemcpyDeviceToHost, s));
         BP_CU(collect_errors());
-        std::vector<uint32_t> lane0_list, serial_list, wide_list;
-        std::vector<uint8_t> lane0(B, 0);
+        // every program takes the record form, except one whose words a record cannot say
+        // (the general form) or whose functions share symbols (the serial order)
+        std::vector<uint32_t> step_list, wide_steps, lane0_list, serial_list, wide_list;
+        std::vector<uint8_t> steps(B, 0), general(B, 0), lane0(B, 0);
         std::vector<uint64_t> nfree(B, 0);
-        uint32_t max_g0 = 1;
+        uint32_t max_g0 = 1, max_step_g0 = 1;
         for (size_t p = 0; p < B; ++p) {
             if (!active[p]) continue;
             active_list.push_back(static_cast<uint32_t>(p));
             const uint64_t g0 = (F[p] + 7) / 8;
-            if (hfl[4 * p + 1] || g0 > 8192) {  // functions share symbols: the serial order
-                serial_list.push_back(static_cast<uint32_t>(p));
-                continue;
-            }
-            if (hfl[4 * p + 2]) hp[p].defpos = nullptr;  // a register with two definitions: hash row 0
-            if (g0 > kRaClusterMin && ra_cluster_fits(static_cast<uint32_t>(g0))) {
-                wide_list.push_back(static_cast<uint32_t>(p));  // its own launches, on a cluster
-                continue;
-            }
-            lane0[p] = 1;
-            lane0_list.push_back(static_cast<uint32_t>(p));
             nfree[p] = F[p] - g0;
-            max_g0 = std::max<uint32_t>(max_g0, static_cast<uint32_t>(g0));
+            if (hfl[4 * p + 1] || g0 > 8192) {
+                serial_list.push_back(static_cast<uint32_t>(p));
+            } else if (!hfl[4 * p + 2] && (g0 <= kStepBlockMax ||
+                                           (!ra_cluster_disabled() && step_cluster_fits(static_cast<uint32_t>(g0))))) {
+                steps[p] = 1;
+                if (g0 > kStepBlockMax) {
+                    wide_steps.push_back(static_cast<uint32_t>(p));  // its own launches, on a cluster
+                } else {
+                    step_list.push_back(static_cast<uint32_t>(p));
+                    max_step_g0 = std::max<uint32_t>(max_step_g0, static_cast<uint32_t>(g0));
+                }
+            } else {
+                general[p] = 1;
+                hp[p].defpos = nullptr;
+                if (g0 > kRaClusterMin && ra_cluster_fits(static_cast<uint32_t>(g0))) {
+                    wide_list.push_back(static_cast<uint32_t>(p));  // its own launches, on a cluster
+                } else {
+                    lane0[p] = 1;
+                    lane0_list.push_back(static_cast<uint32_t>(p));
+                    max_g0 = std::max<uint32_t>(max_g0, static_cast<uint32_t>(g0));
+                }
+            }
+        }
+        auto longest_first = [&](uint32_t x, uint32_t y) { return S[x] > S[y]; };
+        std::stable_sort(step_list.begin(), step_list.end(), longest_first);
+        if (step_list.size() + wide_steps.size() > 0) {
+            std::vector<uint64_t> rows(B), any(B), masks(B);
+            for (size_t p = 0; p < B; ++p) {
+                if (!steps[p]) continue;
+                any[p] = row_tiles(S[p]) * kRowTile;
+                rows[p] = any[p] * kRowPos;
+                masks[p] = wb8[p];
+            }
+            Layout Lm, Lr, La;
+            Lm.build(masks, steps);
+            Lr.build(rows, steps);
+            La.build(any, steps);
+            BP_CU(tmask.ensure(Lm.total * 4));
+            BP_CU(trow.ensure(Lr.total * 4));
+            BP_CU(tany.ensure(La.total * 4));
+            for (size_t p = 0; p < B; ++p) {
+                if (!steps[p]) continue;
+                hp[p].tmask = tmask.at<uint32_t>(Lm.elem(p));
+                hp[p].trow = trow.at<uint32_t>(Lr.elem(p));
+                hp[p].tany = tany.at<uint32_t>(La.elem(p));
+            }
+        }
+        if (lane0_list.size() + wide_list.size() > 0) {
+            std::vector<uint64_t> chunk_words(B);
+            for (size_t p = 0; p < B; ++p) chunk_words[p] = 2 * (S[p] / 32 + 2);
+            Layout Lt, Lc;
+            Lt.build(trig, general);
+            Lc.build(chunk_words, general);
+            BP_CU(trig_min.ensure(Lt.total * 4));
+            BP_CU(trig_max.ensure(Lt.total * 4));
+            BP_CU(cudaMemsetAsync(trig_min.p, 0xFF, Lt.total * 4, s));
+            BP_CU(cudaMemsetAsync(trig_max.p, 0, Lt.total * 4, s));
+            BP_CU(family(Lc, {&ra_chunks}, 4));
+            for (size_t p = 0; p < B; ++p) {
+                if (!general[p]) continue;
+                hp[p].trig_min = trig_min.at<uint32_t>(Lt.elem(p));
+                hp[p].trig_max = trig_max.at<uint32_t>(Lt.elem(p));
+                hp[p].ra_chunks = ra_chunks.at<uint32_t>(Lc.elem(p));
+            }
         }
         upload_progs();
-        // independent functions and lane-0 passes of all programs in one persistent launch,
-        // longest programs (most steps) first
-        std::stable_sort(lane0_list.begin(), lane0_list.end(), [&](uint32_t x, uint32_t y) { return S[x] > S[y]; });
-        const uint32_t ra_T = batch_ra_threads(max_g0);
-        uint32_t ra_items = 0;  // per program: its independent-function tiles, then its lane-0 pass
-        {
-            uint32_t* h = table_slot(8);
+        if (!step_list.empty()) {  // blocks of program order[k], longest program first
+            uint32_t* hf = table_slot(8);
+            uint32_t* hr = table_slot(23);
+            uint32_t nf = 0, nr = 0;
+            for (size_t k = 0; k < step_list.size(); ++k) {
+                hf[k] = nf;
+                hr[k] = nr;
+                nf += static_cast<uint32_t>((nfree[step_list[k]] + 31) / 32);
+                nr += static_cast<uint32_t>(row_tiles(S[step_list[k]]));
+            }
+            for (size_t k = step_list.size(); k <= B; ++k) {
+                hf[k] = nf;
+                hr[k] = nr;
+            }
+            BP_CU(cudaMemcpyAsync(dtable_slot(8), hf, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+            BP_CU(cudaMemcpyAsync(dtable_slot(23), hr, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+            const uint32_t* d_steps = upload_list(0, step_list);
+            const uint32_t count = static_cast<uint32_t>(step_list.size());
+            batch_free_order(progs.at<Prog>(), d_steps, count, s);
+            BP_CU(batch_step_regalloc(StepBatch{progs.at<Prog>(), d_steps, dtable_slot(8), dtable_slot(23), count, nf, nr,
+                                                max_step_g0}, s));
+        }
+        if (!lane0_list.empty()) {
+            // independent functions and lane-0 passes in one persistent launch
+            std::stable_sort(lane0_list.begin(), lane0_list.end(), longest_first);
+            const uint32_t ra_T = batch_ra_threads(max_g0);
+            uint32_t ra_items = 0;  // per program: its independent-function tiles, then its lane-0 pass
+            uint32_t* h = table_slot(24);
             for (size_t k = 0; k < lane0_list.size(); ++k) {
                 h[k] = ra_items;
                 ra_items += static_cast<uint32_t>((nfree[lane0_list[k]] + ra_T - 1) / ra_T) + 1u;
             }
             for (size_t k = lane0_list.size(); k <= B; ++k) h[k] = ra_items;
-            BP_CU(cudaMemcpyAsync(dtable_slot(8), h, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+            BP_CU(cudaMemcpyAsync(dtable_slot(24), h, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+            const uint32_t* d_lane0 = upload_list(4, lane0_list);
+            batch_free_order(progs.at<Prog>(), d_lane0, static_cast<uint32_t>(lane0_list.size()), s);
+            BP_CU(ra_sync.ensure(64));
+            // per program: histogram of the independent functions' last chunks, then counts
+            const uint32_t t_hist = tiles(16, nfree, elem_tile, &lane0);
+            batch_stage(BatchStage::RaHist, bl(16), t_hist, nullptr);
+            BP_CU(batch_regalloc(progs.at<Prog>(), dtable_slot(24), d_lane0, static_cast<uint32_t>(lane0_list.size()),
+                                 ra_items, max_g0, ra_sync.at<uint32_t>(), s, ra_share));
         }
-        const uint32_t* d_lane0 = upload_list(0, lane0_list);
-        batch_free_order(progs.at<Prog>(), d_lane0, static_cast<uint32_t>(lane0_list.size()), s);
-        BP_CU(ra_sync.ensure(64));
-        // per program: histogram of the independent functions' last chunks, then counts
-        const uint32_t t_hist = tiles(16, nfree, elem_tile, &lane0);
-        batch_stage(BatchStage::RaHist, bl(16), t_hist, nullptr);
-        BP_CU(batch_regalloc(progs.at<Prog>(), dtable_slot(8), d_lane0, static_cast<uint32_t>(lane0_list.size()),
-                             ra_items, max_g0, ra_sync.at<uint32_t>(), s, ra_share));
+        for (const uint32_t p : wide_steps) {
+            Prog one = hp[p];
+            one.ra_order = nullptr;
+            BP_CU(run_step_regalloc(one, s));
+        }
         const uint32_t* d_serial = upload_list(1, serial_list);
         batch_serial(progs.at<Prog>(), d_serial, static_cast<uint32_t>(serial_list.size()), s);
         for (const uint32_t p : wide_list) {
-            Prog Pfree = hp[p];
-            Pfree.defpos = nullptr;  // the independent functions never need definition positions
             bool launched = false;
-            BP_CU(launch_ra_wide(hp[p], Pfree, static_cast<uint32_t>((F[p] + 7) / 8), s, &launched));
+            BP_CU(launch_ra_wide(hp[p], hp[p], static_cast<uint32_t>((F[p] + 7) / 8), s, &launched));
             if (!launched) return cuda_fail(cudaErrorLaunchFailure, "lane-0 cluster pass");
         }
         }  // the AVX generator's allocation

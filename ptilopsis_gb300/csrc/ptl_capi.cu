@@ -16,6 +16,7 @@
 
 #include "../../include/ptl_codegen.h"
 #include "ptl_kernels.cuh"
+#include "ptl_steps.cuh"
 
 namespace ptl {
 namespace {
@@ -94,6 +95,7 @@ struct ptl_generator {
     DevBuf decl, fn_id, fn_start, fn_size, fn_end, fn_start0, fn_size0, fn_end0;
     DevBuf fn_ra_start, fn_ra_end, fn_ra_size;
     DevBuf instr, rd, rs1, rs2, jt, owner, used, smark, used_instrs;
+    DevBuf tmask, trow, tany;
     DevBuf symreg, symswp, stamp, defpos, lifetime, trig_min, trig_max, ra_chunks, spill, roffs;
     DevBuf ni, nrd, nr1, nr2, njt, fsz, joffs, out;
     DevBuf sort_a, sort_apos, sort_bpos, sort_seg0, sort_seg1, sort_tile_seg, sort_tile_l, sort_tile_r, sort_stops,
@@ -123,7 +125,7 @@ struct ptl_generator {
         return {&in_type, &in_rtype, &in_parent, &in_depth, &in_child, &in_data, &nt, &rt, &nd1, &nd,
                 &par, &ci, &dep, &fflag, &sizes, &loc0, &loc, &pos, &regs, &decl, &fn_id, &fn_start,
                 &fn_size, &fn_end, &fn_start0, &fn_size0, &fn_end0, &fn_ra_start, &fn_ra_end, &fn_ra_size,
-                &instr, &rd, &rs1, &rs2, &jt, &owner, &used, &smark, &used_instrs, &symreg, &symswp,
+                &instr, &rd, &rs1, &rs2, &jt, &owner, &used, &smark, &used_instrs, &tmask, &trow, &tany, &symreg, &symswp,
                 &stamp, &defpos, &lifetime, &trig_min, &trig_max, &ra_chunks, &spill, &roffs, &ni, &nrd, &nr1, &nr2, &njt,
                 &fsz, &joffs, &out, &sort_a, &sort_apos, &sort_bpos, &sort_seg0, &sort_seg1, &sort_stops,
                 &sort_tile_seg, &sort_tile_l, &sort_tile_r, &sort_leaf, &sort_heap, &sort_counters, &sort_local, &sort_equal,
@@ -251,6 +253,10 @@ Prog make_prog(ptl_generator* g) {
     P.regs = g->regs.at<uint32_t>();
     P.pos = g->pos.at<uint32_t>();
     P.owner = g->owner.at<unsigned long long>();
+    P.rec = P.owner;  // done with after isn_gen
+    P.tmask = g->tmask.at<uint32_t>();
+    P.trow = g->trow.at<uint32_t>();
+    P.tany = g->tany.at<uint32_t>();
     P.decl = g->decl.at<uint32_t>();
     P.fn_id = g->fn_id.at<uint32_t>();
     P.fn_start = g->fn_start.at<uint32_t>();
@@ -538,16 +544,31 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
     } else {
         note_launch();
         k_init_lifetime<<<std::min<size_t>((g->F + 255) / 256, 1024), 256, 0, s>>>(g->lifetime.at<unsigned long long>(), g->F);
-        const size_t trig = static_cast<size_t>(std::max<uint32_t>(g->S, 1)) * 64;
-        PTL_CU(g->trig_min.ensure(trig, 4));
-        PTL_CU(g->trig_min.fill(s, 0xFF));
-        PTL_CU(g->trig_max.ensure(trig, 4));
-        PTL_CU(g->trig_max.zero(s));
-        PTL_CU(g->ra_chunks.ensure(2 * (static_cast<size_t>(g->S) / 32 + 2), 4));
         P = make_prog(g);
-        if (!prog_ready(P, {P.lifetime, P.trig_min, P.trig_max, P.ra_chunks}))
+        if (!prog_ready(P, {P.lifetime, P.rec}))
             return fail(g, PTL_CUDA_ERROR, "internal: unallocated regalloc state");
-        PTL_CU(run_regalloc_steps(P, s, &g->ra_serial, row0_hash));
+        RaForm form = RaForm::Serial;
+        PTL_CU(ra_form(P, s, row0_hash, &form));
+        if (form == RaForm::Steps) {
+            const size_t steps = row_tiles(g->S) * kRowTile;
+            PTL_CU(g->tmask.ensure(wb8, 4));
+            PTL_CU(g->trow.ensure(steps * kRowPos, 4));
+            PTL_CU(g->tany.ensure(steps, 4));
+        } else if (form == RaForm::General) {
+            const size_t trig = static_cast<size_t>(std::max<uint32_t>(g->S, 1)) * 64;
+            PTL_CU(g->trig_min.ensure(trig, 4));
+            PTL_CU(g->trig_min.fill(s, 0xFF));
+            PTL_CU(g->trig_max.ensure(trig, 4));
+            PTL_CU(g->trig_max.zero(s));
+            PTL_CU(g->ra_chunks.ensure(2 * (static_cast<size_t>(g->S) / 32 + 2), 4));
+        }
+        P = make_prog(g);
+        if (form == RaForm::Steps ? !prog_ready(P, {P.tmask, P.trow, P.tany})
+                                  : form == RaForm::General && !prog_ready(P, {P.trig_min, P.trig_max, P.ra_chunks}))
+            return fail(g, PTL_CUDA_ERROR, "internal: unallocated regalloc state");
+        P.defpos = nullptr;
+        PTL_CU(run_regalloc_steps(P, form, s));
+        g->ra_serial = form == RaForm::Serial;
         PTL_CU(scan_for(wb8, &sc));
         launch_regalloc_count_scan(P, sc, s);
     }

@@ -17,12 +17,14 @@
 #include "ptl_sort.cuh"
 #include "ptl_stages.cuh"
 #include "ptl_ra.cuh"
+#include "ptl_steps.cuh"
 #include "ptl_scalar.cuh"
 
 using namespace ptl;
 
 namespace {
 
+uint32_t g_ring_k = 16;  // words per function in the record form's symbol ring (small: old words too)
 uint32_t g_cache_k = 4;  // entries per function of the lane-0 symbol cache
 bool g_force_hashed = false;  // lane-0 pass finds row-0 values by hashing even when definitions are unique
 bool g_last_hashed = false;   // the last compile had a lane-0 virtual register with two definitions
@@ -54,6 +56,7 @@ struct Model {
         used_instrs, symreg, symswp, stamp, trig_min, trig_max, spill, roffs, ni, nrd, nr1, nr2, njt, fsz,
         joffs, out;
     HBuf<unsigned long long> owner, lifetime;
+    HBuf<uint32_t> tmask, tany, trow;
     Prog P{};
 
     void bind() {
@@ -61,7 +64,7 @@ struct Model {
         P.in_child = in_child.p; P.in_data = in_data.p;
         P.nt = nt.p; P.rt = rt.p; P.nd1 = nd1.p; P.nd = nd.p; P.par = par.p; P.ci = ci.p; P.dep = dep.p;
         P.fflag = fflag.p; P.sizes = sizes.p; P.loc0 = loc0.p; P.loc = loc.p; P.regs = regs.p; P.pos = pos.p;
-        P.owner = owner.p; P.decl = decl.p; P.fn_id = fn_id.p; P.fn_start = fn_start.p; P.fn_size = fn_size.p;
+        P.owner = owner.p; P.rec = owner.p; P.tmask = tmask.p; P.tany = tany.p; P.trow = trow.p; P.decl = decl.p; P.fn_id = fn_id.p; P.fn_start = fn_start.p; P.fn_size = fn_size.p;
         P.fn_end = fn_end.p; P.fn_start0 = fn_start0.p; P.fn_size0 = fn_size0.p; P.instr = instr.p;
         P.rd = rd.p; P.rs1 = rs1.p; P.rs2 = rs2.p; P.jt = jt.p; P.used = used.p; P.smark = smark.p;
         P.used_instrs = used_instrs.p; P.symreg = symreg.p; P.symswp = symswp.p; P.stamp = stamp.p;
@@ -211,6 +214,77 @@ struct Model {
         P = Psave;
     }
 
+    // The record form's allocation (ptl_steps.cuh), phase by phase as its kernels run it.
+    void step_regalloc(uint32_t S, uint32_t K) {
+        std::vector<uint8_t> ring(K);
+        for (uint32_t f = 0; f < P.F; ++f)
+            if (f & 7u) step_free_function(P, f, ring.data(), 1, K);
+        const uint32_t G0 = (P.F + 7) / 8;
+        tany.ensure(row_tiles(S) * kRowTile);
+        trow.ensure(row_tiles(S) * kRowTile * kRowPos, kRowNone);
+        bind();
+        for (uint32_t i = 0; i < S; ++i) {
+            for (uint32_t g = 0; g < G0; ++g) {
+                const uint32_t m = group_triggers(P, g, i);
+                P.tany[i] |= m;
+                for (uint32_t t = m; t; t &= t - 1) {
+                    uint32_t& r = P.trow[static_cast<size_t>(i) * kRowPos + low_bit(t)];
+                    r = std::min(row_min(r), g + 1) | (std::max(row_max(r), g + 1) << 16);
+                }
+            }
+        }
+        LaneShared sh{};
+        std::vector<uint8_t> rings(static_cast<size_t>(G0) * K);
+        std::vector<LaneSlot> L(G0);
+        for (uint32_t j = 0; j < G0; ++j) {
+            L[j] = LaneSlot{};
+            lane_init(P, L[j], j);
+            sh.s0 = std::max(sh.s0, L[j].size);
+        }
+        const uint32_t s0 = std::min(sh.s0, S);
+        for (uint32_t i = 0; i < s0; ++i) {
+            LaneStep& st = sh.st[i & 1u];
+            const uint32_t* row = P.trow + static_cast<size_t>(i) * kRowPos;
+            auto ring_of = [&](uint32_t j) { return LaneRing{rings.data() + j, G0, K}; };
+            if (win_wraps(i)) for (LaneStep& x : sh.st) std::memset(x.win, 0, sizeof(x.win));
+            for (uint32_t j = 0; j < G0; ++j) {
+                L[j].rec = i < L[j].size ? L[j].rec_at[i] : kStepIdle;
+                if (G0 == 1) lane_step_a<true>(sh, st, row, L[j], ring_of(j), i, st.m);
+                else lane_step_a<false>(sh, st, row, L[j], ring_of(j), i, st.m);
+            }
+            lane_clear(sh.st[(i + 1u) & 1u]);
+            bool redo = false;
+            for (uint32_t j = 0; j < G0; ++j) {
+                lane_commit(sh, L[j]);
+                redo |= lane_step_t(sh, st, st.m, L[j]);
+            }
+            if (redo) {
+                for (uint32_t round = 0;; ++round) {
+                    for (uint32_t j = 0; j < G0; ++j) lane_round(sh, st, st.m, row, L[j]);
+                    const bool changed = st.before != sh.before2;
+                    st.before = sh.before2;
+                    sh.before2 = 0;
+                    if (!changed) break;
+                    if (round > G0 + 2) { record_error(P.err, ST_DEVICE_TIMEOUT, W_RA2, i); break; }
+                }
+                std::memset(st.win, 0, sizeof(st.win));
+                st.m.wr = st.m.trig = st.later = 0;
+                for (uint32_t j = 0; j < G0; ++j) lane_emit<false>(st, L[j], i, st.m);
+                for (uint32_t j = 0; j < G0; ++j) lane_step_t(sh, st, st.m, L[j]);
+            }
+            for (uint32_t j = 0; j < G0; ++j) {
+                if (G0 == 1) lane_step_b<true>(sh, st, st.m, LaneAbove{0, 0}, P.tany[i], L[j], ring_of(j), i);
+                else lane_step_b<false>(sh, st, st.m, LaneAbove{0, 0}, P.tany[i], L[j], ring_of(j), i);
+            }
+        }
+        uint32_t tail = 0;
+        for (uint32_t i = s0; i < S; ++i) tail |= P.tany[i];
+        for (uint32_t j = 0; j < G0; ++j) {
+            lane_commit(sh, L[j]);
+            lane_tail(sh, L[j], tail);
+        }
+    }
+
     // The scalar generator's register allocation (ptl_scalar.cuh), from the optimized words
     // to the regalloc output (the spill offsets, the count scan, the scatter, the moved
     // function table and the frame words).
@@ -344,19 +418,24 @@ struct Model {
             scalar_regalloc(F, W, wb8);
             if (!check()) return err.code;
         } else {
-            uint32_t flagbits = 0;
-            for (uint32_t i = 0; i < W; ++i) flagbits |= st_ra_cross(P, i, stamp.p);
+            uint32_t flagbits = g_force_hashed ? 2u : 0u;
+            for (uint32_t f = 0; f < F; ++f) flagbits |= st_step_range(P, f);
+            for (uint32_t i = 0; i < W; ++i) flagbits |= st_step_record(P, i);
+            g_last_hashed = (flagbits & 2u) != 0;
             const uint32_t G0 = (F + 7) / 8;
             if ((flagbits & 1u) || G0 > 8192u) {
                 st_ra_serial(P, stamp.p);
-            } else {
+            } else if (flagbits & 2u) {
                 std::vector<uint32_t> tag(64), val(64);
                 const SymCache c1{tag.data(), val.data(), 64};
                 Prog Pfree = P;
                 Pfree.defpos = nullptr;
                 for (uint32_t f = 0; f < F; ++f) if (f & 7u) ra_free_function_cached(Pfree, c1, 0, f);
-                lane0_cached(S, hm_cache_k, (flagbits & 2u) != 0 || g_force_hashed);
-                g_last_hashed = (flagbits & 2u) != 0;
+                lane0_cached(S, hm_cache_k, true);
+            } else {
+                tmask.ensure(wb8);
+                bind();
+                step_regalloc(S, g_ring_k);
             }
             for (uint32_t v = 0; v < W; ++v) st_ra_spill(P, v);
             exclusive_scan(wb8, [&](uint32_t i) { return st_ra_count(P, i); }, roffs.p);
@@ -453,6 +532,7 @@ int ptlhm_gen_desc_ok(void) {
 void ptlhm_set_scalar_serial(int on) { g_force_serial = on != 0; }
 
 void ptlhm_set_cache_entries(uint32_t k) { g_cache_k = k; }
+void ptlhm_set_ring_words(uint32_t k) { g_ring_k = k; }  // a power of two
 void ptlhm_set_hashed(int on) { g_force_hashed = on != 0; }
 int ptlhm_last_hashed(void) { return g_last_hashed ? 1 : 0; }
 

@@ -14,6 +14,7 @@
 
 #include "ptl_kernels.cuh"
 #include "ptl_ra.cuh"
+#include "ptl_steps.cuh"
 
 namespace ptl {
 
@@ -1710,6 +1711,16 @@ __global__ void k_ra_cross(Prog P) {
     if (__syncthreads_or(any & 1u) && threadIdx.x == 0) P.flags[1] = 1;
     if (__syncthreads_or(any & 2u) && threadIdx.x == 0) P.flags[2] = 1;
 }
+// The step records; flags[1]: functions share symbols, flags[2]: a word that a record
+// cannot say, or function ranges that overlap.
+__global__ void k_ra_records(Prog P) {
+    uint32_t any = 0;
+    uint32_t hint = 0xFFFFFFFFu;
+    PTL_FOR(i, P.W) any |= st_step_record(P, i, &hint);
+    PTL_FOR(f, P.F) any |= st_step_range(P, f);
+    if (__syncthreads_or(any & 1u) && threadIdx.x == 0) P.flags[1] = 1;
+    if (__syncthreads_or(any & 2u) && threadIdx.x == 0) P.flags[2] = 1;
+}
 __global__ void k_ra_serial(Prog P) {
     if (blockIdx.x == 0 && threadIdx.x == 0) st_ra_serial(P, P.stamp);
 }
@@ -2255,35 +2266,35 @@ cudaError_t launch_ra_steps(const Prog& P0, const Prog& Pfree, uint32_t G0, cuda
     }
 }
 
-cudaError_t run_regalloc_steps(const Prog& P, cudaStream_t s, bool* serial_out, bool row0_hash) {
-    // Programs whose functions share symbols need the reference's serial order.
+cudaError_t ra_form(const Prog& P, cudaStream_t s, bool general, RaForm* form) {
     cudaMemsetAsync(P.flags + 1, 0, 2 * sizeof(uint32_t), s);
-    cudaMemsetAsync(P.stamp, 0, sizeof(uint32_t) * P.W, s);
-    cudaMemsetAsync(P.defpos, 0, P.W, s);
     g_launches++;
-    k_ra_cross<<<grid_for(P.W), kThreads, 0, s>>>(P);
+    k_ra_records<<<grid_for(P.W), kThreads, 0, s>>>(P);
     uint32_t fl[2] = {0, 0};
     cudaMemcpyAsync(fl, P.flags + 1, sizeof(fl), cudaMemcpyDeviceToHost, s);
     const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
-    const uint32_t cross = fl[0];
-    // independent functions never need the definition positions; the lane-0 pass hashes
-    // row 0 when a virtual register has two definitions
-    Prog Pfree = P, P0 = P;
-    Pfree.defpos = nullptr;
-    if (fl[1] || row0_hash) P0.defpos = nullptr;
+    // functions that share symbols (or too many lane-0 functions) need the serial order
     const uint32_t G0 = (P.F + 7u) / 8u;
-    if (cross || G0 > 8192u) {
-        // functions share symbols (or too many lane-0 functions for one CTA): serial path
+    if (fl[0] || G0 > 8192u) *form = RaForm::Serial;
+    else if (fl[1] || general || (G0 > kStepBlockMax && (ra_cluster_disabled() || !step_cluster_fits(G0)))) *form = RaForm::General;
+    else *form = RaForm::Steps;
+    return cudaSuccess;
+}
+
+cudaError_t run_regalloc_steps(const Prog& P, RaForm form, cudaStream_t s) {
+    cudaError_t ce = cudaSuccess;
+    if (form == RaForm::Serial) {
         g_launches++;
         k_ra_serial<<<1, 1, 0, s>>>(P);
+    } else if (form == RaForm::General) {
+        ce = launch_ra_steps(P, P, (P.F + 7u) / 8u, s);
     } else {
-        const cudaError_t ce = launch_ra_steps(P0, Pfree, G0, s);
-        if (ce != cudaSuccess) return ce;
+        ce = run_step_regalloc(P, s);
     }
+    if (ce != cudaSuccess) return ce;
     g_launches++;
     k_ra_spill<<<grid_for(P.W), kThreads, 0, s>>>(P);
-    if (serial_out) *serial_out = cross != 0;
     return cudaGetLastError();
 }
 
@@ -2534,7 +2545,7 @@ struct BOptMark {
     }
 };
 PTL_BATCH_OP(BOptFinal, P.wb8, st_opt_final(P, i))
-PTL_BATCH_OP(BInitLifetime, P.F, P.lifetime[i] = 0x1Full)
+PTL_BATCH_OP(BInitLifetime, P.F, P.lifetime[i] = 0x1Full; if (st_step_range(P, i)) P.flags[2] = 1u)
 // spill flags and cross checks find each word's function from the thread's previous
 // word (the same program, 256 words earlier within a tile)
 struct BSpill {
@@ -2556,6 +2567,17 @@ PTL_BATCH_OP(BRaHist, P.F - (P.F + 7u) / 8u,
              const uint32_t f = free_function_of(i);
              const uint32_t size = P.fn_size0[f];
              if (s32(size) > 0) atomicAdd(&P.ra_chunks[(size - 1u) / kRaChunk], 1u))
+struct BRecords {
+    static constexpr bool kViewInShared = true;
+    uint32_t hint = 0xFFFFFFFFu, hp = 0xFFFFFFFFu;
+    __device__ static uint32_t count(const Prog& P) { return P.W; }
+    __device__ void operator()(const Prog& P, uint32_t i, uint32_t p) {
+        if (p != hp) { hp = p; hint = 0xFFFFFFFFu; }
+        const uint32_t r = st_step_record(P, i, &hint);
+        if (r & 1u) P.flags[1] = 1u;
+        if (r & 2u) P.flags[2] = 1u;
+    }
+};
 struct BCross {
     static constexpr bool kViewInShared = true;
     uint32_t hint = 0xFFFFFFFFu, hp = 0xFFFFFFFFu;
@@ -2975,6 +2997,7 @@ void batch_stage(BatchStage st, const BatchLaunch& bl, uint32_t total, uint32_t*
         case BatchStage::OptFinal: batch_launch(bl, total, BOptFinal{}); break;
         case BatchStage::InitLifetime: batch_launch(bl, total, BInitLifetime{}); break;
         case BatchStage::Cross: batch_launch(bl, total, BCross{}); break;
+        case BatchStage::Records: batch_launch(bl, total, BRecords{}); break;
         case BatchStage::RaHist: batch_launch(bl, total, BRaHist{}); break;
         case BatchStage::Spill: batch_launch(bl, total, BSpill{}); break;
         case BatchStage::Scatter: batch_launch(bl, total, BScatter{}); break;

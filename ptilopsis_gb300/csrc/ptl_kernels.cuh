@@ -44,6 +44,8 @@ struct ScanScratch {
 // Kernel launches issued by this library since load (counted at each launch site).
 uint64_t launch_count();
 void note_launch();
+// Raises a kernel's dynamic shared memory limit to at least bytes (never lowers it).
+cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes);
 
 // Element-wise stages (grid-stride launches of the per-thread functions).
 void launch_ingest(const Prog& P, cudaStream_t s);  // input checks + copy; flags[3]: max_depth reached
@@ -55,7 +57,32 @@ void launch_functab(const Prog& P, uint32_t* meta, cudaStream_t s);
 
 void launch_gen(const Prog& P, cudaStream_t s);
 cudaError_t run_optimize(const Prog& P, cudaStream_t s, uint32_t* sweeps_out);
-cudaError_t run_regalloc_steps(const Prog& P, cudaStream_t s, bool* serial_out, bool row0_hash);
+// Register allocation of one program.  ra_form builds the step records (P.rec) and tells
+// which form the program takes; the caller then provides that form's arrays:
+//   Steps: tmask (one per word), trow and tany (row_tiles(S) tiles of kRowTile steps);
+//   General: trig_min / trig_max (set to none), ra_chunks;
+//   Serial: none.
+enum class RaForm { Steps, General, Serial };
+cudaError_t ra_form(const Prog& P, cudaStream_t s, bool general, RaForm* form);
+cudaError_t run_regalloc_steps(const Prog& P, RaForm form, cudaStream_t s);
+// The record form of one program, and of the programs order[0..n) of a batch: program
+// order[k] has its independent functions (32 a block) in blocks free_off[k].. and its
+// trigger rows (kRowTile steps a block) in blocks row_off[k]..
+// The lane-0 pass of a program with more than kStepClusterMin groups runs on a
+// thread-block cluster where the device can place one; with more than kStepBlockMax it
+// has to (else the program takes the general form).
+constexpr uint32_t kStepClusterMin = 256, kStepBlockMax = 1024;
+bool step_cluster_fits(uint32_t G0);
+bool ra_cluster_disabled();
+cudaError_t run_step_regalloc(const Prog& P, cudaStream_t s);
+struct StepBatch {
+    const Prog* progs;
+    const uint32_t* order;
+    const uint32_t* free_off;  // [n + 1]
+    const uint32_t* row_off;   // [n + 1]
+    uint32_t n, free_blocks, row_blocks, max_g0;
+};
+cudaError_t batch_step_regalloc(const StepBatch& b, cudaStream_t s);
 // Lane-0 passes too wide for one block: programs with more than kRaClusterMin lane-0
 // groups (at most 8,192) run theirs on a thread-block cluster when the device can place
 // it.  ra_cluster_fits tells whether it can; launch_ra_wide launches the program's
@@ -120,7 +147,7 @@ struct BatchLaunch {
     uint32_t tile;
 };
 enum class BatchStage {
-    Ingest, Preprocess, Fix, Functab, Gen, OptMark, OptFinal, InitLifetime, Cross, RaHist, Spill,
+    Ingest, Preprocess, Fix, Functab, Gen, OptMark, OptFinal, InitLifetime, Cross, Records, RaHist, Spill,
     Scatter, RaFunctab, FjEmit, FjFunctab,
     // the scalar generator's (ptl_scalar.cuh): preprocess, isn_gen, preserve counts
     // (per function), scatter (per word), the function table after regalloc (per

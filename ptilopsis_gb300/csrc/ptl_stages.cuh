@@ -171,6 +171,10 @@ struct Prog {
     // regalloc
     uint32_t* symreg;
     uint32_t* symswp;
+    unsigned long long* rec;    // step records (ptl_steps.cuh); isn_gen's owner array, done with by then
+    uint32_t* tmask;      // per word: positions its step triggers (independent functions)
+    uint32_t* trow;       // [S in whole tiles][kRowPos] trigger rows
+    uint32_t* tany;       // [S in whole tiles] positions triggered at all
     uint32_t* stamp;      // definitions per virtual register (regalloc cross check)
     uint8_t* defpos;      // row-0 position + 1 of each lane-0 definition; null: use the row-0 hash
     unsigned long long* lifetime;

@@ -1,0 +1,63 @@
+"""The record form of register allocation (step records, trigger rows, lane-0 slots on one
+thread, one warp, one block or a cluster) against the oracle, at the widths where the
+launch changes and with symbol rings of every size.  All results are whole numbers."""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from conftest import tree_to_ast
+from ptilopsis_gb300.synth import SynthParams, generate
+
+
+def _program(n_functions, median=40.0, seed=0x50544D00, **more):
+    more = {"sigma": 1.0, "max_nesting": 6, "spill_frac": 0.25, **more}
+    return generate(SynthParams(seed=seed + n_functions, n_functions=n_functions, median_fn_nodes=median, **more))
+
+
+@pytest.mark.parametrize("ring", [4, 16, 1024])
+@pytest.mark.parametrize("n_functions", [1, 8, 9, 40, 300])
+def test_hostmodel_record_form(built, n_functions, ring):
+    """The kernels' step functions on the CPU; a ring of 4 words reads most operands' symbols
+    back from memory."""
+    from test_hostmodel import assert_stages_equal, hostmodel
+    L = hostmodel()
+    L.ptlhm_set_ring_words(ctypes.c_uint32(ring))
+    try:
+        assert_stages_equal(tree_to_ast(_program(n_functions, 150.0, max_expr_depth=12, float_frac=0.5)))
+    finally:
+        L.ptlhm_set_ring_words(ctypes.c_uint32(16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_functions", [1, 8, 9, 256, 257, 2048, 2049, 8192, 8193])
+def test_gpu_lane0_widths(built_cuda, n_functions):
+    """1 group (a lone slot), 2 and 32 (one warp), 33 and 256 (a block), 257 (a cluster of
+    three CTAs), 1,024 and 1,025 (eight)."""
+    from oracle import portbind
+    from ptilopsis_gb300 import RvGenerator
+    tree = _program(n_functions)
+    ref = portbind.compile_ast(tree_to_ast(tree))
+    with RvGenerator(tree) as gen:
+        gen.process()
+        np.testing.assert_array_equal(gen.get_instructions(), ref.words)
+        t = gen.function_table()
+        gen.process(row0_hash=True)  # the general form
+        np.testing.assert_array_equal(gen.get_instructions(), ref.words)
+        np.testing.assert_array_equal(gen.function_table()["starts"], t["starts"])
+
+
+@pytest.mark.gpu
+def test_gpu_batch_of_all_widths(built_cuda):
+    """Programs of every width in one batch (a block per program sized by the widest, the
+    widest of all on a cluster), with operands older than the batch's symbol ring."""
+    from oracle import portbind
+    from ptilopsis_gb300.batch import BatchCompiler
+    trees = [_program(n) for n in (1, 3, 9, 257, 700, 8200)]
+    trees += [_program(5, 3000.0, seed=0x50544D80 + k, max_expr_depth=12, float_frac=0.5, max_nesting=64) for k in range(3)]
+    with BatchCompiler(tiles=None) as b:
+        b.compile(trees)
+        for k, tree in enumerate(trees):
+            np.testing.assert_array_equal(b.words(k), portbind.compile_ast(tree_to_ast(tree)).words, err_msg=str(k))
