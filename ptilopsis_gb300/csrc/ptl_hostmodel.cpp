@@ -243,7 +243,7 @@ struct Model {
         }
         const uint32_t s0 = std::min(sh.s0, S);
         for (uint32_t i = 0; i < s0; ++i) {
-            LaneStep& st = sh.st[i & 1u];
+            LaneStep& st = sh.st[i % 3u];
             const uint32_t* row = P.trow + static_cast<size_t>(i) * kRowPos;
             auto ring_of = [&](uint32_t j) { return LaneRing{rings.data() + j, G0, K}; };
             if (win_wraps(i)) for (LaneStep& x : sh.st) std::memset(x.win, 0, sizeof(x.win));
@@ -252,7 +252,7 @@ struct Model {
                 if (G0 == 1) lane_step_a<true>(sh, st, row, L[j], ring_of(j), i, st.m);
                 else lane_step_a<false>(sh, st, row, L[j], ring_of(j), i, st.m);
             }
-            lane_clear(sh.st[(i + 1u) & 1u]);
+            lane_clear(sh.st[(i + 2u) % 3u]);
             bool redo = false;
             for (uint32_t j = 0; j < G0; ++j) {
                 lane_commit(sh, L[j]);
@@ -273,8 +273,9 @@ struct Model {
                 for (uint32_t j = 0; j < G0; ++j) lane_step_t(sh, st, st.m, L[j]);
             }
             for (uint32_t j = 0; j < G0; ++j) {
-                if (G0 == 1) lane_step_b<true>(sh, st, st.m, LaneAbove{0, 0}, P.tany[i], L[j], ring_of(j), i);
-                else lane_step_b<false>(sh, st, st.m, LaneAbove{0, 0}, P.tany[i], L[j], ring_of(j), i);
+                lane_step_b1(L[j], ring_of(j), i, false);
+                if (G0 == 1) lane_step_b2<true>(sh, st, st.m, LaneAbove{0, 0}, P.tany[i], L[j], ring_of(j), i);
+                else lane_step_b2<false>(sh, st, st.m, LaneAbove{0, 0}, P.tany[i], L[j], ring_of(j), i);
             }
         }
         uint32_t tail = 0;

@@ -109,11 +109,12 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_step_rows(Src src) {
 }
 
 // ---- lane-0 functions in lock-step: a thread per slot (slot = group), a block per
-// program.  Two barriers a step: after phase A (lookups, allocation, row-0 writes) and
-// after phase T (triggers that cross slots), whose barrier also tells whether one changed
-// what phase A assumed.  Trigger rows come in tiles of 32 steps by cp.async, one tile
-// ahead, and a slot's records kLaneAhead steps ahead: one commit group a step.  (Records in
-// registers need the loop unrolled as often, which no longer fits the instruction cache.)
+// program.  At most two barriers a step: after phase A (lookups, allocation, row-0 writes)
+// and, when some slot's operand is open to other slots' triggers, after phase T, whose
+// barrier also tells whether a trigger changed what phase A assumed.  Trigger rows come in tiles of 32 steps by cp.async, one tile
+// ahead, and a slot's records by fours, four steps ahead: one commit group every four
+// steps.  (Records in registers need the loop unrolled as often, which no longer fits the
+// instruction cache; a group every step costs 130 cycles of it.)
 //
 // A program with many groups spreads them over the CTAs of a cluster, ascending by rank.
 // Each CTA resolves a step among its own slots as above, then writes its masks into every
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_step_rows(Src src) {
 // changes what phase A assumed is seen by every CTA in the same masks, so all of them
 // agree on another round.
 enum LaneMode { kAlone, kOneWarp, kManyWarps, kCluster };
-constexpr uint32_t kRowBufs = 2, kClusterMax = 8;
+constexpr uint32_t kRowBufs = 2, kClusterMax = 8, kClusterSlots = 256;
 __device__ __forceinline__ void copy16_async(void* dst, const void* src) {
     const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at), "l"(src));
@@ -133,10 +134,8 @@ __device__ __forceinline__ void copy8_async(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(at), "l"(src));
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::); }
-constexpr uint32_t kRecBufs = 8, kLaneAhead = kRecBufs - 1u;  // a power of two
-// All but the last kLaneAhead - 1 groups: the next step's records, and rows committed that
-// many steps ago.
-__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(kLaneAhead - 1u) : "memory"); }
+constexpr uint32_t kRecBufs = 8, kRecGroup = 4;  // records per slot in shared memory, in groups; powers of two
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Tile t's trigger rows and positions triggered at all, into buffer t % kRowBufs.
 __device__ __forceinline__ void copy_rows_async(const Prog& P, uint32_t* rows, uint32_t* any, uint32_t t,
                                                 uint32_t tid, uint32_t T) {
@@ -189,8 +188,9 @@ __device__ __forceinline__ uint32_t remote_at(uint32_t at, uint32_t rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(rank));
     return to;
 }
-__device__ __forceinline__ void store_async(uint32_t to, uint32_t v, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(to), "r"(v), "r"(bar)
+__device__ __forceinline__ void store_async(uint32_t to, const LaneMasks& m, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.u32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(to),
+                 "r"(m.wr), "r"(m.trig), "r"(m.use), "r"(m.need), "r"(bar)
                  : "memory");
 }
 __device__ __forceinline__ void mbar_init(const void* bar) {
@@ -199,16 +199,20 @@ __device__ __forceinline__ void mbar_init(const void* bar) {
 __device__ __forceinline__ void mbar_expect(const void* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_at(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try(const void* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_test(const void* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(shared_at(bar)), "r"(parity)
         : "memory");
     return ok != 0;
 }
 constexpr long long kExchangeCycles = 1ll << 31;  // about a second
+__device__ __forceinline__ void or_if(uint32_t on, uint32_t* p, uint32_t v) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q red.shared.or.b32 [%0], %1;\n}" ::"r"(shared_at(p)), "r"(v),
+                 "r"(on));  // read after a barrier only
+}
 __device__ __forceinline__ uint32_t warp_or(uint32_t v) { return __reduce_or_sync(0xFFFFFFFFu, v); }
 
 // The masks over all slots.  One warp keeps them in registers (one slot has them already);
@@ -217,14 +221,19 @@ template <int kMode>
 __device__ __forceinline__ void lane_share(LaneStep& st, LaneMasks& m) {
     if constexpr (kMode == kAlone) return;
     LaneMasks all{warp_or(m.wr), warp_or(m.trig), 0, 0};
-    if (warp_any((m.use | m.need) != 0)) {
+    const bool open = warp_any((m.use | m.need) != 0);
+    if (open) {
         all.use = warp_or(m.use);
         all.need = warp_or(m.need);
     }
     if constexpr (kMode >= kManyWarps) {
-        const uint32_t lane = threadIdx.x & 31u;
-        const uint32_t mine = lane == 0 ? all.wr : lane == 1u ? all.trig : lane == 2u ? all.use : all.need;
-        if (lane < 4u && mine) atomicOr(reinterpret_cast<uint32_t*>(&st.m) + lane, mine);
+        const uint32_t first = (threadIdx.x & 31u) == 0;
+        or_if(first, &st.m.wr, all.wr);
+        or_if(first, &st.m.trig, all.trig);
+        if (open) {
+            or_if(first, &st.m.use, all.use);
+            or_if(first, &st.m.need, all.need);
+        }
     } else {
         m = all;
     }
@@ -234,10 +243,10 @@ __device__ __forceinline__ void lane_masks(const LaneStep& st, LaneMasks& m) {
     if constexpr (kMode >= kManyWarps) m = st.m;
 }
 
-// The cluster's masks of a step: [buffer][rank][wr, trig, use, need].
+// The cluster's masks of a step, by buffer and rank.
 struct LaneExchange {
-    unsigned long long bar[2];  // mbarriers, one per buffer
-    uint32_t m[2][kClusterMax][4];
+    LaneMasks m[2][kClusterMax];  // 16-byte stores
+    unsigned long long bar[2];    // mbarriers, one per buffer
 };
 
 // Dynamic shared memory of a CTA with T slots.
@@ -254,8 +263,6 @@ struct LaneLayout {
     __host__ __device__ size_t bytes(uint32_t T) const { return ring_at(T) + static_cast<size_t>(K) * stride(T); }
 };
 
-static_assert(sizeof(LaneMasks) == 16, "lane_share addresses the masks by word");
-
 // The program's slots [j0, j1) on the first T threads of this CTA (rank of C).
 template <int kMode>
 __device__ void lane_pass(const Prog& P, unsigned char* smem, uint32_t T, uint32_t K, uint32_t j0, uint32_t j1,
@@ -270,18 +277,21 @@ __device__ void lane_pass(const Prog& P, unsigned char* smem, uint32_t T, uint32
     unsigned long long* recs = reinterpret_cast<unsigned long long*>(smem + LaneLayout::rec_at()) + tid;  // [kRecBufs][T]
     const uint32_t G0 = (P.F + 7u) / 8u;
     auto clear_win = [&] {
-        for (uint32_t p = tid; p < kRowPos; p += T) sh.st[0].win[p] = sh.st[1].win[p] = 0;
+        for (uint32_t p = tid; p < kRowPos; p += T) sh.st[0].win[p] = sh.st[1].win[p] = sh.st[2].win[p] = 0;
     };
     clear_win();
     if (tid == 0) {
         lane_clear(sh.st[0]);
         lane_clear(sh.st[1]);
+        lane_clear(sh.st[2]);
         sh.before2 = sh.tail = 0;
         sh.s0 = 0;
         if (kMode == kCluster) {
             mbar_init(&ex.bar[0]);
             mbar_init(&ex.bar[1]);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            mbar_expect(&ex.bar[0], C * 16u);
+            mbar_expect(&ex.bar[1], C * 16u);
         }
     }
     if (kMode == kCluster) cluster_barrier();  // every CTA's mbarriers are ready before a store to it
@@ -299,16 +309,26 @@ __device__ void lane_pass(const Prog& P, unsigned char* smem, uint32_t T, uint32
     } else if (L.size) {
         atomicMax(&sh.s0, L.size);
     }
-    auto fetch = [&](uint32_t i) {  // step i's record
-        if (i < L.size) copy8_async(recs + (i & (kRecBufs - 1u)) * T, L.rec_at + i);
-        copy_commit();
+    auto fetch = [&](uint32_t i) {  // the records of the group from step i on
+#pragma unroll
+        for (uint32_t k = 0; k < kRecGroup; ++k)
+            if (i + k < L.size) copy8_async(recs + ((i + k) & (kRecBufs - 1u)) * T, L.rec_at + i + k);
     };
     copy_rows_async(P, rows, any, 0, tid, T);
-    for (uint32_t i = 0; i < kLaneAhead; ++i) fetch(i);
+    fetch(0);
+    copy_commit();
     copy_wait();
     bar.sync();
     const uint32_t s0 = min(sh.s0, P.S);
     uint32_t turn = 0;   // exchanges so far
+    uint32_t remote_m = 0, remote_bar = 0;  // where thread k < C puts this CTA's masks in CTA k
+    if (kMode == kCluster && tid < C) {
+        remote_m = remote_at(shared_at(&ex.m[0][rank]), tid);
+        remote_bar = remote_at(shared_at(&ex.bar[0]), tid);
+    }
+    uint32_t at = 0;     // i % 3
+    bool busy = true;
+    unsigned long long next = L.size ? recs[0] : kStepIdle;
 #pragma unroll 1
     for (uint32_t i = 0; i < s0; ++i) {
         if (PTL_RARE(win_wraps(i))) {
@@ -316,25 +336,30 @@ __device__ void lane_pass(const Prog& P, unsigned char* smem, uint32_t T, uint32
             clear_win();
             bar.sync();
         }
-        LaneStep& st = sh.st[i & 1u];
+        LaneStep& st = sh.st[at];
         const uint32_t slot = i & (kRowBufs * kRowTile - 1u);
         const uint32_t* row = rows + slot * kRowPos;
+        const uint32_t others = any[slot];
         LaneMasks m{0, 0, 0, 0};
-        // a warp whose functions have ended and left row 0 only keeps the barriers
-        const bool busy = kMode <= kOneWarp || __any_sync(0xFFFFFFFFu, i < L.size || L.held != 0);
         if (busy) {
-            L.rec = i < L.size ? recs[(i & (kRecBufs - 1u)) * T] : kStepIdle;
+            L.rec = next;
             lane_step_a<kOne>(sh, st, row, L, ring, i, m);
             lane_share<kMode>(st, m);
         }
         bar.sync();
-        if ((i & (kRowTile - 1u)) == 0 && i + kRowTile < s0) copy_rows_async(P, rows, any, i / kRowTile + 1u, tid, T);
-        fetch(i + kLaneAhead);
-        copy_wait();
+        if ((i & (kRecGroup - 1u)) == kRecGroup - 1u) copy_wait();  // the next group
+        if ((i & (kRecGroup - 1u)) == 0) {
+            fetch(i + kRecGroup);
+            if ((i & (kRowTile - 1u)) == 0 && i + kRowTile < s0) copy_rows_async(P, rows, any, i / kRowTile + 1u, tid, T);
+            copy_commit();
+            // a warp whose functions have ended and left row 0 only keeps the barriers
+            if constexpr (kMode >= kManyWarps) busy = __any_sync(0xFFFFFFFFu, i < L.size || L.held != 0);
+        }
+        next = i + 1u < L.size ? recs[((i + 1u) & (kRecBufs - 1u)) * T] : kStepIdle;
         lane_masks<kMode>(st, m);
         LaneAbove above{0, 0};
         if constexpr (!kOne) {
-            if (tid == 0) lane_clear(sh.st[(i + 1u) & 1u]);
+            if (tid == 0) lane_clear(sh.st[at == 0 ? 2u : at - 1u]);
             // Jacobi rounds among this CTA's slots: until the positions triggered before
             // their owners stop changing (a DAG in group order), then the step's writes
             // and triggers again.
@@ -370,58 +395,57 @@ __device__ void lane_pass(const Prog& P, unsigned char* smem, uint32_t T, uint32
                 if (busy) lane_step_t(sh, st, m, L);
                 bar.sync();
             };
-            const bool redo = busy && lane_step_t(sh, st, m, L);
             if (busy) lane_commit(sh, L);
-            if (PTL_RARE(bar.any(redo))) settle();
+            // with nothing open no trigger can act across slots: no phase T, and no barrier
+            if (m.use | m.need) {
+                const bool redo = busy && lane_step_t(sh, st, m, L);
+                if (PTL_RARE(bar.any(redo))) settle();
+            }
             if constexpr (kMode == kCluster) {
                 uint32_t used = 0;  // of rank `lane`: what its last round took from lower ranks
                 for (uint32_t round = 0;; ++round) {
                     // A buffer is written again two exchanges later, when every CTA has
                     // sent its part of the one between, which each does after a barrier
                     // of its own threads behind their reads of this one.
-                    uint32_t(*x)[4] = ex.m[turn & 1u];
+                    LaneMasks* x = ex.m[turn & 1u];
                     const void* xbar = &ex.bar[turn & 1u];
-                    if (tid < 32u) {
-                        if (lane < 4u * C) {
-                            const uint32_t to = lane >> 2, k = lane & 3u;
-                            const uint32_t v = k == 0 ? m.wr : k == 1u ? m.trig : k == 2u ? m.use : m.need;
-                            store_async(remote_at(shared_at(&x[rank][k]), to), v, remote_at(shared_at(xbar), to));
-                        }
-                        if (lane == 0) mbar_expect(xbar, C * 16u);
+                    if (tid < C) {
+                        const uint32_t off = (turn & 1u) * static_cast<uint32_t>(sizeof(ex.m[0]));
+                        store_async(remote_m + off, m, remote_bar + (turn & 1u) * 8u);
                     }
+                    if (busy) lane_step_b1(L, ring, i, round != 0);  // while the masks travel
                     // The first warp waits for the masks, then the block's barrier lets the
                     // others at them and tells all whether the wait gave up.
                     bool lost = false;
                     if (tid < 32u) {
                         const uint32_t parity = (turn >> 1) & 1u;
                         const long long since = clock64();
-                        while (!lost && !mbar_try(xbar, parity)) lost = clock64() - since > kExchangeCycles;
+                        while (!lost && !mbar_test(xbar, parity)) lost = clock64() - since > kExchangeCycles;
+                        if (lane == 0) mbar_expect(xbar, C * 16u);  // its next phase
                     }
                     if (bar.any(lost)) {
                         if (tid == 0) record_error(P.err, ST_DEVICE_TIMEOUT, W_RA2, i);
                         return;  // this CTA sends no more, so the others' waits end too
                     }
                     ++turn;
-                    uint32_t wr = 0, trig = 0, need = 0;
-                    if (lane < C) {
-                        wr = x[lane][0];
-                        trig = x[lane][1];
-                        need = x[lane][3];
-                    }
-                    above.wr = warp_or(lane > rank ? wr : 0u);
-                    above.trig = warp_or(lane > rank ? trig : 0u);
+                    const LaneMasks theirs = lane < C ? x[lane] : LaneMasks{0, 0, 0, 0};
+                    above.wr = warp_or(lane > rank ? theirs.wr : 0u);
+                    above.trig = warp_or(lane > rank ? theirs.trig : 0u);
                     // every rank's triggers from lower ranks: a prefix over the lanes
-                    uint32_t lower = trig;
+                    uint32_t takes = 0;
+                    if (warp_any(theirs.need != 0)) {
+                        uint32_t lower = theirs.trig;
 #pragma unroll
-                    for (uint32_t d = 1; d < kClusterMax; d <<= 1) {
-                        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, lower, d);
-                        if (lane >= d) lower |= y;
+                        for (uint32_t d = 1; d < kClusterMax; d <<= 1) {
+                            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, lower, d);
+                            if (lane >= d) lower |= y;
+                        }
+                        lower = __shfl_up_sync(0xFFFFFFFFu, lower, 1);
+                        takes = lane > 0 ? lower & theirs.need : 0u;
                     }
-                    lower = __shfl_up_sync(0xFFFFFFFFu, lower, 1);
-                    const uint32_t takes = lane > 0 && lane < C ? lower & need : 0u;
-                    if (!__any_sync(0xFFFFFFFFu, takes != used)) {
-                        m.wr = warp_or(wr);
-                        m.trig = warp_or(trig);
+                    if (!warp_any(takes != used)) {
+                        m.wr = warp_or(theirs.wr);
+                        m.trig = warp_or(theirs.trig);
                         break;
                     }
                     if (round > G0 + 2u) {
@@ -436,9 +460,12 @@ __device__ void lane_pass(const Prog& P, unsigned char* smem, uint32_t T, uint32
         } else {
             lane_commit(sh, L);
         }
-        if (busy) lane_step_b<kOne>(sh, st, m, above, any[slot], L, ring, i);
+        if (busy) {
+            if constexpr (kMode != kCluster) lane_step_b1(L, ring, i, false);
+            lane_step_b2<kOne>(sh, st, m, above, others, L, ring, i);
+        }
+        at = at == 2u ? 0u : at + 1u;
     }
-    if (s0 >= P.S) return;
     uint32_t tail = 0;
     for (uint32_t i = s0 + tid; i < P.S; i += T) tail |= P.tany[i];
     if (tail) atomicOr(&sh.tail, tail);
@@ -503,7 +530,7 @@ cudaError_t launch_lane0(const Src& src, uint32_t programs, uint32_t max_g0, uin
 // (nothing is launched otherwise, nor with dry set).
 cudaError_t launch_lane0_cluster(const Prog& P, uint32_t G0, cudaStream_t s, bool dry, bool* placed) {
     *placed = false;
-    const uint32_t C = std::min(kClusterMax, (G0 + 127u) / 128u), per_cta = (G0 + C - 1u) / C;
+    const uint32_t C = std::min(kClusterMax, (G0 + kClusterSlots - 1u) / kClusterSlots), per_cta = (G0 + C - 1u) / C;
     const uint32_t T = (per_cta + 31u) & ~31u;
     const LaneLayout l = lane_layout(T, 256u);
     auto go = [&](auto kernel) -> cudaError_t {

@@ -213,8 +213,9 @@ PTL_HD uint32_t group_triggers(const Prog& P, uint32_t g, uint32_t i) {
 // written after them; oidx: that symbol's word within its function, read by its owner
 // only and written by the new owner one step late, after the next barrier (a displaced
 // owner may still read its own until then; LaneSlot::new_p is the write not yet made).
-// The step's buffers alternate by step parity: the next one is cleared between a step's
-// barriers.  win needs no clearing but where the step tags of its values start again.
+// Three sets of the step's buffers take turns: the one after next is cleared behind a
+// step's first barrier, when every slot is done with the step before.  win needs no
+// clearing but where the step tags of its values start again.
 struct LaneMasks {
     uint32_t wr;      // positions written in the step
     uint32_t trig;  // positions triggered by a lane-0 function
@@ -232,7 +233,7 @@ struct LaneStep {
     uint32_t later;             // of use: a later lane-0 group does
 };
 struct LaneShared {
-    LaneStep st[2];
+    LaneStep st[3];
     uint32_t own[kRowPos], oidx[kRowPos];
     uint32_t before2;            // the next Jacobi round's
     uint32_t tail;               // positions triggered after the last lane-0 function has ended
@@ -259,8 +260,7 @@ PTL_HD void max_if(bool on, uint32_t* p, uint32_t v) {
 #if defined(__CUDA_ARCH__)
     asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q red.shared.max.u32 [%0], %1;\n}" ::"r"(
                      static_cast<uint32_t>(__cvta_generic_to_shared(p))),
-                 "r"(v), "r"(static_cast<uint32_t>(on))
-                 : "memory");
+                 "r"(v), "r"(static_cast<uint32_t>(on)));  // read after a barrier only
 #else
     if (on && v > *p) *p = v;
 #endif
@@ -277,7 +277,10 @@ PTL_HD void or_u32(uint32_t* p, uint32_t v) {
 // register is no longer the row-0 position its definition wrote).
 constexpr uint32_t kSymSwapped = 0x40u, kSymMoved = 0x80u;
 struct LaneSlot {
-    uint32_t live, held, marked;  // held: positions where row 0 has a symbol of this slot; marked: already marked
+    // held: positions where row 0 has a symbol of this slot; marked: those of them whose
+    // symbol is swapped -- the symbol's own swapped state is written when it leaves row 0
+    // (most are read before that, which ends the swap).
+    uint32_t live, held, marked;
     uint32_t j, size;
     uint32_t* symreg;   // of the function's first word
     uint32_t* symswp;
@@ -332,8 +335,8 @@ PTL_HD uint32_t lane_find(const uint32_t* oidx, const LaneSlot& L, uint32_t idx)
 PTL_HD void lane_allocate(LaneSlot& L) {
     const uint32_t hi = static_cast<uint32_t>(L.rec >> 32);
     const bool fop = (hi & kStepFloat) != 0;
-    L.c1 = ((L.e1 & kSymSwapped) || L.b1) ? (fop ? 0u : 5u) : (L.e1 & 63u);
-    L.c2 = ((L.e2 & kSymSwapped) || L.b2) ? (fop ? kCode38 : 6u) : (L.e2 & 63u);
+    L.c1 = ((L.e1 & kSymSwapped) || (L.m1 & L.marked) || L.b1) ? (fop ? 0u : 5u) : (L.e1 & 63u);
+    L.c2 = ((L.e2 & kSymSwapped) || (L.m2 & L.marked) || L.b2) ? (fop ? kCode38 : 6u) : (L.e2 & 63u);
     L.o = step_allocate(hi, L.live, L.c1, L.c2);
 }
 // The step's row-0 writes (rd's symbol or physical register, the cleared rs1 / rs2
@@ -426,30 +429,54 @@ PTL_HD void lane_round(LaneShared& sh, const LaneStep& st, const LaneMasks& m, c
         if (L.j < sh.own[low_bit(t)]) or_u32(&sh.before2, t & (~t + 1u));
 }
 
-PTL_HD void lane_store(const LaneSlot& L, const LaneRing& r, uint32_t i, uint32_t d, uint32_t old, uint32_t code,
-                       bool swapped) {
-    const uint32_t now = code | (swapped ? kSymSwapped : 0u) | ((old & kSymMoved) || code != (old & 63u) ? kSymMoved : 0u);
+// An operand's symbol keeps the register it was read into, and is no longer swapped.
+PTL_HD void lane_store(const LaneSlot& L, const LaneRing& r, uint32_t i, uint32_t d, uint32_t old, uint32_t code) {
     const uint32_t idx = i - d;
-    if (d < r.K) r.at[(idx & (r.K - 1u)) * r.stride] = static_cast<uint8_t>(now);
-    if ((now ^ old) & 63u) L.symreg[idx] = reg_of(code);
-    if ((now ^ old) & kSymSwapped) L.symswp[idx] = swapped ? 0xFFFFFFFFu : 0u;
+    if (d < r.K)
+        r.at[(idx & (r.K - 1u)) * r.stride] =
+            static_cast<uint8_t>(code | ((old & kSymMoved) || code != (old & 63u) ? kSymMoved : 0u));
+    L.symreg[idx] = reg_of(code);
+    if (old & kSymSwapped) L.symswp[idx] = 0;
 }
 
-// Phase B: symbols, marks and row 0 after the step (a slot whose function has ended takes
-// part while row 0 has symbols of it).  m: the masks over all slots; others: positions the
-// independent functions trigger.
-template <bool kAlone>
-PTL_HD void lane_step_b(LaneShared& sh, const LaneStep& st, const LaneMasks& m, const LaneAbove& ab, uint32_t others,
-                        LaneSlot& L, const LaneRing& r, uint32_t i) {
+// Phase B, first part: the symbols after the step, but for swaps.  again: after the
+// allocation has changed.
+PTL_HD void lane_step_b1(LaneSlot& L, const LaneRing& r, uint32_t i, bool again) {
     const uint32_t hi = static_cast<uint32_t>(L.rec >> 32);
     const uint32_t d1 = step_d1(L.rec), d2 = step_d2(L.rec);
-    L.live = L.o.live;
     const bool def = (hi & (kStepDef | kStepSelf)) == kStepDef;
     r.at[(i & (r.K - 1u)) * r.stride] =
         static_cast<uint8_t>((def ? L.o.rd : kCodeNone) | ((hi & kStepSelf) ? kSymMoved : 0u));
     if (def) L.symreg[i] = L.o.rd ? L.o.rd : 37u;
-    // an operand's symbol keeps the register it was read into, swapped only when a later
-    // group triggers its row-0 position in this step
+    const bool s1 = d1 && d1 != d2 && (L.e1 != L.c1 || again), s2 = d2 && (L.e2 != L.c2 || again);
+    if (warp_any(s1 || s2)) {
+        if (s1) lane_store(L, r, i, d1, L.e1, L.c1);
+        if (s2) lane_store(L, r, i, d2, L.e2, L.c2);
+    }
+}
+
+// Swapped symbols at the positions of t leave row 0.
+PTL_HD void lane_leave(const LaneShared& sh, const LaneSlot& L, const LaneRing& r, uint32_t i, uint32_t t) {
+    do {  // seldom more than one
+        if (t) {
+            const uint32_t idx = sh.oidx[low_bit(t)];
+            t &= t - 1;
+            L.symswp[idx] = 0xFFFFFFFFu;
+            if (i - idx < r.K) r.at[(idx & (r.K - 1u)) * r.stride] |= kSymSwapped;
+        }
+    } while (PTL_RARE(warp_any(t != 0)));
+}
+
+// Phase B, second part: swaps and row 0 after the step (a slot whose function has ended
+// takes part while row 0 has symbols of it).  m: the masks over all slots; others:
+// positions the independent functions trigger.
+template <bool kAlone>
+PTL_HD void lane_step_b2(LaneShared& sh, const LaneStep& st, const LaneMasks& m, const LaneAbove& ab, uint32_t others,
+                         LaneSlot& L, const LaneRing& r, uint32_t i) {
+    const uint32_t hi = static_cast<uint32_t>(L.rec >> 32);
+    L.live = L.o.live;
+    // a symbol in row 0 that the slot reads ends swapped only when a later group triggers
+    // its position in this step; one that it does not read, when any function does
     bool l1 = L.l1, l2 = L.l2;
     if (!kAlone) {
         const uint32_t later = st.later | ab.trig;
@@ -457,22 +484,9 @@ PTL_HD void lane_step_b(LaneShared& sh, const LaneStep& st, const LaneMasks& m, 
         l2 = l2 || (L.m2 & later) != 0;
     }
     const uint32_t operands = L.m1 | L.m2;
-    L.marked = (L.marked & ~operands) | (l1 ? L.m1 : 0u) | (l2 ? L.m2 : 0u);
-    const bool s1 = d1 && d1 != d2 && (L.e1 != L.c1 || l1), s2 = d2 && (L.e2 != L.c2 || l2);
-    if (warp_any(s1 || s2)) {
-        if (s1) lane_store(L, r, i, d1, L.e1, L.c1, l1);
-        if (s2) lane_store(L, r, i, d2, L.e2, L.c2, l2);
-    }
-    uint32_t t = L.held & ~L.marked & ~operands & (others | m.trig);
-    L.marked |= t;
-    while (warp_any(t != 0)) {
-        if (t) {
-            const uint32_t idx = sh.oidx[low_bit(t)];
-            t &= t - 1;
-            L.symswp[idx] = 0xFFFFFFFFu;
-            if (i - idx < r.K) r.at[(idx & (r.K - 1u)) * r.stride] |= kSymSwapped;
-        }
-    }
+    L.marked = (L.marked & ~operands) | (l1 ? L.m1 : 0u) | (l2 ? L.m2 : 0u) | (L.held & ~operands & (others | m.trig));
+    const uint32_t leave = L.marked & m.wr;
+    if (warp_any(leave != 0)) lane_leave(sh, L, r, i, leave);
     L.held &= ~m.wr;
     L.marked &= L.held;
     const uint32_t bit = code_bit(L.o.rd);
@@ -487,7 +501,7 @@ PTL_HD void lane_step_b(LaneShared& sh, const LaneStep& st, const LaneMasks& m, 
 // After the last lane-0 function's last step: the remaining steps only mark the symbols
 // that row 0 holds at positions an independent function triggers (tail: those positions).
 PTL_HD void lane_tail(const LaneShared& sh, const LaneSlot& L, uint32_t tail) {
-    for (uint32_t m = L.held & ~L.marked & tail; m; m &= m - 1) L.symswp[sh.oidx[low_bit(m)]] = 0xFFFFFFFFu;
+    for (uint32_t m = L.held & (L.marked | tail); m; m &= m - 1) L.symswp[sh.oidx[low_bit(m)]] = 0xFFFFFFFFu;
 }
 
 }  // namespace ptl
