@@ -9,17 +9,26 @@
 // root) and its place among the parent's children is child_idx[v].
 //
 // The walk becomes an Euler tour and a list ranking:
-//   1. children per node (counts, an exclusive scan, each child in its slot
-//      off[parent] + child_idx: a child index out of range or taken twice is an error);
-//   2. the tour: events enter(v) = 2v and exit(v) = 2v+1, plus an end event 2n.  enter(v)
+//   1. children per node (the greatest child index + 1; their sum must be n - 1), an
+//      exclusive scan, each child in its slot off[parent] + child_idx: a child index out
+//      of range or taken twice, or a slot left empty, is an error;
+//   2. the tour: events enter(v) = 2v and exit(v) = 2v+1, and an end event 2n.  enter(v)
 //      goes to enter(first child) or exit(v); exit(v) to enter(next sibling), exit(parent)
 //      or, for the root, the end;
-//   3. pointer jumping, ceil(log2(2n+1)) rounds: each event sums two weights over the rest
-//      of the tour -- 1 per exit (post-order: v's index is n minus the exits from exit(v)
-//      on) and +1 per enter / -1 per exit (depth: minus the sum from enter(v) on);
-//   4. the scatter of the six arrays to post-order.
+//   3. the ranking by splitters: one enter in 8 or 16 (by a hash of the node) and the root's.
+//      A thread per splitter walks the tour to the next splitter and sums two weights --
+//      1 per exit (post-order: v's index is n minus the exits from exit(v) on) and +1 per
+//      enter / -1 per exit (depth); pointer jumping sums them over the splitters to the
+//      end; a second walk gives every node its index and depth;
+//   4. the six arrays in post-order.
 // The root's enter must see all n exits; fewer means nodes the root does not reach (a
 // cycle of parents), an INVALID_AST.  No kernel waits on another block.
+//
+// What bounds it: random 4-byte reads of the tour out of L2, twice, by dependent chains of
+// some 16 to 32 events (the longest, about ln(splitters) times that, ends last).  4.3M
+// nodes on the device: 0.90 ms; pointer jumping over all events, which read and wrote 32
+// bytes per event in each of 24 rounds, with a same-address atomic per node for the depth
+// and per child for the counts, took 4.1 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -35,20 +44,33 @@ constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kScanThreads = 1024;
 constexpr uint32_t kScanTile = 4096;  // elements per scan tile (4 per thread)
 
-struct Event {
-    uint32_t succ;  // next event of the tour (2n: the end)
-    uint32_t exits; // exits from here to the end
-    int32_t level;  // enters minus exits from here to the end
+struct Rank {
+    uint32_t next;  // splitter further on (count: the end)
+    uint32_t exits; // exits from here up to there
+    int32_t level;  // enters minus exits
     uint32_t pad;
 };
+
+// A node's inputs, one sector of a random read.
+struct NodeRec {
+    int32_t parent, child;
+    uint32_t data, types;
+};
+
+// Whether enter(v) is a splitter (besides the root's): one node in 2^lg, spread evenly over
+// any run of consecutive nodes (multiplicative hashing by the golden ratio).
+__host__ __device__ __forceinline__ bool is_splitter(uint32_t v, uint32_t lg) {
+    return ((v * 0x9E3779B1u) >> (32u - lg)) == 0;
+}
 
 struct FlatErr {
     uint32_t code;     // 0 ok, 1 invalid
     uint32_t detail;   // the first node found bad
     uint32_t roots;    // nodes with parent -1
-    uint32_t root;     // one of them
     uint32_t max_depth;
     uint32_t reached;  // exits the root's enter sees
+    uint32_t splitters;
+    unsigned long long slots;  // sum of the children counts
 };
 
 __device__ void flag(FlatErr* e, uint32_t v) {
@@ -64,17 +86,24 @@ unsigned grid_of(uint64_t n) {
     return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((n + kThreads - 1) / kThreads, 152u * 16u)));
 }
 
-// children per node; the root
-__global__ void k_fl_count(const int32_t* parent, const int32_t* child, uint32_t n, uint32_t* deg, FlatErr* e) {
+// one thread per splitter: the walks are latency-bound
+unsigned walk_grid(uint64_t n) { return static_cast<unsigned>(std::max<uint64_t>(1, (n + kThreads - 1) / kThreads)); }
+
+// children per node (greatest child index + 1); the root; the nodes' records.  deg is
+// read before it is raised: with the children of a node in any order few of them raise
+// it, and a node with many children (a function or statement list) would serialise one
+// atomic per child (430k children of a root: 300 us).
+__global__ void k_fl_count(const int32_t* parent, const int32_t* child, const uint32_t* data, const uint8_t* type,
+                           const uint8_t* rtype, uint32_t n, uint32_t* deg, NodeRec* rec, FlatErr* e) {
     FL_FOR(v, n) {
-        const int32_t p = parent[v];
+        const int32_t p = parent[v], c = child[v];
+        rec[v] = NodeRec{p, c, data[v], type[v] | static_cast<uint32_t>(rtype[v]) << 8};
         if (p == -1) {
             atomicAdd(&e->roots, 1u);
-            e->root = v;
-        } else if (p < 0 || static_cast<uint32_t>(p) >= n || child[v] < 0) {
+        } else if (p < 0 || static_cast<uint32_t>(p) >= n || c < 0 || static_cast<uint32_t>(c) >= n) {
             flag(e, v);
-        } else {
-            atomicAdd(&deg[p], 1u);
+        } else if (deg[p] <= static_cast<uint32_t>(c)) {
+            atomicMax(&deg[p], static_cast<uint32_t>(c) + 1u);
         }
     }
 }
@@ -108,18 +137,29 @@ __device__ uint32_t block_excl(uint32_t x, uint32_t* total) {
     return r;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_fl_tile_sums(const uint32_t* deg, uint32_t n, uint32_t* tsum) {
+__global__ void __launch_bounds__(kScanThreads) k_fl_tile_sums(const uint32_t* deg, uint32_t n, uint32_t* tsum,
+                                                               FlatErr* e) {
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kScanTile;
-    uint32_t s = 0;
+    unsigned long long s = 0;  // the counts of a malformed input may add up past 32 bits
     for (uint32_t k = threadIdx.x; k < kScanTile; k += kScanThreads)
         if (base + k < n) s += deg[base + k];
+    __shared__ unsigned long long wide;
     __shared__ uint32_t total;
-    block_excl(s, &total);
-    if (threadIdx.x == 0) tsum[blockIdx.x] = total;
+    if (threadIdx.x == 0) wide = 0;
+    block_excl(static_cast<uint32_t>(s), &total);  // its barriers publish wide
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_down_sync(0xFFFFFFFFu, s, d);
+    if ((threadIdx.x & 31u) == 0 && s) atomicAdd(&wide, s);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        tsum[blockIdx.x] = total;
+        if (wide) atomicAdd(&e->slots, wide);
+    }
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_fl_scan_sums(uint32_t* tsum, uint32_t tiles) {
+__global__ void __launch_bounds__(kScanThreads) k_fl_scan_sums(uint32_t* tsum, uint32_t tiles, uint32_t n, FlatErr* e) {
     __shared__ uint32_t total;
+    if (threadIdx.x == 0 && e->slots != n - 1u) flag(e, 0);  // a gap in some node's child indices
     uint32_t carry = 0;
     for (uint32_t b = 0; b < tiles; b += kScanThreads) {
         const uint32_t k = b + threadIdx.x;
@@ -152,81 +192,145 @@ __global__ void __launch_bounds__(kScanThreads) k_fl_tiles(const uint32_t* deg, 
     }
 }
 
-// each child into its slot
-__global__ void k_fl_place(const int32_t* parent, const int32_t* child, uint32_t n, const uint32_t* deg,
-                           const uint32_t* off, uint32_t* kids, FlatErr* e) {
+__device__ __forceinline__ bool bad(const FlatErr* e) { return *reinterpret_cast<const volatile uint32_t*>(&e->code) != 0; }
+
+// each child into its slot (the counts add up to n - 1, so every slot is in range)
+__global__ void k_fl_place(const NodeRec* rec, uint32_t n, const uint32_t* deg, const uint32_t* off, uint32_t* kids,
+                           FlatErr* e) {
+    if (bad(e)) return;
     FL_FOR(v, n) {
-        const int32_t p = parent[v];
-        if (p < 0 || static_cast<uint32_t>(p) >= n || child[v] < 0) continue;  // the root, or flagged
-        const uint32_t c = static_cast<uint32_t>(child[v]);
-        if (c >= deg[p] || atomicCAS(&kids[off[p] + c], kEmpty, v) != kEmpty) flag(e, v);
+        const int2 r = *reinterpret_cast<const int2*>(&rec[v]);  // parent, child
+        if (r.x < 0) continue;  // the root
+        const uint32_t c = static_cast<uint32_t>(r.y);
+        if (c >= deg[r.x] || atomicCAS(&kids[off[r.x] + c], kEmpty, v) != kEmpty) flag(e, v);
     }
 }
 
-// the tour's events; an unfilled slot (flagged input) ends the tour there
-__global__ void k_fl_tour(const int32_t* parent, const int32_t* child, uint32_t n, const uint32_t* deg,
-                          const uint32_t* off, const uint32_t* kids, Event* ev) {
+// The tour (successors of enter(v) and exit(v)), and the splitters in any order: split[k]
+// is splitter k's node, sidx its k.  From here on the input is flagged or every slot holds
+// one child, so no two events have the same successor but the end.
+__global__ void k_fl_tour(const NodeRec* rec, uint32_t n, const uint32_t* deg, const uint32_t* off,
+                          const uint32_t* kids, uint32_t lg, uint2* succ, uint32_t* split, uint32_t cap, uint32_t* sidx,
+                          FlatErr* e) {
+    if (bad(e)) return;
     const uint32_t end = 2u * n;
     FL_FOR(v, n) {
+        const int2 r = *reinterpret_cast<const int2*>(&rec[v]);  // parent, child
         uint32_t s = 2u * v + 1u;  // enter(v) -> exit(v) for a leaf
         if (deg[v] > 0) {
             const uint32_t c = kids[off[v]];
             s = c < n ? 2u * c : end;
         }
-        ev[2u * v] = Event{s, 0u, 1, 0u};
-        const int32_t p = parent[v];
         uint32_t x = end;  // exit(root) -> the end
-        if (p >= 0 && static_cast<uint32_t>(p) < n && child[v] >= 0) {
-            const uint32_t c = static_cast<uint32_t>(child[v]) + 1u;
-            if (c < deg[p]) {
-                const uint32_t sib = kids[off[p] + c];
+        if (r.x >= 0) {
+            const uint32_t c = static_cast<uint32_t>(r.y) + 1u;
+            if (c < deg[r.x]) {
+                const uint32_t sib = kids[off[r.x] + c];
                 x = sib < n ? 2u * sib : end;
             } else {
-                x = 2u * static_cast<uint32_t>(p) + 1u;
+                x = 2u * static_cast<uint32_t>(r.x) + 1u;
             }
         }
-        ev[2u * v + 1u] = Event{x, 1u, -1, 0u};
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) ev[end] = Event{end, 0u, 0, 0u};
-}
-
-// one round of pointer jumping
-__global__ void k_fl_jump(const Event* __restrict__ in, Event* __restrict__ out, uint32_t events) {
-    FL_FOR(x, events) {
-        const Event a = in[x];
-        const Event b = in[a.succ];
-        out[x] = Event{b.succ, a.exits + b.exits, a.level + b.level, 0u};
-    }
-}
-
-// post-order index and depth of every node
-__global__ void k_fl_rank(const Event* ev, uint32_t n, int32_t* post, FlatErr* e) {
-    FL_FOR(v, n) {
-        const uint32_t q = n - ev[2u * v + 1u].exits;
-        if (q >= n) flag(e, v);  // a node the root does not reach
-        post[v] = static_cast<int32_t>(q);
-        const int32_t d = -ev[2u * v].level;
-        if (d >= 0) atomicMax(&e->max_depth, static_cast<uint32_t>(d));
-        if (v == e->root && e->roots == 1u) e->reached = ev[2u * v].exits;
+        succ[v] = make_uint2(s, x);
+        if (r.x < 0 || is_splitter(v, lg)) {
+            const uint32_t k = atomicAdd(&e->splitters, 1u);
+            if (k < cap) {
+                split[k] = v;
+                sidx[v] = k;
+            } else {
+                flag(e, v);  // several roots
+            }
+        }
     }
 }
 
-__global__ void k_fl_scatter(const uint8_t* type, const uint8_t* rtype, const int32_t* parent, const int32_t* child,
-                             const uint32_t* data, uint32_t n, const int32_t* post, const Event* ev, uint8_t* o_type,
-                             uint8_t* o_rtype, int32_t* o_parent, int32_t* o_depth, int32_t* o_child,
-                             uint32_t* o_data, int32_t* order) {
-    FL_FOR(v, n) {
-        const int32_t q = post[v];
-        if (q < 0 || static_cast<uint32_t>(q) >= n) continue;
-        const int32_t p = parent[v];
-        const bool ok_p = p >= 0 && static_cast<uint32_t>(p) < n;
-        o_type[q] = type[v];
-        o_rtype[q] = rtype[v];
-        o_parent[q] = ok_p ? post[p] : -1;
-        o_depth[q] = -ev[2u * v].level;
-        o_child[q] = ok_p ? child[v] : -1;
-        o_data[q] = data[v];
-        if (order) order[v] = q;
+// From each splitter to the next: how far, and to which.  The walk ends: no two events
+// share a successor, so it leads to the end or back to a splitter.
+__global__ void k_fl_walk(const uint32_t* succ, const uint32_t* split, const uint32_t* sidx,
+                          uint32_t n, uint32_t lg, Rank* rank, FlatErr* e) {
+    if (bad(e)) return;
+    const uint32_t count = e->splitters, end = 2u * n;
+    FL_FOR(k, count) {
+        uint32_t x = 2u * split[k], exits = 0;
+        int32_t level = 0;
+        uint32_t next = count;
+        for (;;) {
+            exits += x & 1u;
+            level += (x & 1u) ? -1 : 1;
+            x = succ[x];
+            if (x == end) break;
+            if (!(x & 1u) && is_splitter(x >> 1, lg)) {  // the root's enter follows nothing
+                next = sidx[x >> 1];
+                break;
+            }
+        }
+        rank[k] = Rank{next, exits, level, 0u};
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) rank[count] = Rank{count, 0u, 0, 0u};
+}
+
+// one round of pointer jumping over the splitters
+__global__ void k_fl_jump(const Rank* __restrict__ in, Rank* __restrict__ out, const FlatErr* e) {
+    if (bad(e)) return;
+    FL_FOR(k, static_cast<uint64_t>(e->splitters) + 1u) {
+        const uint4 a = reinterpret_cast<const uint4*>(in)[k];
+        const uint4 b = reinterpret_cast<const uint4*>(in)[a.x];
+        reinterpret_cast<uint4*>(out)[k] = make_uint4(b.x, a.y + b.y, a.z + b.z, 0u);
+    }
+}
+
+// The walks again, with what lies behind each splitter known: every node's post-order
+// index (post), and by index its node and depth (at).
+__global__ void k_fl_number(const uint32_t* succ, const NodeRec* rec, const uint32_t* split, uint32_t n, uint32_t lg,
+                            const Rank* rank, int32_t* post, uint2* at, FlatErr* e) {
+    if (bad(e)) return;
+    const uint32_t count = e->splitters, end = 2u * n;
+    uint32_t deepest = 0;
+    FL_FOR(k, count) {
+        uint32_t x = 2u * split[k];
+        uint32_t exits = rank[k].exits;  // from x to the end
+        int32_t level = rank[k].level;
+        if (rec[x >> 1].parent == -1) e->reached = exits;
+        for (;;) {
+            if (x & 1u) {
+                const uint32_t v = x >> 1, q = n - exits;
+                const int32_t depth = -(level + 1);
+                if (q < n) {
+                    post[v] = static_cast<int32_t>(q);
+                    at[q] = make_uint2(v, static_cast<uint32_t>(depth));
+                }
+                if (depth > 0) deepest = max(deepest, static_cast<uint32_t>(depth));
+                --exits;
+                ++level;
+            } else {
+                --level;
+            }
+            x = succ[x];
+            if (x == end || (!(x & 1u) && is_splitter(x >> 1, lg))) break;
+        }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) deepest = max(deepest, __shfl_down_sync(0xFFFFFFFFu, deepest, d));
+    if ((threadIdx.x & 31u) == 0 && deepest) atomicMax(&e->max_depth, deepest);
+}
+
+// The outputs in post-order: coalesced but for one read of the node's record and one of
+// its parent's index.
+__global__ void k_fl_emit(const NodeRec* rec, uint32_t n, const int32_t* post, const uint2* at, uint8_t* o_type,
+                          uint8_t* o_rtype, int32_t* o_parent, int32_t* o_depth, int32_t* o_child, uint32_t* o_data,
+                          int32_t* order, const FlatErr* e) {
+    if (bad(e) || e->roots != 1u || e->reached != n) return;
+    FL_FOR(q, n) {
+        const uint2 a = at[q];
+        const uint4 r = reinterpret_cast<const uint4*>(rec)[a.x];
+        const int32_t p = static_cast<int32_t>(r.x);
+        o_type[q] = static_cast<uint8_t>(r.w);
+        o_rtype[q] = static_cast<uint8_t>(r.w >> 8);
+        o_parent[q] = p >= 0 ? post[p] : -1;
+        o_depth[q] = static_cast<int32_t>(a.y);
+        o_child[q] = p >= 0 ? static_cast<int32_t>(r.y) : -1;
+        o_data[q] = r.z;
+        if (order) order[q] = post[q];  // q as a node here
     }
 }
 
@@ -260,11 +364,17 @@ extern "C" ptl_status ptl_flatten(const ptl_tree_view* in, ptl_depth_tree_out* o
     uint8_t* out_bytes = nullptr;  // staged outputs (host views): 22 bytes per node
     uint32_t *deg = nullptr, *off = nullptr, *kids = nullptr, *tsum = nullptr;
     int32_t* post = nullptr;
-    Event *ev0 = nullptr, *ev1 = nullptr;
+    NodeRec* rec = nullptr;
+    uint2 *succ = nullptr, *at = nullptr;
+    uint32_t *split = nullptr, *sidx = nullptr;
+    Rank *rank0 = nullptr, *rank1 = nullptr;
     FlatErr* err = nullptr;
     FlatErr herr{};
     const uint32_t tiles = static_cast<uint32_t>((n64 + 1 + kScanTile - 1) / kScanTile);
-    const uint32_t events = 2u * n + 1u;
+    // A splitter per 16 nodes of a large tree, per 8 of a small one (whose walks are over
+    // sooner than the jumps between more splitters cost).
+    const uint32_t lg = n >= (1u << 20) ? 4u : 3u;
+    const uint32_t cap = (n >> lg) + (n >> (lg + 2u)) + 64u;
     ptl_status st = PTL_OK;
     cudaError_t ce = cudaSuccess;
 #define FL_CU(x)                       \
@@ -302,30 +412,34 @@ extern "C" ptl_status ptl_flatten(const ptl_tree_view* in, ptl_depth_tree_out* o
     FL_CU(dev_alloc(&kids, n64, s));
     FL_CU(dev_alloc(&tsum, tiles, s));
     FL_CU(dev_alloc(&post, n64, s));
-    FL_CU(dev_alloc(&ev0, events, s));
-    FL_CU(dev_alloc(&ev1, events, s));
+    FL_CU(dev_alloc(&rec, n64, s));
+    FL_CU(dev_alloc(&succ, n64, s));
+    FL_CU(dev_alloc(&at, n64, s));
+    FL_CU(dev_alloc(&split, cap, s));
+    FL_CU(dev_alloc(&sidx, n64, s));
+    FL_CU(dev_alloc(&rank0, cap + 1u, s));
+    FL_CU(dev_alloc(&rank1, cap + 1u, s));
     FL_CU(dev_alloc(&err, 1, s));
     FL_CU(cudaMemsetAsync(deg, 0, 4 * n64, s));
     FL_CU(cudaMemsetAsync(kids, 0xFF, 4 * n64, s));
     FL_CU(cudaMemsetAsync(err, 0, sizeof(FlatErr), s));
 
-    k_fl_count<<<grid_of(n), kThreads, 0, s>>>(d_parent, d_child, n, deg, err);
-    k_fl_tile_sums<<<tiles, kScanThreads, 0, s>>>(deg, n, tsum);
-    k_fl_scan_sums<<<1, kScanThreads, 0, s>>>(tsum, tiles);
+    k_fl_count<<<grid_of(n), kThreads, 0, s>>>(d_parent, d_child, d_data, d_type, d_rtype, n, deg, rec, err);
+    k_fl_tile_sums<<<tiles, kScanThreads, 0, s>>>(deg, n, tsum, err);
+    k_fl_scan_sums<<<1, kScanThreads, 0, s>>>(tsum, tiles, n, err);
     k_fl_tiles<<<tiles, kScanThreads, 0, s>>>(deg, n, tsum, off);
-    k_fl_place<<<grid_of(n), kThreads, 0, s>>>(d_parent, d_child, n, deg, off, kids, err);
-    k_fl_tour<<<grid_of(n), kThreads, 0, s>>>(d_parent, d_child, n, deg, off, kids, ev0);
-    {
-        uint32_t rounds = 0;
-        while ((1ull << rounds) < events) ++rounds;
-        for (uint32_t r = 0; r < rounds; ++r) {
-            k_fl_jump<<<grid_of(events), kThreads, 0, s>>>(ev0, ev1, events);
-            std::swap(ev0, ev1);
-        }
+    k_fl_place<<<grid_of(n), kThreads, 0, s>>>(rec, n, deg, off, kids, err);
+    k_fl_tour<<<grid_of(n), kThreads, 0, s>>>(rec, n, deg, off, kids, lg, succ, split, cap, sidx, err);
+    k_fl_walk<<<walk_grid(cap), kThreads, 0, s>>>(reinterpret_cast<const uint32_t*>(succ), split, sidx, n, lg, rank0,
+                                                  err);
+    for (uint32_t r = 0; (1ull << r) < cap + 1ull; ++r) {
+        k_fl_jump<<<grid_of(cap), kThreads, 0, s>>>(rank0, rank1, err);
+        std::swap(rank0, rank1);
     }
-    k_fl_rank<<<grid_of(n), kThreads, 0, s>>>(ev0, n, post, err);
-    k_fl_scatter<<<grid_of(n), kThreads, 0, s>>>(d_type, d_rtype, d_parent, d_child, d_data, n, post, ev0, o_type,
-                                                 o_rtype, o_parent, o_depth, o_child, o_data, o_order);
+    k_fl_number<<<walk_grid(cap), kThreads, 0, s>>>(reinterpret_cast<const uint32_t*>(succ), rec, split, n, lg, rank0,
+                                                    post, at, err);
+    k_fl_emit<<<grid_of(n), kThreads, 0, s>>>(rec, n, post, at, o_type, o_rtype, o_parent, o_depth, o_child, o_data,
+                                              o_order, err);
     FL_CU(cudaGetLastError());
     FL_CU(cudaMemcpyAsync(&herr, err, sizeof(herr), cudaMemcpyDeviceToHost, s));
     if (!out->on_device) {
@@ -344,8 +458,9 @@ done:
 #undef FL_CU
     for (void* p : {static_cast<void*>(in_bytes), static_cast<void*>(out_bytes), static_cast<void*>(deg),
                     static_cast<void*>(off), static_cast<void*>(kids), static_cast<void*>(tsum),
-                    static_cast<void*>(post), static_cast<void*>(ev0), static_cast<void*>(ev1),
-                    static_cast<void*>(err)})
+                    static_cast<void*>(post), static_cast<void*>(rec), static_cast<void*>(succ),
+                    static_cast<void*>(at), static_cast<void*>(split), static_cast<void*>(sidx),
+                    static_cast<void*>(rank0), static_cast<void*>(rank1), static_cast<void*>(err)})
         if (p) cudaFreeAsync(p, s);
     if (ce != cudaSuccess) {
         cudaStreamSynchronize(s);

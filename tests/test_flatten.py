@@ -174,3 +174,48 @@ def test_gpu_flatten_on_device_then_compile(built_cuda):
     with RvGenerator(flat) as g:
         g.process()
         np.testing.assert_array_equal(g.get_instructions(), compile_tree(t))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 7, 8, 9, 255, 4097, (1 << 20) - 1, 1 << 20])
+def test_gpu_flatten_splitter_walks(built_cuda, n):
+    """Random trees with and without long runs between splitters, at the sizes where the
+    splitters' spacing changes: nodes in post-order, reversed and shuffled.  The tree is
+    built in post-order, so the expected arrays are its own."""
+    from ptilopsis_gb300 import flatten
+    rng = np.random.default_rng(n)
+    # a random recursive tree numbered from the root, then its post-order by one sweep
+    up = np.zeros(n, np.int64)
+    up[1:] = np.maximum(np.arange(1, n) - 1 - rng.integers(0, np.minimum(np.arange(1, n), 40)), 0)
+    up[0] = -1
+    size = np.ones(n, np.int64)
+    for v in range(n - 1, 0, -1):
+        size[up[v]] += size[v]
+    nth, used, first = np.zeros(n, np.int64), np.zeros(n, np.int64), np.zeros(n, np.int64)
+    count, depth = np.zeros(n, np.int64), np.zeros(n, np.int64)
+    for v in range(1, n):  # children in number order; first: post-order index where v's subtree begins
+        p = up[v]
+        nth[v], count[p] = count[p], count[p] + 1
+        first[v] = first[p] + used[p]
+        used[p] += size[v]
+        depth[v] = depth[p] + 1
+    post = first + size - 1
+    parent, child = np.empty(n, np.int32), np.empty(n, np.int32)
+    parent[post] = np.where(up >= 0, post[np.maximum(up, 0)], -1)
+    child[post] = np.where(up >= 0, nth, -1)
+    type_, rtype = rng.integers(0, 40, n).astype(np.uint8), rng.integers(0, 6, n).astype(np.uint8)
+    data = rng.integers(0, 1 << 32, n, dtype=np.uint64).astype(np.uint32)
+    for at in (np.arange(n), np.arange(n)[::-1], rng.permutation(n)):  # node q goes to at[q]
+        arrs = []
+        for a in (type_, rtype, np.where(parent >= 0, at[np.maximum(parent, 0)], -1).astype(np.int32), child, data):
+            b = np.empty_like(a)
+            b[at] = a
+            arrs.append(b)
+        tree, order = flatten(*arrs)
+        for name, want in (("type", type_), ("rtype", rtype), ("parent", parent), ("child_idx", child), ("data", data)):
+            np.testing.assert_array_equal(getattr(tree, name), want, err_msg=name)
+        want_depth = np.empty(n, np.int32)
+        want_depth[post] = depth
+        np.testing.assert_array_equal(tree.depth, want_depth)
+        np.testing.assert_array_equal(order[at], np.arange(n))
+        assert tree.max_depth == depth.max()
