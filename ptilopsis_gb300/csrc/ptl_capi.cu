@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstdint>
 #include <initializer_list>
 #include <cstdio>
@@ -55,6 +56,7 @@ struct DevBuf {
         return cudaSuccess;
     }
     cudaError_t zero(cudaStream_t s) const { return base ? cudaMemsetAsync(base, 0, (count + kFrontPad + kBackPad) * elem, s) : cudaSuccess; }
+    void zero(ZeroList& z) const { if (base) z.add(base, (count + kFrontPad + kBackPad) * elem); }
     cudaError_t fill(cudaStream_t s, int byte) const { return base ? cudaMemsetAsync(base, byte, (count + kFrontPad + kBackPad) * elem, s) : cudaSuccess; }
     void release() { if (base) cudaFreeAsync(base, s); base = nullptr; bytes = 0; }
     // elements the allocation holds (at least the last ensure's n)
@@ -100,9 +102,22 @@ struct ptl_generator {
     DevBuf ni, nrd, nr1, nr2, njt, fsz, joffs, out;
     DevBuf sort_a, sort_apos, sort_bpos, sort_seg0, sort_seg1, sort_tile_seg, sort_tile_l, sort_tile_r, sort_stops,
         sort_leaf, sort_heap, sort_counters, sort_local, sort_equal;
-    DevBuf scan_status, scan_counter, meta, flags, errw, tables;
+    DevBuf scan_status, meta, flags, errw, tables;
     DevBuf preserve, sregs, ssteps, sextra, sclaim;  // scalar register allocation
     bool scalar = false;  // the scalar generator's semantics (rv_generator_st)
+
+    // Pinned host memory for read-backs (a copy to pageable memory waits for the stream by
+    // itself, so several of them are several waits): the error word and a few sizes, then
+    // room for small results.
+    static constexpr size_t kPinnedResults = size_t(256) << 10;
+    struct Pinned {
+        ErrorWord err;
+        uint32_t v[12];
+        alignas(16) unsigned char results[kPinnedResults];
+    };
+    Pinned* pinned = nullptr;
+    cudaError_t take_pinned();
+    void give_pinned();
 
     // results
     uint32_t F = 0, W = 0, W2 = 0, W3 = 0, S = 0;
@@ -116,6 +131,7 @@ struct ptl_generator {
     ~ptl_generator() {
         for (DevBuf* b : all()) b->release();
         if (stream) cudaStreamDestroy(stream);
+        give_pinned();
     }
     // The buffers allocate and free in this generator's stream order (after it exists).
     void bind_stream() {
@@ -129,10 +145,49 @@ struct ptl_generator {
                 &stamp, &defpos, &lifetime, &trig_min, &trig_max, &ra_chunks, &spill, &roffs, &ni, &nrd, &nr1, &nr2, &njt,
                 &fsz, &joffs, &out, &sort_a, &sort_apos, &sort_bpos, &sort_seg0, &sort_seg1, &sort_stops,
                 &sort_tile_seg, &sort_tile_l, &sort_tile_r, &sort_leaf, &sort_heap, &sort_counters, &sort_local, &sort_equal,
-                &scan_status, &scan_counter, &meta, &flags, &errw, &tables, &preserve, &sregs, &ssteps,
+                &scan_status, &meta, &flags, &errw, &tables, &preserve, &sregs, &ssteps,
                 &sextra, &sclaim};
     }
 };
+
+// Pinning memory takes longer than a small compile, and programs make a generator per
+// compile (ptl_compile): up to kPinnedKept blocks wait here for the next generator, on any
+// thread and device; more are freed.
+namespace {
+constexpr size_t kPinnedKept = 8;
+std::mutex pinned_mu;
+std::vector<ptl_generator::Pinned*>& pinned_kept() {
+    static std::vector<ptl_generator::Pinned*> kept;
+    return kept;
+}
+}  // namespace
+cudaError_t ptl_generator::take_pinned() {
+    {
+        std::lock_guard<std::mutex> lk(pinned_mu);
+        auto& kept = pinned_kept();
+        if (!kept.empty()) {
+            pinned = kept.back();
+            kept.pop_back();
+            return cudaSuccess;
+        }
+    }
+    return cudaHostAlloc(reinterpret_cast<void**>(&pinned), sizeof(Pinned), cudaHostAllocPortable);
+}
+// After the stream's last use of it.
+void ptl_generator::give_pinned() {
+    if (!pinned) return;
+    {
+        std::lock_guard<std::mutex> lk(pinned_mu);
+        auto& kept = pinned_kept();
+        if (kept.size() < kPinnedKept) {
+            kept.push_back(pinned);
+            pinned = nullptr;
+            return;
+        }
+    }
+    cudaFreeHost(pinned);
+    pinned = nullptr;
+}
 
 namespace {
 
@@ -297,8 +352,9 @@ Prog make_prog(ptl_generator* g) {
     return P;
 }
 
+// Reads the error word (and waits for the stream, so for every copy issued before).
 ptl_status check_error_word(ptl_generator* g) {
-    ErrorWord e{};
+    ErrorWord& e = g->pinned->err;
     cudaError_t ce = cudaMemcpyAsync(&e, g->errw.at<ErrorWord>(), sizeof(e), cudaMemcpyDeviceToHost, g->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(g->stream);
     if (ce != cudaSuccess) return cuda_fail(g, ce, "error word");
@@ -315,11 +371,9 @@ ptl_status check_error_word(ptl_generator* g) {
     return fail(g, static_cast<ptl_status>(e.code), buf);
 }
 
-template <typename T>
-cudaError_t read1(ptl_generator* g, const T* dptr, T* out) {
-    cudaError_t e = cudaMemcpyAsync(out, dptr, sizeof(T), cudaMemcpyDeviceToHost, g->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-    return e;
+// Issues the copy of count words to the pinned read-back words at k.
+cudaError_t read_back(ptl_generator* g, const uint32_t* src, int k, size_t count = 1) {
+    return cudaMemcpyAsync(g->pinned->v + k, src, count * sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream);
 }
 
 struct StageTimer {
@@ -348,6 +402,65 @@ struct StageTimer {
         if (on) for (auto& e : ev) cudaEventDestroy(e);
     }
 };
+
+// The function table on the device, in the order of the host vectors.
+struct TablePart {
+    const DevBuf* from;
+    std::vector<uint32_t>* to;
+};
+std::array<TablePart, 4> table_parts(ptl_generator* g) {
+    return {{{&g->fn_start, &g->fn_start_h}, {&g->fn_end, &g->fn_end_h}, {&g->fn_size, &g->fn_size_h}, {&g->fn_id, &g->fn_id_h}}};
+}
+
+// The function table to the host, through the pinned results when it fits (one wait for
+// its four parts; a copy to pageable memory is a wait each).  used: bytes of the pinned
+// results taken already.  take_table after the stream has been waited for.
+cudaError_t copy_table(ptl_generator* g, size_t used = 0) {
+    const bool pinned = used + g->F * 16ull <= ptl_generator::kPinnedResults;
+    uint32_t* at = reinterpret_cast<uint32_t*>(g->pinned->results + used);
+    for (const TablePart& t : table_parts(g)) {
+        t.to->resize(g->F);
+        const cudaError_t e =
+            cudaMemcpyAsync(pinned ? at : t.to->data(), t.from->at<uint32_t>(), g->F * 4ull, cudaMemcpyDeviceToHost, g->stream);
+        if (e != cudaSuccess) return e;
+        at += g->F;
+    }
+    return cudaSuccess;
+}
+void take_table(ptl_generator* g, size_t used = 0) {
+    if (used + g->F * 16ull <= ptl_generator::kPinnedResults) {
+        const uint32_t* at = reinterpret_cast<const uint32_t*>(g->pinned->results + used);
+        for (const TablePart& t : table_parts(g)) {
+            std::copy(at, at + g->F, t.to->begin());
+            at += g->F;
+        }
+    }
+    g->table_valid = true;
+}
+
+// The words and the table; small words go through the pinned results too.
+size_t pinned_words(const ptl_generator* g) {
+    return g->W3 * 4ull <= ptl_generator::kPinnedResults / 2 ? g->W3 * 4ull : 0;
+}
+cudaError_t copy_results(ptl_generator* g) {
+    g->words.resize(g->W3);
+    cudaError_t e = cudaSuccess;
+    if (pinned_words(g))
+        e = cudaMemcpyAsync(g->pinned->results, g->out.at<uint32_t>(), g->W3 * 4ull, cudaMemcpyDeviceToHost, g->stream);
+    // Where the device accesses pageable memory coherently (ATS), kernel stores put the
+    // words straight into the vector; otherwise the copy engine stages them.
+    else if (g->W3 && pageable_paths(g->device).write && (reinterpret_cast<uintptr_t>(g->words.data()) & 15u) == 0)
+        e = kernel_copy(g->out.at<uint32_t>(), g->words.data(), g->W3 * 4ull, g->stream);
+    else if (g->W3)
+        e = cudaMemcpyAsync(g->words.data(), g->out.at<uint32_t>(), g->W3 * 4ull, cudaMemcpyDeviceToHost, g->stream);
+    return e == cudaSuccess ? copy_table(g, pinned_words(g)) : e;
+}
+void take_results(ptl_generator* g) {
+    const uint32_t* at = reinterpret_cast<const uint32_t*>(g->pinned->results);
+    if (pinned_words(g)) std::copy(at, at + g->W3, g->words.begin());
+    take_table(g, pinned_words(g));
+    g->words_valid = true;
+}
 
 // The depth sort's scratch for n keys (grown as needed), in ss.
 cudaError_t sort_scratch(ptl_generator* g, size_t n, SortScratch* ss) {
@@ -409,33 +522,25 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
     g->words_valid = g->table_valid = false;
     StageTimer timer(g, profile);
 
-    // fixed-size scratch first, so every Prog view below sees it
-    PTL_CU(g->flags.ensure(4, 4));
-    PTL_CU(g->flags.zero(s));
-    PTL_CU(g->errw.zero(s));
-    PTL_CU(g->meta.zero(s));
-    // node arrays
-    for (DevBuf* b : {&g->nt, &g->rt}) {
-        PTL_CU(b->ensure(nb8, 1));
-        PTL_CU(b->zero(s));
+    // fixed-size scratch and node arrays, cleared by one launch
+    {
+        PTL_CU(g->flags.ensure(4, 4));
+        for (DevBuf* b : {&g->nt, &g->rt, &g->fflag}) PTL_CU(b->ensure(nb8, 1));
+        for (DevBuf* b : {&g->nd1, &g->nd, &g->par, &g->ci, &g->dep, &g->sizes, &g->loc0, &g->loc, &g->pos, &g->decl})
+            PTL_CU(b->ensure(nb8, 4));
+        PTL_CU(g->regs.ensure(3 * n, 4));
+        ZeroList z;
+        for (const DevBuf* b : {&g->flags, &g->errw, &g->meta, &g->nt, &g->rt, &g->fflag, &g->nd1, &g->nd, &g->par, &g->ci,
+                                &g->dep, &g->sizes, &g->loc0, &g->loc, &g->pos, &g->decl, &g->regs})
+            b->zero(z);
+        PTL_CU(launch_zero(z, s));
     }
-    for (DevBuf* b : {&g->nd1, &g->nd, &g->par, &g->ci, &g->dep, &g->sizes, &g->loc0, &g->loc, &g->pos}) {
-        PTL_CU(b->ensure(nb8, 4));
-        PTL_CU(b->zero(s));
-    }
-    PTL_CU(g->fflag.ensure(nb8, 1));
-    PTL_CU(g->fflag.zero(s));
-    PTL_CU(g->decl.ensure(nb8, 4));
-    PTL_CU(g->decl.zero(s));
-    PTL_CU(g->regs.ensure(3 * n, 4));
-    PTL_CU(g->regs.zero(s));
-    PTL_CU(g->scan_counter.ensure(1, 4));
     // Tile-status scratch for a scan over `count` elements (grows with the word counts).
     auto scan_for = [&](size_t count, ScanScratch* sc) -> cudaError_t {
         const size_t tiles = (std::max(count, size_t(1)) + kScanTileElems - 1) / kScanTileElems + 8;
-        const cudaError_t e = g->scan_status.ensure(tiles, 8);
+        const cudaError_t e = g->scan_status.ensure(tiles + 1, 8);  // the ticket, then the status words
         if (e != cudaSuccess) return e;
-        *sc = ScanScratch{g->scan_status.at<unsigned long long>(), g->scan_counter.at<uint32_t>(),
+        *sc = ScanScratch{g->scan_status.at<unsigned long long>() + 1, g->scan_status.at<uint32_t>(),
                           static_cast<uint32_t>(tiles)};
         return cudaSuccess;
     };
@@ -450,10 +555,9 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
         return fail(g, PTL_CUDA_ERROR, "internal: unallocated node arrays");
     launch_ingest(P, s);
     {
-        uint32_t reach = 0;  // some node sits at max_depth (read with the error word's sync)
-        PTL_CU(cudaMemcpyAsync(&reach, P.flags + 3, sizeof(reach), cudaMemcpyDeviceToHost, s));
+        PTL_CU(read_back(g, P.flags + 3, 0));  // some node sits at max_depth (read with the error word's wait)
         if (ptl_status st = check_error_word(g); st != PTL_OK) return st;
-        if (!reach) return fail(g, PTL_INVALID_AST, "input: depths 0..max_depth are not all populated");
+        if (!g->pinned->v[0]) return fail(g, PTL_INVALID_AST, "input: depths 0..max_depth are not all populated");
     }
     if (g->scalar) launch_preprocess_scalar(P, s);
     else launch_preprocess(P, s);
@@ -463,23 +567,27 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
     launch_count_scan(P, sc, s);
     launch_fix(P, s);
     launch_decl_scan(P, g->meta.at<uint32_t>(), sc, s);
-    uint32_t meta[3] = {0, 0, 0};
-    PTL_CU(cudaMemcpyAsync(meta, g->meta.at<uint32_t>(), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    PTL_CU(cudaStreamSynchronize(s));
+    const uint32_t* meta = g->pinned->v;
+    PTL_CU(read_back(g, g->meta.at<uint32_t>(), 0));
     if (ptl_status st = check_error_word(g); st != PTL_OK) return st;
     g->F = meta[0];
     if (g->F == 0) return fail(g, PTL_UNSUPPORTED, "isn_cnt: program has no function (the reference takes the max of an empty range)");
     const size_t fb8 = r8(g->F);
     for (DevBuf* b : {&g->fn_id, &g->fn_start, &g->fn_size, &g->fn_end, &g->fn_start0, &g->fn_size0, &g->fn_end0,
-                      &g->fn_ra_start, &g->fn_ra_end, &g->fn_ra_size}) {
+                      &g->fn_ra_start, &g->fn_ra_end, &g->fn_ra_size})
         PTL_CU(b->ensure(fb8 + 8, 4));
-        PTL_CU(b->zero(s));
+    {
+        ZeroList z;
+        for (const DevBuf* b : {&g->fn_id, &g->fn_start, &g->fn_size, &g->fn_end, &g->fn_start0, &g->fn_size0, &g->fn_end0,
+                                &g->fn_ra_start, &g->fn_ra_end, &g->fn_ra_size})
+            b->zero(z);
+        PTL_CU(launch_zero(z, s));
     }
     P = make_prog(g);
     if (!prog_ready(P, {P.fn_id, P.fn_start, P.fn_size, P.fn_end, P.fn_start0, P.fn_size0}))
         return fail(g, PTL_CUDA_ERROR, "internal: unallocated function table");
     launch_functab(P, g->meta.at<uint32_t>(), s);
-    PTL_CU(cudaMemcpyAsync(meta, g->meta.at<uint32_t>(), sizeof(meta), cudaMemcpyDeviceToHost, s));
+    PTL_CU(read_back(g, g->meta.at<uint32_t>(), 0, 3));
     PTL_CU(cudaStreamSynchronize(s));
     g->W = meta[1];
     g->S = meta[2];
@@ -492,16 +600,18 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
 
     const size_t wb8 = r8(g->W);
     for (DevBuf* b : {&g->instr, &g->rd, &g->rs1, &g->rs2, &g->jt, &g->used_instrs, &g->symreg, &g->symswp,
-                      &g->stamp, &g->spill, &g->roffs}) {
+                      &g->stamp, &g->spill, &g->roffs})
         PTL_CU(b->ensure(wb8, 4));
-        PTL_CU(b->zero(s));
-    }
     PTL_CU(g->owner.ensure(wb8, 8));
-    PTL_CU(g->owner.zero(s));
-    PTL_CU(g->used.ensure(wb8, 1));
-    PTL_CU(g->used.zero(s));
-    PTL_CU(g->smark.ensure(wb8, 1));
-    PTL_CU(g->smark.zero(s));
+    for (DevBuf* b : {&g->used, &g->smark}) PTL_CU(b->ensure(wb8, 1));
+    PTL_CU(g->lifetime.ensure(fb8, 8));
+    {
+        ZeroList z;
+        for (const DevBuf* b : {&g->instr, &g->rd, &g->rs1, &g->rs2, &g->jt, &g->used_instrs, &g->symreg, &g->symswp,
+                                &g->stamp, &g->spill, &g->roffs, &g->owner, &g->used, &g->smark, &g->lifetime})
+            b->zero(z);
+        PTL_CU(launch_zero(z, s));
+    }
     PTL_CU(g->defpos.ensure(wb8, 1));
     P = make_prog(g);
     if (!prog_ready(P, {P.instr, P.rd, P.rs1, P.rs2, P.jt, P.used_instrs, P.symreg, P.symswp, P.stamp, P.spill,
@@ -519,8 +629,6 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
     timer.mark();
 
     // ---- regalloc
-    PTL_CU(g->lifetime.ensure(fb8, 8));
-    PTL_CU(g->lifetime.zero(s));
     if (g->scalar) {
         PTL_CU(g->preserve.ensure(fb8, 8));
         PTL_CU(g->preserve.zero(s));
@@ -572,14 +680,15 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
         PTL_CU(scan_for(wb8, &sc));
         launch_regalloc_count_scan(P, sc, s);
     }
-    uint32_t last_off = 0;
-    PTL_CU(read1(g, P.roffs + (g->W - 1), &last_off));
+    PTL_CU(read_back(g, P.roffs + (g->W - 1), 0));
     if (ptl_status st = check_error_word(g); st != PTL_OK) return st;
-    g->W2 = last_off + 1;
+    g->W2 = g->pinned->v[0] + 1;
     const size_t w2b8 = r8(g->W2);
-    for (DevBuf* b : {&g->ni, &g->nrd, &g->nr1, &g->nr2, &g->njt, &g->fsz, &g->joffs}) {
-        PTL_CU(b->ensure(w2b8 + 16, 4));
-        PTL_CU(b->zero(s));
+    for (DevBuf* b : {&g->ni, &g->nrd, &g->nr1, &g->nr2, &g->njt, &g->fsz, &g->joffs}) PTL_CU(b->ensure(w2b8 + 16, 4));
+    {
+        ZeroList z;
+        for (const DevBuf* b : {&g->ni, &g->nrd, &g->nr1, &g->nr2, &g->njt, &g->fsz, &g->joffs}) b->zero(z);
+        PTL_CU(launch_zero(z, s));
     }
     P = make_prog(g);
     if (!prog_ready(P, {P.ni, P.nrd, P.nr1, P.nr2, P.njt, P.fsz, P.joffs}))
@@ -600,11 +709,10 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
     // ---- fix_jumps (+ postprocess)
     PTL_CU(scan_for(w2b8, &sc));
     launch_fixjumps_scan(P, sc, s);
-    uint32_t last_size = 0, last_joff = 0;
-    PTL_CU(read1(g, P.fsz + (g->W2 - 1), &last_size));
-    PTL_CU(read1(g, P.joffs + (g->W2 - 1), &last_joff));
+    PTL_CU(read_back(g, P.fsz + (g->W2 - 1), 0));
+    PTL_CU(read_back(g, P.joffs + (g->W2 - 1), 1));
     if (ptl_status st = check_error_word(g); st != PTL_OK) return st;
-    g->W3 = last_size + last_joff;
+    g->W3 = g->pinned->v[0] + g->pinned->v[1];  // the last word's size and offset
     PTL_CU(g->out.ensure(r8(g->W3) + 8, 4));
     PTL_CU(g->out.zero(s));
     P = make_prog(g);
@@ -612,30 +720,10 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
     launch_fixjumps_emit(P, s);
     timer.mark();
     timer.mark();  // postprocess is fused into fix_jumps
+    if (to_host) PTL_CU(copy_results(g));
     if (ptl_status st = check_error_word(g); st != PTL_OK) return st;
     timer.finish();
-
-    if (to_host) {
-        g->words.resize(g->W3);
-        g->fn_start_h.resize(g->F);
-        g->fn_end_h.resize(g->F);
-        g->fn_size_h.resize(g->F);
-        g->fn_id_h.resize(g->F);
-        if (g->W3) {
-            // Where the device accesses pageable memory coherently (ATS), kernel stores put
-            // the words straight into the vector; otherwise the copy engine stages them.
-            if (pageable_paths(g->device).write && (reinterpret_cast<uintptr_t>(g->words.data()) & 15u) == 0)
-                PTL_CU(kernel_copy(P.out, g->words.data(), g->W3 * 4ull, s));
-            else
-                PTL_CU(cudaMemcpyAsync(g->words.data(), P.out, g->W3 * 4ull, cudaMemcpyDeviceToHost, s));
-        }
-        PTL_CU(cudaMemcpyAsync(g->fn_start_h.data(), P.fn_start, g->F * 4ull, cudaMemcpyDeviceToHost, s));
-        PTL_CU(cudaMemcpyAsync(g->fn_end_h.data(), P.fn_end, g->F * 4ull, cudaMemcpyDeviceToHost, s));
-        PTL_CU(cudaMemcpyAsync(g->fn_size_h.data(), P.fn_size, g->F * 4ull, cudaMemcpyDeviceToHost, s));
-        PTL_CU(cudaMemcpyAsync(g->fn_id_h.data(), P.fn_id, g->F * 4ull, cudaMemcpyDeviceToHost, s));
-        PTL_CU(cudaStreamSynchronize(s));
-        g->words_valid = g->table_valid = true;
-    }
+    if (to_host) take_results(g);
     return PTL_OK;
 }
 
@@ -708,6 +796,7 @@ ptl_status ptl_generator_create(const ptl_ast_view* tree, int device, ptl_genera
     cudaError_t e = on_device.err;
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) g->bind_stream();
+    if (e == cudaSuccess) e = g->take_pinned();
     if (e == cudaSuccess) e = upload_inputs(g, tree);
     if (e == cudaSuccess) e = g->tables.ensure(sizeof(CodeTables), 1);
     if (e == cudaSuccess) e = cudaMemcpyAsync(g->tables.at<char>(), &host_tables(), sizeof(CodeTables), cudaMemcpyHostToDevice, g->stream);
@@ -793,17 +882,10 @@ ptl_status ptl_generator_function_table(ptl_generator* g, const uint32_t** start
     if (!g->table_valid) {
         const DeviceScope on_device(g->device);
         if (!on_device.ok()) return fail(g, PTL_CUDA_ERROR, "cudaSetDevice");
-        g->fn_start_h.resize(g->F);
-        g->fn_end_h.resize(g->F);
-        g->fn_size_h.resize(g->F);
-        g->fn_id_h.resize(g->F);
-        cudaMemcpyAsync(g->fn_start_h.data(), g->fn_start.at<uint32_t>(), g->F * 4ull, cudaMemcpyDeviceToHost, g->stream);
-        cudaMemcpyAsync(g->fn_end_h.data(), g->fn_end.at<uint32_t>(), g->F * 4ull, cudaMemcpyDeviceToHost, g->stream);
-        cudaMemcpyAsync(g->fn_size_h.data(), g->fn_size.at<uint32_t>(), g->F * 4ull, cudaMemcpyDeviceToHost, g->stream);
-        cudaMemcpyAsync(g->fn_id_h.data(), g->fn_id.at<uint32_t>(), g->F * 4ull, cudaMemcpyDeviceToHost, g->stream);
-        const cudaError_t e = cudaStreamSynchronize(g->stream);
+        cudaError_t e = copy_table(g);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
         if (e != cudaSuccess) return cuda_fail(g, e, "function table");
-        g->table_valid = true;
+        take_table(g);
     }
     if (starts) *starts = g->fn_start_h.data();
     if (ends) *ends = g->fn_end_h.data();
@@ -850,6 +932,7 @@ ptl_status ptl_depth_order(const int32_t* keys, size_t n, uint32_t* pos, int dev
     g.n = n;
     cudaError_t e = cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) g.bind_stream();
+    if (e == cudaSuccess) e = g.take_pinned();
     if (e == cudaSuccess) e = g.dep.ensure(r8(n), 4);
     if (e == cudaSuccess) e = g.pos.ensure(r8(n), 4);
     if (e == cudaSuccess) e = g.errw.ensure(1, sizeof(ErrorWord));

@@ -47,6 +47,21 @@ void note_launch();
 // Raises a kernel's dynamic shared memory limit to at least bytes (never lowers it).
 cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes);
 
+// Up to kZeroMost memory ranges zeroed by one launch: a compile clears some 45 buffers,
+// and a memset of a small one costs the stream about 2 us whatever its size.  Ranges start
+// on 16-byte boundaries; their lengths round up to 16 bytes.
+constexpr int kZeroMost = 24;
+struct ZeroList {
+    uint4* p[kZeroMost];
+    uint64_t n16[kZeroMost];
+    int count = 0;
+    void add(void* q, size_t bytes) {
+        p[count] = static_cast<uint4*>(q);
+        n16[count++] = (bytes + 15u) / 16u;
+    }
+};
+cudaError_t launch_zero(const ZeroList& z, cudaStream_t s);
+
 // Element-wise stages (grid-stride launches of the per-thread functions).
 void launch_ingest(const Prog& P, cudaStream_t s);  // input checks + copy; flags[3]: max_depth reached
 void launch_preprocess(const Prog& P, cudaStream_t s);
