@@ -332,11 +332,14 @@ ptl_status Pipeline::scalar_regalloc(const std::vector<uint64_t>& F, const std::
     }
     upload_progs();
     const uint32_t t_w = tiles(7, W, elem_tile);
-    batch_stage(BatchStage::Cross, bl(7), t_w, nullptr);  // flags[1]: functions share symbols
+    const uint32_t t_f = tiles(6, F, elem_tile);
+    batch_stage(BatchStage::ScalarRange, bl(6), t_f, nullptr);
+    // flags[1]: functions share symbols; flags[2]: not sayable in records
+    batch_stage(BatchStage::ScalarRecords, bl(7), t_w, nullptr);
     BP_CU(cudaMemcpyAsync(hfl, flags.p, B * 16, cudaMemcpyDeviceToHost, s));
     BP_CU(collect_errors());
     std::vector<uint8_t> on_warp(B, 0);
-    std::vector<uint32_t> serial, alone;
+    std::vector<uint32_t> steps, serial, alone;
     uint64_t longest = 1, serial_f = 1;
     for (size_t p = 0; p < B; ++p) {
         if (!active[p]) continue;
@@ -344,12 +347,30 @@ ptl_status Pipeline::scalar_regalloc(const std::vector<uint64_t>& F, const std::
         if (hfl[4 * p + 1]) {
             serial.push_back(static_cast<uint32_t>(p));
             serial_f = std::max(serial_f, F[p]);
+        } else if (!hfl[4 * p + 2]) {
+            steps.push_back(static_cast<uint32_t>(p));
         } else if (S[p] <= scalar_warp_cap()) {
             on_warp[p] = 1;
             longest = std::max(longest, S[p]);
         } else {
             alone.push_back(static_cast<uint32_t>(p));
         }
+    }
+    if (!steps.empty()) {  // a lane per function, longest programs first
+        std::stable_sort(steps.begin(), steps.end(), [&](uint32_t x, uint32_t y) { return S[x] > S[y]; });
+        uint32_t* hf = table_slot(8);
+        uint32_t nf = 0;
+        uint64_t functions = 0;
+        for (const uint32_t p : steps) functions += F[p];
+        const uint32_t per = scalar_per_warp(functions);
+        for (size_t k = 0; k <= B; ++k) {
+            hf[k] = nf;
+            if (k < steps.size()) nf += static_cast<uint32_t>((F[steps[k]] + per - 1) / per);
+        }
+        BP_CU(cudaMemcpyAsync(dtable_slot(8), hf, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+        const uint32_t* d_steps = upload_list(0, steps);
+        BP_CU(batch_step_scalar(StepBatch{progs.at<Prog>(), d_steps, dtable_slot(8), nullptr,
+                                          static_cast<uint32_t>(steps.size()), nf, 0, 0, per}, s));
     }
     const uint32_t t_sw = tiles(16, F, scalar_warp_fns(), &on_warp);
     batch_scalar_ra_warp(bl(16), t_sw, static_cast<uint32_t>((longest + 15) & ~uint64_t(15)));
@@ -976,7 +997,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
             const uint32_t count = static_cast<uint32_t>(step_list.size());
             batch_free_order(progs.at<Prog>(), d_steps, count, s);
             BP_CU(batch_step_regalloc(StepBatch{progs.at<Prog>(), d_steps, dtable_slot(8), dtable_slot(23), count, nf, nr,
-                                                max_step_g0}, s));
+                                                max_step_g0, 0}, s));
         }
         if (!lane0_list.empty()) {
             // independent functions and lane-0 passes in one persistent launch

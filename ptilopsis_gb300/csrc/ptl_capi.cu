@@ -636,17 +636,20 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
         P = make_prog(g);
         if (!prog_ready(P, {P.lifetime, g->preserve.at<void>(), g->sextra.at<void>()}))
             return fail(g, PTL_CUDA_ERROR, "internal: unallocated regalloc state");
-        bool cross = false;
-        PTL_CU(scalar_regalloc_cross(P, s, &cross));
-        if (cross || serial) {
+        RaForm form = RaForm::Serial;
+        PTL_CU(scalar_ra_form(P, s, &form));
+        if (serial) form = RaForm::Serial;
+        if (form == RaForm::Serial) {
             PTL_CU(g->sregs.ensure(static_cast<size_t>(g->F) * 64, 4));
             PTL_CU(g->ssteps.ensure(g->F, sizeof(SRaStep)));
             launch_scalar_ra_serial(P, g->sregs.at<int32_t>(), g->ssteps.at<SRaStep>(),
                                     g->preserve.at<unsigned long long>(), s);
-        } else {
+        } else if (form == RaForm::General) {
             launch_scalar_ra_free(P, g->preserve.at<unsigned long long>(), s);
+        } else {
+            PTL_CU(run_step_scalar(P, g->preserve.at<unsigned long long>(), s));
         }
-        g->ra_serial = cross || serial;
+        g->ra_serial = form == RaForm::Serial;
         PTL_CU(scan_for(wb8, &sc));
         launch_scalar_ra_count_scan(P, g->preserve.at<unsigned long long>(), g->sextra.at<uint32_t>(), sc, s);
     } else {

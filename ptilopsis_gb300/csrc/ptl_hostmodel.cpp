@@ -29,6 +29,7 @@ uint32_t g_cache_k = 4;  // entries per function of the lane-0 symbol cache
 bool g_force_hashed = false;  // lane-0 pass finds row-0 values by hashing even when definitions are unique
 bool g_last_hashed = false;   // the last compile had a lane-0 virtual register with two definitions
 bool g_last_cross = false;    // the last scalar compile took the serial register allocation
+bool g_force_tiles = false;   // scalar register allocation by word tiles for every program
 bool g_force_serial = false;  // scalar register allocation in the reference's order for every program
 
 template <typename T>
@@ -290,16 +291,23 @@ struct Model {
     // to the regalloc output (the spill offsets, the count scan, the scatter, the moved
     // function table and the frame words).
     void scalar_regalloc(uint32_t F, uint32_t W, uint32_t wb8) {
-        uint32_t cross = 0;
-        for (uint32_t i = 0; i < W; ++i) cross |= st_ra_cross(P, i, stamp.p) & 1u;
+        uint32_t flagbits = g_force_tiles ? 2u : 0u;
+        for (uint32_t f = 0; f < F; ++f) flagbits |= st_scalar_range(P, f);
+        for (uint32_t i = 0; i < W; ++i) flagbits |= st_scalar_record(P, i);
+        const uint32_t cross = flagbits & 1u;
         std::vector<unsigned long long> preserve(F, 0);
         if (cross || g_force_serial) {
             std::vector<int32_t> sregs(static_cast<size_t>(F) * 64);
             std::vector<SRaStep> steps(F);
             s_ra_serial(P, sregs.data(), steps.data(), preserve.data());
+        } else if (!(flagbits & 2u)) {
+            std::vector<uint8_t> ring(g_ring_k);
+            std::vector<uint32_t> oidx(32);
+            for (uint32_t f = 0; f < F; ++f)
+                step_scalar_function(P, f, ring.data(), 1, g_ring_k, oidx.data(), 1, preserve.data());
         } else {
-            // the GPU's word tiles (functions by their first word, symbols as bytes)
             int32_t sregs[64];
+            // the GPU's word tiles (functions by their first word, symbols as bytes)
             constexpr uint32_t T = 4096;
             std::vector<uint8_t> sym;
             for (uint32_t b = 0; b <= W / T; ++b) {
@@ -530,6 +538,7 @@ int ptlhm_gen_desc_ok(void) {
     build_code_tables(&t);
     return gen_desc_ok(&t) ? 1 : 0;
 }
+void ptlhm_set_scalar_tiles(int on) { g_force_tiles = on != 0; }
 void ptlhm_set_scalar_serial(int on) { g_force_serial = on != 0; }
 
 void ptlhm_set_cache_entries(uint32_t k) { g_cache_k = k; }

@@ -1714,14 +1714,6 @@ __global__ void __launch_bounds__(kRaClusterThreads, 1)
     if (rank == 0 && row && ra2_tail_hit(P, loc, tid, s0, S)) P.symswp[loc.R0[tid] - 64u] = 0xFFFFFFFFu;
 }
 
-// flags[1]: functions share symbols; flags[2]: a lane-0 virtual register has two
-// definitions.  stamp counts the definitions (zeroed before).
-__global__ void k_ra_cross(Prog P) {
-    uint32_t any = 0;
-    PTL_FOR(i, P.W) any |= st_ra_cross(P, i, P.stamp);
-    if (__syncthreads_or(any & 1u) && threadIdx.x == 0) P.flags[1] = 1;
-    if (__syncthreads_or(any & 2u) && threadIdx.x == 0) P.flags[2] = 1;
-}
 // The step records; flags[1]: functions share symbols, flags[2]: a word that a record
 // cannot say, or function ranges that overlap.
 __global__ void k_ra_records(Prog P) {
@@ -1729,6 +1721,14 @@ __global__ void k_ra_records(Prog P) {
     uint32_t hint = 0xFFFFFFFFu;
     PTL_FOR(i, P.W) any |= st_step_record(P, i, &hint);
     PTL_FOR(f, P.F) any |= st_step_range(P, f);
+    if (__syncthreads_or(any & 1u) && threadIdx.x == 0) P.flags[1] = 1;
+    if (__syncthreads_or(any & 2u) && threadIdx.x == 0) P.flags[2] = 1;
+}
+__global__ void k_scalar_records(Prog P) {
+    uint32_t any = 0;
+    uint32_t hint = 0xFFFFFFFFu;
+    PTL_FOR(i, P.W) any |= st_scalar_record(P, i, &hint);
+    PTL_FOR(f, P.F) any |= st_scalar_range(P, f);
     if (__syncthreads_or(any & 1u) && threadIdx.x == 0) P.flags[1] = 1;
     if (__syncthreads_or(any & 2u) && threadIdx.x == 0) P.flags[2] = 1;
 }
@@ -2350,15 +2350,14 @@ void launch_gen_scalar(const Prog& P, cudaStream_t s) {
     k_s_gen_write<<<grid_for(P.n), kThreads, 0, s>>>(P);
 }
 
-cudaError_t scalar_regalloc_cross(const Prog& P, cudaStream_t s, bool* cross) {
+cudaError_t scalar_ra_form(const Prog& P, cudaStream_t s, RaForm* form) {
     cudaMemsetAsync(P.flags + 1, 0, 2 * sizeof(uint32_t), s);
-    cudaMemsetAsync(P.stamp, 0, sizeof(uint32_t) * P.W, s);
     g_launches++;
-    k_ra_cross<<<grid_for(P.W), kThreads, 0, s>>>(P);
-    uint32_t fl = 0;
-    cudaMemcpyAsync(&fl, P.flags + 1, sizeof(fl), cudaMemcpyDeviceToHost, s);
+    k_scalar_records<<<grid_for(P.W), kThreads, 0, s>>>(P);
+    uint32_t fl[2] = {0, 0};
+    cudaMemcpyAsync(fl, P.flags + 1, sizeof(fl), cudaMemcpyDeviceToHost, s);
     const cudaError_t e = cudaStreamSynchronize(s);
-    *cross = fl != 0;
+    *form = fl[0] ? RaForm::Serial : (fl[1] ? RaForm::General : RaForm::Steps);
     return e;
 }
 
@@ -2599,17 +2598,18 @@ struct BRecords {
         if (r & 2u) P.flags[2] = 1u;
     }
 };
-struct BCross {
+struct BScalarRecords {
     static constexpr bool kViewInShared = true;
     uint32_t hint = 0xFFFFFFFFu, hp = 0xFFFFFFFFu;
     __device__ static uint32_t count(const Prog& P) { return P.W; }
     __device__ void operator()(const Prog& P, uint32_t i, uint32_t p) {
         if (p != hp) { hp = p; hint = 0xFFFFFFFFu; }
-        const uint32_t r = st_ra_cross(P, i, P.stamp, &hint);
-        if (r & 1u) atomicOr(&P.flags[1], 1u);
-        if (r & 2u) atomicOr(&P.flags[2], 1u);
+        const uint32_t r = st_scalar_record(P, i, &hint);
+        if (r & 1u) P.flags[1] = 1u;
+        if (r & 2u) P.flags[2] = 1u;
     }
 };
+PTL_BATCH_OP(BScalarRange, P.F, if (st_scalar_range(P, i)) P.flags[2] = 1u)
 
 // per program: word count and longest function (meta[4p + 1], meta[4p + 2])
 struct BFunctabEnd {
@@ -3017,7 +3017,8 @@ void batch_stage(BatchStage st, const BatchLaunch& bl, uint32_t total, uint32_t*
         case BatchStage::OptMark: batch_launch(bl, total, BOptMark{meta}); break;  // meta: the odd flag
         case BatchStage::OptFinal: batch_launch(bl, total, BOptFinal{}); break;
         case BatchStage::InitLifetime: batch_launch(bl, total, BInitLifetime{}); break;
-        case BatchStage::Cross: batch_launch(bl, total, BCross{}); break;
+        case BatchStage::ScalarRecords: batch_launch(bl, total, BScalarRecords{}); break;
+        case BatchStage::ScalarRange: batch_launch(bl, total, BScalarRange{}); break;
         case BatchStage::Records: batch_launch(bl, total, BRecords{}); break;
         case BatchStage::RaHist: batch_launch(bl, total, BRaHist{}); break;
         case BatchStage::Spill: batch_launch(bl, total, BSpill{}); break;

@@ -96,8 +96,14 @@ struct StepBatch {
     const uint32_t* free_off;  // [n + 1]
     const uint32_t* row_off;   // [n + 1]
     uint32_t n, free_blocks, row_blocks, max_g0;
+    uint32_t per_block;        // batch_step_scalar: functions per block (scalar_per_warp)
 };
 cudaError_t batch_step_regalloc(const StepBatch& b, cudaStream_t s);
+uint32_t scalar_per_warp(uint64_t functions);
+// The same for the scalar generator (free_off: blocks of per_block functions), leaving the
+// preserve masks (one program: preserve; a batch: each program's s_preserve).
+cudaError_t run_step_scalar(const Prog& P, unsigned long long* preserve, cudaStream_t s);
+cudaError_t batch_step_scalar(const StepBatch& b, cudaStream_t s);
 // Lane-0 passes too wide for one block: programs with more than kRaClusterMin lane-0
 // groups (at most 8,192) run theirs on a thread-block cluster when the device can place
 // it.  ra_cluster_fits tells whether it can; launch_ra_wide launches the program's
@@ -112,13 +118,14 @@ void launch_fixjumps_scan(const Prog& P, const ScanScratch& sc, cudaStream_t s);
 void launch_fixjumps_emit(const Prog& P, cudaStream_t s);
 
 // The scalar generator's stages where they differ (ptl_scalar.cuh).  Register
-// allocation: the cross check (functions naming each other's words take the serial
-// order), then one thread per function or the serial kernel (regs: F x 64, steps: F),
+// allocation: scalar_ra_form builds the step records (functions naming each other's words
+// take the serial order, words that a record cannot say the general form, a warp or a
+// thread per function), then that form's launch (regs: F x 64, steps: F),
 // each leaving the preserve masks; the count scan with the preserve words (extra: wb8
 // counts); the scatter, the moved function table and the frame words (claim: W2 keys).
 void launch_preprocess_scalar(const Prog& P, cudaStream_t s);
 void launch_gen_scalar(const Prog& P, cudaStream_t s);
-cudaError_t scalar_regalloc_cross(const Prog& P, cudaStream_t s, bool* cross);
+cudaError_t scalar_ra_form(const Prog& P, cudaStream_t s, RaForm* form);
 void launch_scalar_ra_free(const Prog& P, unsigned long long* preserve, cudaStream_t s);
 void launch_scalar_ra_serial(const Prog& P, int32_t* regs, SRaStep* steps, unsigned long long* preserve,
                              cudaStream_t s);
@@ -162,7 +169,7 @@ struct BatchLaunch {
     uint32_t tile;
 };
 enum class BatchStage {
-    Ingest, Preprocess, Fix, Functab, Gen, OptMark, OptFinal, InitLifetime, Cross, Records, RaHist, Spill,
+    Ingest, Preprocess, Fix, Functab, Gen, OptMark, OptFinal, InitLifetime, Records, ScalarRecords, ScalarRange, RaHist, Spill,
     Scatter, RaFunctab, FjEmit, FjFunctab,
     // the scalar generator's (ptl_scalar.cuh): preprocess, isn_gen, preserve counts
     // (per function), scatter (per word), the function table after regalloc (per

@@ -64,6 +64,22 @@ __global__ void __launch_bounds__(32) k_step_free(Src src) {
     step_free_function(P, f, ring + threadIdx.x, kFreeStride, kFreeRing);
 }
 
+// ---- the scalar generator's functions: one thread each, one warp a block.  The warp form
+// (k_s_ra_warp: every lane runs the same function) took 790 cycles a step and a warp per
+// function; this one takes half as long and a lane.
+constexpr uint32_t kScalarRing = 256, kScalarStride = 36;
+template <class Src>
+__global__ void __launch_bounds__(32) k_step_scalar(Src src, unsigned long long* preserve, uint32_t per_warp) {
+    __shared__ Prog P;
+    __shared__ uint8_t ring[kScalarRing * kScalarStride];
+    __shared__ uint32_t oidx[32 * 32];
+    uint32_t local;
+    src.take(blockIdx.x, &local, P);
+    const uint32_t lane = threadIdx.x;
+    step_scalar_function(P, lane < per_warp ? local * per_warp + lane : P.F, ring + threadIdx.x, kScalarStride, kScalarRing,
+                         oidx + threadIdx.x, 32u, preserve ? preserve : P.s_preserve);
+}
+
 // ---- trigger rows: a block per 32 steps; lane = step, so a function's masks load
 // coalesced, and the warps share out the groups.  The least group of a position is the
 // first to show it on the way up, the greatest the first on the way down.
@@ -587,6 +603,27 @@ cudaError_t run_step_regalloc(const Prog& P, cudaStream_t s) {
         if (G0 > kStepBlockMax) return cudaErrorInvalidConfiguration;  // not a program of this form (ra_form)
     }
     return launch_lane0(src, 1, G0, 1024u, s);
+}
+
+// Functions per warp: a warp's step takes the branches of all its lanes, so as few as keep
+// the chip's warps busy (one function: 560 cycles a step; 32 side by side: 720).
+uint32_t scalar_per_warp(uint64_t functions) {
+    constexpr uint64_t kWarps = 152u * 8u;
+    return static_cast<uint32_t>(std::min<uint64_t>(32, (functions + kWarps - 1u) / kWarps));
+}
+
+cudaError_t run_step_scalar(const Prog& P, unsigned long long* preserve, cudaStream_t s) {
+    note_launch();
+    const uint32_t per = scalar_per_warp(P.F);
+    k_step_scalar<<<(P.F + per - 1u) / per, 32, 0, s>>>(OneProgram{P}, preserve, per);
+    return cudaGetLastError();
+}
+
+cudaError_t batch_step_scalar(const StepBatch& b, cudaStream_t s) {
+    if (b.n == 0 || b.free_blocks == 0) return cudaSuccess;
+    note_launch();
+    k_step_scalar<<<b.free_blocks, 32, 0, s>>>(ManyPrograms{b.progs, b.free_off, b.order, b.n}, nullptr, b.per_block);
+    return cudaGetLastError();
 }
 
 cudaError_t batch_step_regalloc(const StepBatch& b, cudaStream_t s) {

@@ -22,6 +22,7 @@
 #pragma once
 
 #include "ptl_ra.cuh"
+#include "ptl_scalar.cuh"
 
 #if defined(__GNUC__) || defined(__CUDACC__)
 #define PTL_RARE(x) __builtin_expect(!!(x), 0)
@@ -502,6 +503,172 @@ PTL_HD void lane_step_b2(LaneShared& sh, const LaneStep& st, const LaneMasks& m,
 // that row 0 holds at positions an independent function triggers (tail: those positions).
 PTL_HD void lane_tail(const LaneShared& sh, const LaneSlot& L, uint32_t tail) {
     for (uint32_t m = L.held & (L.marked | tail); m; m &= m - 1) L.symswp[sh.oidx[low_bit(m)]] = 0xFFFFFFFFu;
+}
+
+// ---------------------------------------------------------------- the scalar generator
+// Its functions (ptl_scalar.cuh) have a register state each, so every function is on its
+// own like a lone lane-0 slot, with three differences: physical operands clear and swap
+// like symbols' registers, a call out of the function frees and swaps the caller-saved
+// registers, and the live mask's callee-saved registers are gathered (preserve).
+//
+// Records: bits 0-19 and 20-39, distances of the operand symbols (0: none); 40-45 rd's
+// code, 46-51 and 52-57 physical operands' codes; 58 rd is the word itself, 59 an operand
+// is, 60 float result, 61 float operands, 62 a call out of the function, 63 used.
+constexpr uint32_t kScalarDist = 1u << 20;
+constexpr uint32_t kSDef = 1u << 26, kSSelf = 1u << 27, kSFloatRd = 1u << 28, kSFloatOp = 1u << 29, kSCall = 1u << 30,
+                   kSUsed = 1u << 31;  // in the high word
+constexpr uint32_t kScalarPreserved = 0x0FFC031Eu;  // kPreservedRegisterMask in register codes
+
+PTL_HD uint32_t st_scalar_record(const Prog& P, uint32_t i, uint32_t* hint = nullptr) {
+    const uint32_t lo = function_of(P, i, hint ? *hint : 0xFFFFFFFFu);
+    if (hint) *hint = lo;
+    const uint32_t op[2] = {P.rs1[i], P.rs2[i]}, rd = P.rd[i];
+    if (!ra_own(P, lo, op[0]) || !ra_own(P, lo, op[1]) || !ra_own(P, lo, rd)) return 1u;
+    const uint32_t st = P.fn_start0[lo], size = P.fn_size0[lo];
+    uint64_t rec = 0;
+    uint32_t out = 0;
+    if (i >= st && i - st < size && P.used_instrs[i]) {
+        const uint32_t ins = P.instr[i], j = P.jt[i];
+        uint32_t hi = kSUsed;
+        if (ins == 0x000000EFu && (j < st || j - st >= size)) hi |= kSCall;
+        if (s_needs_float(ins, 0)) hi |= kSFloatRd;
+        if (s_needs_float(ins, 1)) hi |= kSFloatOp;
+        rec = 0;
+        uint32_t code[3] = {kCodeNone, kCodeNone, kCodeNone};
+        if (rd >= 64u) {
+            if (rd - 64u == i) hi |= kSDef;
+            else out = 2u;
+        } else {
+            code[0] = code_of(rd);
+            if (rd >= 32u && ((kNonscratchRegisters >> rd) & 1ull)) out = 2u;  // not in the 32-bit live mask
+        }
+        for (int k = 0; k < 2; ++k) {
+            if (op[k] < 64u) {
+                code[k + 1] = code_of(op[k]);
+                continue;
+            }
+            const uint32_t x = op[k] - 64u;
+            if (x == i) hi |= kSSelf;
+            if (x >= i) continue;  // not defined yet: reads and writes the initial state
+            if (i - x >= kScalarDist) out = 2u;
+            rec |= static_cast<uint64_t>((i - x) & (kScalarDist - 1u)) << (20 * k);
+        }
+        rec |= static_cast<uint64_t>(code[0]) << 40 | static_cast<uint64_t>(code[1]) << 46 |
+               static_cast<uint64_t>(code[2]) << 52 | static_cast<uint64_t>(hi) << 32;
+    }
+    P.rec[i] = rec;
+    return out;
+}
+PTL_HD uint32_t st_scalar_range(const Prog& P, uint32_t f) {
+    return s_ra_function_ok(P, f) ? st_step_range(P, f) : 2u;  // the other forms report the error
+}
+
+// Function f (past the end: nothing but the other lanes' turns; a whole warp calls this).
+// Ring entries as in the lane-0 pass; oidx[p * ostride]: the word whose symbol position p
+// holds.
+PTL_HD void step_scalar_function(const Prog& P, uint32_t f, uint8_t* ring, uint32_t stride, uint32_t K, uint32_t* oidx,
+                                 uint32_t ostride, unsigned long long* preserve) {
+    const bool real = f < P.F;
+    const uint32_t start = real ? P.fn_start0[f] : 0u, n = real ? P.fn_size0[f] : 0u, mask = K - 1u;
+    const unsigned long long* rec = P.rec + start;
+    uint32_t* symreg = P.symreg + start;
+    uint32_t* symswp = P.symswp + start;
+    uint32_t live = kLiveInit, held = 0, marked = 0, kept = 0;
+#if defined(__CUDA_ARCH__)
+    const uint32_t steps = __reduce_max_sync(0xFFFFFFFFu, n);
+#else
+    const uint32_t steps = n;
+#endif
+    constexpr uint32_t kAhead = 4;
+    unsigned long long next[kAhead];
+#pragma unroll
+    for (uint32_t k = 0; k < kAhead; ++k) next[k] = k < n ? rec[k] : 0ull;
+    for (uint32_t b = 0; b < steps; b += kAhead) {
+        unsigned long long now[kAhead];
+#pragma unroll
+        for (uint32_t k = 0; k < kAhead; ++k) {
+            now[k] = next[k];
+            next[k] = b + kAhead + k < n ? rec[b + kAhead + k] : 0ull;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kAhead; ++k) {
+            const uint32_t i = b + k;
+            const uint32_t hi = static_cast<uint32_t>(now[k] >> 32);
+            const uint32_t d1 = static_cast<uint32_t>(now[k]) & (kScalarDist - 1u);
+            const uint32_t d2 = static_cast<uint32_t>(now[k] >> 20) & (kScalarDist - 1u);
+            const bool used = (hi & kSUsed) != 0, call = (hi & kSCall) != 0;
+            uint32_t e1 = ring[((i - d1) & mask) * stride], e2 = ring[((i - d2) & mask) * stride];
+            // seldom: an operand older than the ring, or one whose register has moved
+            const bool old = (d1 | d2) >= K;
+            const bool rare = warp_any(old || ((d1 ? e1 : 0u) | (d2 ? e2 : 0u)) & kSymMoved);
+            if (PTL_RARE(rare)) {
+                if (d1 >= K) e1 = code_of(symreg[i - d1]) | (symswp[i - d1] ? kSymSwapped : 0u) | kSymMoved;
+                if (d2 >= K) e2 = code_of(symreg[i - d2]) | (symswp[i - d2] ? kSymSwapped : 0u) | kSymMoved;
+            }
+            e1 = d1 ? e1 : (hi >> 14) & 63u;
+            e2 = d2 ? e2 : (hi >> 20) & 63u;
+            e1 = used ? e1 : kCodeNone;
+            e2 = used ? e2 : kCodeNone;
+            // an operand symbol's position: the one it was defined in, while it is held
+            uint32_t m1 = d1 && oidx[(e1 & 31u) * ostride] == i - d1 ? code_bit(e1 & 63u) & held : 0u;
+            uint32_t m2 = d2 && oidx[(e2 & 31u) * ostride] == i - d2 ? code_bit(e2 & 63u) & held : 0u;
+            if (PTL_RARE(rare)) {
+                for (uint32_t m = held; m; m &= m - 1) {
+                    const uint32_t x = oidx[low_bit(m) * ostride], bit = m & (~m + 1u);
+                    if (d1 && x == i - d1) m1 = bit;
+                    if (d2 && x == i - d2) m2 = bit;
+                }
+            }
+            const bool fop = (hi & kSFloatOp) != 0;
+            const uint32_t c1 = (e1 & kSymSwapped) || (m1 & marked) ? (fop ? 0u : 5u) : e1 & 63u;
+            const uint32_t c2 = (e2 & kSymSwapped) || (m2 & marked) ? (fop ? kCode38 : 6u) : e2 & 63u;
+            // step_allocate's fields in their places of a lane-0 record's high word
+            const StepOut o = step_allocate(((hi & kSDef) ? kStepDef : 0u) | ((hi & kSFloatRd) ? kStepFloat : 0u) |
+                                                (used ? ((hi >> 8) & 63u) << 16 : kCodeNone << 16),
+                                            live, c1, c2);
+            const bool def = (hi & (kSDef | kSSelf)) == kSDef && !call;
+            if (i < n) ring[(i & mask) * stride] = static_cast<uint8_t>((def ? o.rd : kCodeNone) | ((hi & kSSelf) ? kSymMoved : 0u));
+            if (def) symreg[i] = o.rd ? o.rd : 37u;
+            const bool s1 = d1 && d1 != d2 && e1 != c1 && !call, s2 = d2 && e2 != c2 && !call;
+            // swapped: the held symbols of the triggered registers, but those just read; a
+            // call triggers the caller-saved ones
+            const uint32_t trig = call ? live & ~kScalarPreserved : o.trig;
+            live = call ? live & kScalarPreserved : o.live;
+            marked = (marked | (held & trig)) & ~(call ? 0u : m1 | m2);
+            const uint32_t gone = call ? ~live : code_bit(o.rd) | code_bit(c1) | code_bit(c2);
+            uint32_t t = held & marked & gone;  // swapped symbols that leave their positions
+            if (warp_any(s1 || s2 || t != 0)) {
+                if (s1) {
+                    if (d1 < K)
+                        ring[((i - d1) & mask) * stride] =
+                            static_cast<uint8_t>(c1 | ((e1 & kSymMoved) || c1 != (e1 & 63u) ? kSymMoved : 0u));
+                    symreg[i - d1] = reg_of(c1);
+                    if (e1 & kSymSwapped) symswp[i - d1] = 0;
+                }
+                if (s2) {
+                    if (d2 < K)
+                        ring[((i - d2) & mask) * stride] =
+                            static_cast<uint8_t>(c2 | ((e2 & kSymMoved) || c2 != (e2 & 63u) ? kSymMoved : 0u));
+                    symreg[i - d2] = reg_of(c2);
+                    if (e2 & kSymSwapped) symswp[i - d2] = 0;
+                }
+                for (; t; t &= t - 1) {
+                    const uint32_t idx = oidx[low_bit(t) * ostride];
+                    symswp[idx] = 0xFFFFFFFFu;
+                    if (i - idx < K) ring[(idx & mask) * stride] |= kSymSwapped;
+                }
+            }
+            held &= ~gone;
+            marked &= held;
+            if ((hi & kSDef) && !call) {
+                oidx[o.rd * ostride] = i;
+                held |= code_bit(o.rd);
+            }
+            kept |= live;
+        }
+    }
+    for (uint32_t m = held & marked; m; m &= m - 1) symswp[oidx[low_bit(m) * ostride]] = 0xFFFFFFFFu;
+    if (real) preserve[f] = kept & static_cast<uint32_t>(kNonscratchRegisters);
 }
 
 }  // namespace ptl

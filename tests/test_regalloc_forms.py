@@ -61,3 +61,42 @@ def test_gpu_batch_of_all_widths(built_cuda):
         b.compile(trees)
         for k, tree in enumerate(trees):
             np.testing.assert_array_equal(b.words(k), portbind.compile_ast(tree_to_ast(tree)).words, err_msg=str(k))
+
+
+@pytest.mark.parametrize("form", ["records", "records, ring of 8 words", "tiles", "serial"])
+def test_hostmodel_scalar_forms(built, form):
+    """The scalar generator's allocation by step records (old words read back with a small
+    ring), by word tiles and in the reference's order, against its oracle."""
+    from oracle import portbind
+    from test_hostmodel import hostmodel
+    from test_scalar import hm_compile_scalar
+    L = hostmodel()
+    L.ptlhm_set_ring_words(ctypes.c_uint32(8 if "8" in form else 256))
+    L.ptlhm_set_scalar_tiles(1 if form == "tiles" else 0)
+    try:
+        for tree in (_program(9), _program(40, 150.0, max_expr_depth=12, float_frac=0.5),
+                     _program(3, 2500.0, max_nesting=32, spill_frac=1.0)):
+            rc, err, got = hm_compile_scalar(tree_to_ast(tree), serial=form == "serial")
+            assert rc == 0, f"host model error {err}"
+            np.testing.assert_array_equal(got[0], portbind.compile_ast(tree_to_ast(tree), scalar=True).words)
+    finally:
+        L.ptlhm_set_ring_words(ctypes.c_uint32(16))
+        L.ptlhm_set_scalar_tiles(0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_functions", [1, 31, 32, 33, 300])
+def test_gpu_scalar_records(built_cuda, n_functions):
+    """A warp's lanes partly and wholly used, functions of very different lengths side by
+    side, alone and in a batch."""
+    from oracle import portbind
+    from ptilopsis_gb300 import RvGenerator
+    from ptilopsis_gb300.batch import BatchCompiler
+    tree = _program(n_functions, 300.0, max_expr_depth=12, float_frac=0.5, max_nesting=32)
+    want = portbind.compile_ast(tree_to_ast(tree), scalar=True).words
+    with RvGenerator(tree, scalar=True) as gen:
+        gen.process()
+        np.testing.assert_array_equal(gen.get_instructions(), want)
+    with BatchCompiler(tiles=None, scalar=True) as b:
+        b.compile([_program(5), tree, _program(2)])
+        np.testing.assert_array_equal(b.words(1), want)
