@@ -97,7 +97,7 @@ struct ptl_generator {
     DevBuf decl, fn_id, fn_start, fn_size, fn_end, fn_start0, fn_size0, fn_end0;
     DevBuf fn_ra_start, fn_ra_end, fn_ra_size;
     DevBuf instr, rd, rs1, rs2, jt, owner, used, smark, used_instrs;
-    DevBuf tmask, trow, tany;
+    DevBuf tmask, trow, tany, opt_work;
     DevBuf symreg, symswp, stamp, defpos, lifetime, trig_min, trig_max, ra_chunks, spill, roffs;
     DevBuf ni, nrd, nr1, nr2, njt, fsz, joffs, out;
     DevBuf sort_a, sort_apos, sort_bpos, sort_seg0, sort_seg1, sort_tile_seg, sort_tile_l, sort_tile_r, sort_stops,
@@ -141,7 +141,7 @@ struct ptl_generator {
         return {&in_type, &in_rtype, &in_parent, &in_depth, &in_child, &in_data, &nt, &rt, &nd1, &nd,
                 &par, &ci, &dep, &fflag, &sizes, &loc0, &loc, &pos, &regs, &decl, &fn_id, &fn_start,
                 &fn_size, &fn_end, &fn_start0, &fn_size0, &fn_end0, &fn_ra_start, &fn_ra_end, &fn_ra_size,
-                &instr, &rd, &rs1, &rs2, &jt, &owner, &used, &smark, &used_instrs, &tmask, &trow, &tany, &symreg, &symswp,
+                &instr, &rd, &rs1, &rs2, &jt, &owner, &used, &smark, &used_instrs, &tmask, &trow, &tany, &opt_work, &symreg, &symswp,
                 &stamp, &defpos, &lifetime, &trig_min, &trig_max, &ra_chunks, &spill, &roffs, &ni, &nrd, &nr1, &nr2, &njt,
                 &fsz, &joffs, &out, &sort_a, &sort_apos, &sort_bpos, &sort_seg0, &sort_seg1, &sort_stops,
                 &sort_tile_seg, &sort_tile_l, &sort_tile_r, &sort_leaf, &sort_heap, &sort_counters, &sort_local, &sort_equal,
@@ -624,7 +624,8 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
     timer.mark();
 
     // ---- optimize
-    PTL_CU(run_optimize(P, s, &g->opt_sweeps));
+    PTL_CU(g->opt_work.ensure(optimize_work_bytes(g->W), 1));
+    PTL_CU(run_optimize(P, g->opt_work.at<char>(), s, &g->opt_sweeps));
     if (ptl_status st = check_error_word(g); st != PTL_OK) return st;
     timer.mark();
 

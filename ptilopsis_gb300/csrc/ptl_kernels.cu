@@ -996,16 +996,25 @@ __global__ void __launch_bounds__(kSortBlockThreads) k_sort_block(SortScratch ss
     }
 }
 
-// Equal-key ranges found by the rounds: one block per range places each (key, index)
-// pair at its closed-form position, through apos (free after the rounds).
+// Equal-key ranges found by the rounds: each (key, index) pair to its closed-form position
+// through apos (free after the rounds), then back.  Few ranges hold most of the keys (a
+// level of a large program), so every range is cut into kEqualParts block shares: with
+// one block per range the 19M-node program's ranges took 2.0 ms.
+constexpr uint32_t kEqualParts = 64;
 __global__ void __launch_bounds__(kThreads) k_sort_equal(SortScratch ss, uint32_t count) {
-    for (uint32_t r = blockIdx.x; r < count; r += gridDim.x) {
+    for (uint32_t w = blockIdx.x; w < count * kEqualParts; w += gridDim.x) {
+        const uint32_t r = w / kEqualParts, part = w % kEqualParts;
         const uint32_t first = ss.equal[2 * r], m = ss.equal[2 * r + 1] - first;
-        for (uint32_t i = threadIdx.x; i < m; i += kThreads) ss.apos[first + equal_final_index(i, m)] = sidx(ss.a[first + i]);
-        __syncthreads();
-        const unsigned long long key = ss.a[first] & 0xFFFFFFFF00000000ull;
-        for (uint32_t i = threadIdx.x; i < m; i += kThreads) ss.a[first + i] = key | ss.apos[first + i];
-        __syncthreads();
+        for (uint32_t i = part * kThreads + threadIdx.x; i < m; i += kEqualParts * kThreads)
+            ss.apos[first + equal_final_index(i, m)] = sidx(ss.a[first + i]);
+    }
+}
+__global__ void __launch_bounds__(kThreads) k_sort_equal_back(SortScratch ss, uint32_t count) {
+    for (uint32_t w = blockIdx.x; w < count * kEqualParts; w += gridDim.x) {
+        const uint32_t r = w / kEqualParts, part = w % kEqualParts;
+        const uint32_t first = ss.equal[2 * r], m = ss.equal[2 * r + 1] - first;
+        for (uint32_t i = part * kThreads + threadIdx.x; i < m; i += kEqualParts * kThreads)  // the keys are equal
+            reinterpret_cast<uint32_t*>(ss.a + first + i)[0] = ss.apos[first + i];
     }
 }
 __global__ void k_sort_heaps(SortScratch ss, uint32_t count) {
@@ -1018,11 +1027,21 @@ __global__ void k_gen_prop(Prog P) { PTL_FOR(x, P.n) st_gen_prop(P, x); }
 __global__ void k_gen_claim(Prog P) { PTL_FOR(x, P.n) st_gen_claim(P, x); }
 __global__ void k_gen_write(Prog P) { PTL_FOR(x, P.n) st_gen_write(P, x); }
 
-__global__ void k_opt_mark(Prog P) { PTL_FOR(i, P.wb8) st_opt_mark(P, i); }
-__global__ void k_opt_sweep(Prog P) {
-    bool any = false;
-    PTL_FOR(i, P.wb8) any |= st_opt_sweep(P, i);
-    if (__syncthreads_or(any) && threadIdx.x == 0) P.flags[0] = 1;
+// The marks, and the sweeps' start; flags[0]: some virtual result is not its instruction's
+// own word.
+constexpr uint32_t kOptTile = 1024, kOptSweeps = 4;
+__global__ void k_opt_mark(Prog P, uint32_t tiles, uint8_t* cur, uint8_t* next, uint32_t* run) {
+    bool odd = false;
+    PTL_FOR(t, tiles) {  // the first sweep takes every tile
+        cur[t] = 1;
+        next[t] = 0;
+    }
+    if (blockIdx.x == 0 && threadIdx.x <= kOptSweeps) run[threadIdx.x] = threadIdx.x == 0 ? 1u : 0u;
+    PTL_FOR(i, P.wb8) {
+        st_opt_mark(P, i);
+        odd |= s32(P.rd[i]) > 63 && P.rd[i] - 64u != i;
+    }
+    if (__syncthreads_or(odd) && threadIdx.x == 0) P.flags[0] = 1u;
 }
 __global__ void k_opt_final(Prog P) { PTL_FOR(i, P.wb8) st_opt_final(P, i); }
 
@@ -2066,8 +2085,10 @@ cudaError_t run_sort_rounds(const SortScratch& ss, uint32_t nseg0, uint32_t firs
     if (lh[1]) { g_launches++; k_sort_heaps<<<grid_for(lh[1]), kThreads, 0, s>>>(ss, lh[1]); }
     if (lh[0]) { g_launches++; k_sort_leaves<<<grid_for(lh[0]), kThreads, 0, s>>>(ss, lh[0]); }
     if (lh[5]) {
-        g_launches++;
-        k_sort_equal<<<static_cast<unsigned>(std::min<uint32_t>(lh[5], 152u * 8u)), kThreads, 0, s>>>(ss, lh[5]);
+        const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(static_cast<uint64_t>(lh[5]) * kEqualParts, 152u * 8u));
+        g_launches += 2;
+        k_sort_equal<<<grid, kThreads, 0, s>>>(ss, lh[5]);
+        k_sort_equal_back<<<grid, kThreads, 0, s>>>(ss, lh[5]);
     }
     if (lh[4]) {
         const size_t smem = sizeof(BlockSortSmem);
@@ -2120,30 +2141,6 @@ void launch_gen(const Prog& P, cudaStream_t s) {
     k_gen_claim<<<grid_for(P.n), kThreads, 0, s>>>(P);
     g_launches++;
     k_gen_write<<<grid_for(P.n), kThreads, 0, s>>>(P);
-}
-
-cudaError_t run_optimize(const Prog& P, cudaStream_t s, uint32_t* sweeps_out) {
-    g_launches++;
-    k_opt_mark<<<grid_for(P.wb8), kThreads, 0, s>>>(P);
-    uint32_t sweeps = 0;
-    for (;;) {
-        cudaMemsetAsync(P.flags, 0, sizeof(uint32_t), s);
-        for (int k = 0; k < 4; ++k) {
-            g_launches++;
-            k_opt_sweep<<<grid_for(P.wb8), kThreads, 0, s>>>(P);
-        }
-        sweeps += 4;
-        uint32_t changed = 0;
-        cudaMemcpyAsync(&changed, P.flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-        const cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) return e;
-        if (!changed) break;
-        if (sweeps > P.W + 8u) break;  // cannot happen: every sweep clears a mark
-    }
-    g_launches++;
-    k_opt_final<<<grid_for(P.wb8), kThreads, 0, s>>>(P);
-    if (sweeps_out) *sweeps_out = sweeps;
-    return cudaGetLastError();
 }
 
 // Shape of the register allocation launch: T threads (at least 64, one per physical
@@ -2649,73 +2646,101 @@ struct BSortOut {
 // clears make another sweep necessary; otherwise every tile is swept until a sweep
 // changes nothing.  The block writes back zeros only, so clears by other blocks are
 // never undone.
+// sweep_tile: one tile of a program to its fixed point; marks in next (the program's tiles)
+// the tiles whose marks it cleared.  Returns (block-uniform) whether it cleared marks of
+// other tiles (bit 0) or its own (bit 1).
+template <uint32_t TILE>
+__device__ uint32_t sweep_tile(const Prog& P, uint32_t base, uint8_t* s_used, uint8_t* next) {
+    constexpr uint32_t kSweepItems = TILE / kThreads;
+    static_assert(kSweepItems >= 1 && kSweepItems <= 32, "pending bits");
+    const uint32_t W = P.W, lim = min(TILE, P.wb8 - base);
+    uint32_t rd[kSweepItems], r1[kSweepItems], r2[kSweepItems];
+    uint32_t pending = 0;  // bit e: instruction e of this thread may still act
+#pragma unroll
+    for (uint32_t e = 0; e < kSweepItems; ++e) {
+        const uint32_t k = threadIdx.x + e * kThreads;
+        if (k < lim) {
+            s_used[k] = P.used[base + k];
+            rd[e] = P.rd[base + k];
+            r1[e] = P.rs1[base + k];
+            r2[e] = P.rs2[base + k];
+            if (s32(rd[e]) > 63) pending |= 1u << e;
+        }
+    }
+    __syncthreads();
+    bool cross = false, local = false;
+    for (;;) {
+        bool ch = false;
+#pragma unroll
+        for (uint32_t e = 0; e < kSweepItems; ++e) {
+            if (!((pending >> e) & 1u)) continue;
+            const uint32_t r = rd[e] - 64u;
+            if (r >= W) {
+                record_error(P.err, ST_UNSUPPORTED, W_OPT, base + threadIdx.x + e * kThreads);
+                pending &= ~(1u << e);
+                continue;
+            }
+            const bool live = r - base < lim ? s_used[r - base] != 0
+                                             : *reinterpret_cast<const volatile uint8_t*>(&P.used[r]) != 0;
+            if (live) continue;
+            pending &= ~(1u << e);  // dead: its operands lose their marks, once
+#pragma unroll
+            for (uint32_t o = 0; o < 2; ++o) {
+                const int32_t a = s32((o == 0 ? r1[e] : r2[e]) - 64u);
+                if (a < 0 || u32(a) >= W || P.smark[a]) continue;
+                if (u32(a) - base < lim) {
+                    if (s_used[u32(a) - base]) { s_used[u32(a) - base] = 0; ch = true; }
+                } else if (*reinterpret_cast<volatile uint8_t*>(&P.used[a])) {
+                    P.used[a] = 0;
+                    next[u32(a) / TILE] = 1;
+                    cross = true;
+                }
+            }
+        }
+        local |= ch;
+        if (!__syncthreads_or(ch)) break;
+    }
+#pragma unroll
+    for (uint32_t e = 0; e < kSweepItems; ++e) {
+        const uint32_t k = threadIdx.x + e * kThreads;
+        if (k < lim && s_used[k] == 0) P.used[base + k] = 0;
+    }
+    return (__syncthreads_or(cross) ? 1u : 0u) | (__syncthreads_or(local) ? 2u : 0u);
+}
+
 template <uint32_t TILE>
 __global__ void __launch_bounds__(kThreads) k_batch_sweep(const Prog* progs, const uint32_t* off, uint32_t B,
                                                           uint32_t total, uint32_t* changed, const uint8_t* cur,
                                                           uint8_t* next) {
-    constexpr uint32_t kSweepItems = TILE / kThreads;
-    static_assert(kSweepItems >= 1 && kSweepItems <= 32, "pending bits");
     __shared__ uint8_t s_used[TILE];
     if (cur && !cur[total]) return;  // no tile was marked: nothing to sweep
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
         if (cur && !cur[t]) continue;  // block-uniform
         const uint32_t p = batch_program(off, B, t);
-        const Prog& P = progs[p];
-        const uint32_t base = (t - off[p]) * TILE;
-        const uint32_t W = P.W, lim = min(TILE, P.wb8 - base);
-        uint32_t rd[kSweepItems], r1[kSweepItems], r2[kSweepItems];
-        uint32_t pending = 0;  // bit e: instruction e of this thread may still act
-#pragma unroll
-        for (uint32_t e = 0; e < kSweepItems; ++e) {
-            const uint32_t k = threadIdx.x + e * kThreads;
-            if (k < lim) {
-                s_used[k] = P.used[base + k];
-                rd[e] = P.rd[base + k];
-                r1[e] = P.rs1[base + k];
-                r2[e] = P.rs2[base + k];
-                if (s32(rd[e]) > 63) pending |= 1u << e;
-            }
+        const uint32_t did = sweep_tile<TILE>(progs[p], (t - off[p]) * TILE, s_used, next + off[p]);
+        if (threadIdx.x == 0) {
+            if (did & 1u) next[total] = 1;  // some tile is marked
+            if ((did & 1u) || (cur == nullptr && did)) *changed = 1u;
         }
-        __syncthreads();
-        bool cross = false, local = false;
-        for (;;) {
-            bool ch = false;
-#pragma unroll
-            for (uint32_t e = 0; e < kSweepItems; ++e) {
-                if (!((pending >> e) & 1u)) continue;
-                const uint32_t r = rd[e] - 64u;
-                if (r >= W) {
-                    record_error(P.err, ST_UNSUPPORTED, W_OPT, base + threadIdx.x + e * kThreads);
-                    pending &= ~(1u << e);
-                    continue;
-                }
-                const bool live = r - base < lim ? s_used[r - base] != 0
-                                                 : *reinterpret_cast<const volatile uint8_t*>(&P.used[r]) != 0;
-                if (live) continue;
-                pending &= ~(1u << e);  // dead: its operands lose their marks, once
-#pragma unroll
-                for (uint32_t o = 0; o < 2; ++o) {
-                    const int32_t a = s32((o == 0 ? r1[e] : r2[e]) - 64u);
-                    if (a < 0 || u32(a) >= W || P.smark[a]) continue;
-                    if (u32(a) - base < lim) {
-                        if (s_used[u32(a) - base]) { s_used[u32(a) - base] = 0; ch = true; }
-                    } else if (*reinterpret_cast<volatile uint8_t*>(&P.used[a])) {
-                        P.used[a] = 0;
-                        next[off[p] + u32(a) / TILE] = 1;
-                        next[total] = 1;  // some tile is marked
-                        cross = true;
-                    }
-                }
-            }
-            local |= ch;
-            if (!__syncthreads_or(ch)) break;
+    }
+}
+
+// One program's sweep number k of a run (see k_batch_sweep): run[k] says whether there is
+// anything to do, run[k + 1] whether another sweep has to follow.  P.flags[0] (set by
+// k_opt_mark): some virtual result is not its instruction's own word, so every tile is
+// swept until a sweep changes nothing; else only the tiles marked in cur.
+__global__ void __launch_bounds__(kThreads) k_opt_sweep(Prog P, uint32_t tiles, uint8_t* cur, uint8_t* next, uint32_t* run,
+                                                        uint32_t k) {
+    __shared__ uint8_t s_used[kOptTile];
+    if (!run[k]) return;
+    const bool all = P.flags[0] != 0;
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        if (!all && !cur[t]) continue;  // block-uniform
+        const uint32_t did = sweep_tile<kOptTile>(P, t * kOptTile, s_used, next);
+        if (threadIdx.x == 0) {
+            cur[t] = 0;  // the next sweep's next
+            if ((did & 1u) || (all && did)) run[k + 1u] = 1u;
         }
-#pragma unroll
-        for (uint32_t e = 0; e < kSweepItems; ++e) {
-            const uint32_t k = threadIdx.x + e * kThreads;
-            if (k < lim && s_used[k] == 0) P.used[base + k] = 0;
-        }
-        if (__syncthreads_or(cross || (cur == nullptr && local)) && threadIdx.x == 0) *changed = 1u;
     }
 }
 
@@ -2964,6 +2989,42 @@ void batch_launch(const BatchLaunch& bl, uint32_t total, const Op& op) {
 }  // namespace
 
 static_assert(sizeof(Prog) % 8 == 0, "Prog copies in 8-byte words");
+
+size_t optimize_work_bytes(uint32_t W) {
+    return 64u + 2u * ((static_cast<size_t>((W + 7u) & ~7u) + kOptTile - 1u) / kOptTile + 16u);
+}
+
+cudaError_t run_optimize(const Prog& P, void* work, cudaStream_t s, uint32_t* sweeps_out) {
+    // work: whether sweep k has anything to do, then the tiles marked for it and the next
+    uint32_t* run = static_cast<uint32_t*>(work);
+    const uint32_t tiles = (P.wb8 + kOptTile - 1u) / kOptTile;
+    uint8_t* dirty[2] = {static_cast<uint8_t*>(work) + 64, static_cast<uint8_t*>(work) + 64 + tiles};
+    // Marks cleared in other tiles make further sweeps, a few of them; a lone tile needs one
+    // (when every result is its own word).  A sweep with nothing to do returns at once.
+    const uint32_t batch = tiles == 1u ? 1u : kOptSweeps;
+    g_launches++;
+    k_opt_mark<<<grid_for(P.wb8), kThreads, 0, s>>>(P, tiles, dirty[0], dirty[1], run);
+    uint32_t sweeps = 0;
+    for (;;) {
+        for (uint32_t k = 0; k < batch; ++k) {
+            g_launches++;
+            k_opt_sweep<<<std::min<unsigned>(tiles, 152u * 8u), kThreads, 0, s>>>(P, tiles, dirty[sweeps & 1u],
+                                                                             dirty[(sweeps & 1u) ^ 1u], run, k);
+            ++sweeps;
+        }
+        uint32_t more = 0;
+        cudaMemcpyAsync(&more, run + batch, sizeof(more), cudaMemcpyDeviceToHost, s);
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return e;
+        if (!more) break;
+        if (sweeps > P.W + 8u) break;  // cannot happen: every sweep clears a mark
+        cudaMemsetAsync(run + 1, 0, kOptSweeps * sizeof(uint32_t), s);
+    }
+    g_launches++;
+    k_opt_final<<<grid_for(P.wb8), kThreads, 0, s>>>(P);
+    if (sweeps_out) *sweeps_out = sweeps;
+    return cudaGetLastError();
+}
 
 uint32_t batch_tile() { return kBTile; }
 uint32_t batch_scan_tile() { return kScanTile; }

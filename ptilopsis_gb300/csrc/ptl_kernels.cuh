@@ -71,7 +71,9 @@ void launch_decl_scan(const Prog& P, uint32_t* flags_tmp, const ScanScratch& sc,
 void launch_functab(const Prog& P, uint32_t* meta, cudaStream_t s);
 
 void launch_gen(const Prog& P, cudaStream_t s);
-cudaError_t run_optimize(const Prog& P, cudaStream_t s, uint32_t* sweeps_out);
+// work: optimize_work_bytes(W) of scratch, 16-byte aligned.
+size_t optimize_work_bytes(uint32_t W);
+cudaError_t run_optimize(const Prog& P, void* work, cudaStream_t s, uint32_t* sweeps_out);
 // Register allocation of one program.  ra_form builds the step records (P.rec) and tells
 // which form the program takes; the caller then provides that form's arrays:
 //   Steps: tmask (one per word), trow and tany (row_tiles(S) tiles of kRowTile steps);
