@@ -17,7 +17,7 @@ from typing import List, Optional, Sequence
 
 import numpy as np
 
-from .codegen import DepthTree, PtlError, _AstView, _view, device_info, lib
+from .codegen import DepthTree, PtlError, _AstView, _copy_u32, _view, device_info, lib
 
 _u32p = ctypes.POINTER(ctypes.c_uint32)
 
@@ -78,7 +78,7 @@ def _bind(L):
 def _arr(p, n) -> np.ndarray:
     if n == 0:
         return np.zeros(0, np.uint32)
-    return np.ctypeslib.as_array(p, shape=(n,)).copy()
+    return _copy_u32(p, n)
 
 
 @dataclass
