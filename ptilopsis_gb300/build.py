@@ -29,7 +29,7 @@ CUDA_LIB = os.path.join(LIBDIR, "libptl_gb300.so")
 SYNTH_LIB = os.path.join(LIBDIR, "libptlsynth.so")
 HOSTMODEL_LIB = os.path.join(LIBDIR, "libptl_hostmodel.so")
 
-HEADERS = ["ptl_device.h", "ptl_common.cuh", "ptl_stages.cuh", "ptl_sort.cuh", "ptl_ra.cuh", "ptl_steps.cuh", "ptl_scalar.cuh", "ptl_kernels.cuh",
+HEADERS = ["ptl_device.h", "ptl_common.cuh", "ptl_stages.cuh", "ptl_sort.cuh", "ptl_ra.cuh", "ptl_steps.cuh", "ptl_chunks.cuh", "ptl_scalar.cuh", "ptl_kernels.cuh",
            "ptl_bpipe.h"]
 
 
@@ -59,7 +59,7 @@ def _src(*names: str) -> list[str]:
 
 def build_cuda(force: bool = False) -> str:
     hdrs = _src(*HEADERS) + [os.path.join(ROOT, "include", "ptl_codegen.h")]
-    units = [("ptl_kernels.cu", "nvcc"), ("ptl_regalloc.cu", "nvcc"), ("ptl_capi.cu", "nvcc"), ("ptl_noalloc.cu", "nvcc"), ("ptl_bpipe.cu", "nvcc"),
+    units = [("ptl_kernels.cu", "nvcc"), ("ptl_regalloc.cu", "nvcc"), ("ptl_chunks.cu", "nvcc"), ("ptl_capi.cu", "nvcc"), ("ptl_noalloc.cu", "nvcc"), ("ptl_bpipe.cu", "nvcc"),
              ("ptl_flatten.cu", "nvcc"), ("ptl_tables.cpp", "cxx"), ("ptl_batch.cpp", "cxx"), ("ptl_disasm.cpp", "cxx"), ("ptl_elf.cpp", "cxx")]
     all_src = _src(*(u for u, _ in units)) + hdrs
     if not force and _newer(CUDA_LIB, all_src):
@@ -92,7 +92,7 @@ def build_synth(force: bool = False) -> str:
 
 def build_hostmodel(force: bool = False) -> str:
     srcs = _src("ptl_hostmodel.cpp", "ptl_tables.cpp", "ptl_common.cuh", "ptl_stages.cuh", "ptl_sort.cuh", "ptl_ra.cuh", "ptl_steps.cuh",
-                "ptl_scalar.cuh")
+                "ptl_chunks.cuh", "ptl_scalar.cuh")
     if not force and _newer(HOSTMODEL_LIB, srcs):
         return HOSTMODEL_LIB
     os.makedirs(LIBDIR, exist_ok=True)

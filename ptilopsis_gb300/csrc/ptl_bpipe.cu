@@ -137,7 +137,7 @@ public:
     DBuf nt, rt, nd1, nd, par, ci, dep, loc0, loc, pos, decl, fflag, regs;
     DBuf fn_id, fn_start, fn_size, fn_end, fn_start0, fn_size0, ra_order, lifetime;
     DBuf instr, rd, rs1, rs2, jt, used_instrs, symreg, symswp, stamp, spill, roffs, owner, used, smark, defpos;
-    DBuf tmask, trow, tany;
+    DBuf tmask, trow, tany, lane_zero, lane_rest;
     DBuf trig_min, trig_max, ra_chunks;
     DBuf ni, nrd, nr1, nr2, njt, joffs, out;
     DBuf errw, flags, meta, progs, tabs, lists, changed, sort_err, a_off, dirty, ra_sync;
@@ -171,7 +171,7 @@ public:
         return {&tab, &in_type, &in_rtype, &in_parent, &in_depth, &in_child, &in_data, &nt, &rt, &nd1, &nd, &par,
                 &ci, &dep, &loc0, &loc, &pos, &decl, &fflag, &regs, &fn_id, &fn_start, &fn_size,
                 &fn_end, &fn_start0, &fn_size0, &ra_order, &lifetime, &instr, &rd, &rs1, &rs2, &jt, &used_instrs, &symreg,
-                &symswp, &stamp, &spill, &roffs, &owner, &used, &smark, &defpos, &tmask, &trow, &tany, &trig_min, &trig_max, &ra_chunks, &ni, &nrd,
+                &symswp, &stamp, &spill, &roffs, &owner, &used, &smark, &defpos, &tmask, &trow, &tany, &lane_zero, &lane_rest, &trig_min, &trig_max, &ra_chunks, &ni, &nrd,
                 &nr1, &nr2, &njt, &joffs, &out, &errw, &flags, &meta, &progs, &tabs, &lists, &changed,
                 &sort_err, &a_off, &dirty, &ra_sync, &sa, &sapos, &sbpos, &seg0, &seg1, &tile_seg, &tile_l, &tile_r,
                 &sort_stops, &leaf, &heap, &counters, &scan_status, &scan_counter, &sort_local, &sort_equal,
@@ -425,7 +425,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
     for (auto& x : hns) x = 0;
 
     // ---- small per-program state and the pinned small area
-    constexpr int kTables = 25, kLists = 5;  // table slots 0..24 are used
+    constexpr int kTables = 27, kLists = 6;  // table slots 0..26 are used
     small_progs_off = static_cast<size_t>(kTables) * (B + 1) * 4;
     small_meta_off = small_progs_off + B * sizeof(Prog);
     small_err_off = small_meta_off + B * 16;
@@ -895,6 +895,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
             if (sr != PTL_OK) return sr;
         } else {
         const uint32_t t_f = tiles(6, F, elem_tile);
+        BP_CU(cudaMemsetAsync(flags.p, 0, B * 16, s));
         batch_stage(BatchStage::InitLifetime, bl(6), t_f, nullptr);
         const uint32_t t_w = tiles(7, W, elem_tile);
         batch_stage(BatchStage::Records, bl(7), t_w, nullptr);
@@ -902,7 +903,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
         BP_CU(collect_errors());
         // every program takes the record form, except one whose words a record cannot say
         // (the general form) or whose functions share symbols (the serial order)
-        std::vector<uint32_t> step_list, wide_steps, lane0_list, serial_list, wide_list;
+        std::vector<uint32_t> step_list, chunk_list, wide_steps, lane0_list, serial_list, wide_list;
         std::vector<uint8_t> steps(B, 0), general(B, 0), lane0(B, 0);
         std::vector<uint64_t> nfree(B, 0);
         uint32_t max_g0 = 1, max_step_g0 = 1;
@@ -958,6 +959,62 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
                 hp[p].tany = tany.at<uint32_t>(La.elem(p));
             }
         }
+        // the long programs have their lane-0 functions in chunks where that pays; one run of a kernel has those of step_list, and each of the widest
+        // has its own
+        std::vector<ChunkSizes> chunk(B);
+        std::vector<uint8_t> in_chunks(B, 0);
+        ChunkBatch chunks{};
+        uint64_t zero_bytes = 0, rest_bytes = 0, sync_words = 0;
+        auto groups = [&](uint32_t p) { return static_cast<uint32_t>((F[p] + 7) / 8); };
+        auto long_enough = [&](uint32_t p) { return S[p] >= kChunkMinSteps && hfl[4 * p] != 0; };
+        auto put_in_chunks = [&](uint32_t p) {
+            in_chunks[p] = 1;
+            chunk[p] = chunk_sizes(static_cast<uint32_t>(F[p]), static_cast<uint32_t>(S[p]), static_cast<uint32_t>(W[p]), hfl[4 * p]);
+            zero_bytes += chunk[p].zeroed;
+            rest_bytes += chunk[p].total - chunk[p].zeroed;
+        };
+        size_t taken = 0;  // of step_list, longest first
+        uint64_t work = 0, before = 0, after = 0;  // before, after: the lock-step's time
+        for (size_t k = 0; k < step_list.size(); ++k) {
+            const uint32_t p = step_list[k];
+            const uint64_t t = lock_step_cycles(S[p], groups(p));
+            before = std::max(before, t);
+            if (long_enough(p) && taken == k) {
+                ++taken;
+                work += chunk_work(row_tiles(S[p]), groups(p));
+            } else {
+                after = std::max(after, t);
+            }
+        }
+        if (taken && !chunk_pays(row_tiles(S[step_list[0]]), work, before, after)) taken = 0;
+        for (size_t k = 0; k < taken; ++k) {
+            const uint32_t p = step_list[k];
+            put_in_chunks(p);
+            chunks.classes |= chunk_class(groups(p));
+            chunks.rounds = std::max(chunks.rounds, chunk_rounds(static_cast<uint32_t>(chunk[p].tiles)));
+        }
+        for (const uint32_t p : wide_steps) {
+            if (!long_enough(p)) continue;
+            put_in_chunks(p);
+            sync_words += chunk_sync_words(chunk_rounds(static_cast<uint32_t>(chunk[p].tiles)));
+        }
+        for (const uint32_t p : step_list)
+            if (in_chunks[p]) chunk_list.push_back(p);
+        if (!chunk_list.empty()) sync_words += chunk_sync_words(chunks.rounds);
+        uint64_t sync_at = zero_bytes / 4;  // of the next words for a kernel's rounds
+        if (zero_bytes) {
+            zero_bytes += 4 * sync_words;
+            BP_CU(lane_zero.ensure(zero_bytes));
+            BP_CU(lane_rest.ensure(rest_bytes));
+            BP_CU(cudaMemsetAsync(lane_zero.p, 0, zero_bytes, s));
+            uint64_t z = 0, r = 0;
+            for (size_t p = 0; p < B; ++p) {
+                if (!in_chunks[p]) continue;
+                chunk_bind(hp[p].ch, chunk[p], lane_zero.at<char>(z), lane_rest.at<char>(r));
+                z += chunk[p].zeroed;
+                r += chunk[p].total - chunk[p].zeroed;
+            }
+        }
         if (lane0_list.size() + wide_list.size() > 0) {
             std::vector<uint64_t> chunk_words(B);
             for (size_t p = 0; p < B; ++p) chunk_words[p] = 2 * (S[p] / 32 + 2);
@@ -985,6 +1042,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
                 hf[k] = nf;
                 hr[k] = nr;
                 nf += static_cast<uint32_t>((nfree[step_list[k]] + 31) / 32);
+                if (in_chunks[step_list[k]]) nf += static_cast<uint32_t>((F[step_list[k]] - nfree[step_list[k]] + 31) / 32);
                 nr += static_cast<uint32_t>(row_tiles(S[step_list[k]]));
             }
             for (size_t k = step_list.size(); k <= B; ++k) {
@@ -993,11 +1051,32 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
             }
             BP_CU(cudaMemcpyAsync(dtable_slot(8), hf, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
             BP_CU(cudaMemcpyAsync(dtable_slot(23), hr, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+            if (!chunk_list.empty()) {
+                uint32_t* hr2 = table_slot(25);
+                uint32_t* ht = table_slot(26);
+                for (size_t k = 0; k <= B; ++k) {
+                    hr2[k] = chunks.runs;
+                    ht[k] = chunks.tiles;
+                    if (k < chunk_list.size()) {
+                        chunks.runs += static_cast<uint32_t>(chunk[chunk_list[k]].runs);
+                        chunks.tiles += static_cast<uint32_t>(chunk[chunk_list[k]].tiles);
+                    }
+                }
+                BP_CU(cudaMemcpyAsync(dtable_slot(25), hr2, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+                BP_CU(cudaMemcpyAsync(dtable_slot(26), ht, (B + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+                chunks.progs = progs.at<Prog>();
+                chunks.order = upload_list(5, chunk_list);
+                chunks.run_off = dtable_slot(25);
+                chunks.tile_off = dtable_slot(26);
+                chunks.n = static_cast<uint32_t>(chunk_list.size());
+                chunks.sync = lane_zero.at<uint32_t>(sync_at);
+                sync_at += chunk_sync_words(chunks.rounds);
+            }
             const uint32_t* d_steps = upload_list(0, step_list);
             const uint32_t count = static_cast<uint32_t>(step_list.size());
             batch_free_order(progs.at<Prog>(), d_steps, count, s);
             BP_CU(batch_step_regalloc(StepBatch{progs.at<Prog>(), d_steps, dtable_slot(8), dtable_slot(23), count, nf, nr,
-                                                max_step_g0, 0}, s));
+                                                max_step_g0, 0, chunk_list.empty() ? nullptr : &chunks}, s));
         }
         if (!lane0_list.empty()) {
             // independent functions and lane-0 passes in one persistent launch
@@ -1023,7 +1102,17 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
         for (const uint32_t p : wide_steps) {
             Prog one = hp[p];
             one.ra_order = nullptr;
-            BP_CU(run_step_regalloc(one, s));
+            ChunkBatch c{};
+            if (in_chunks[p]) {
+                c.n = 1;
+                c.runs = static_cast<uint32_t>(chunk[p].runs);
+                c.tiles = static_cast<uint32_t>(chunk[p].tiles);
+                c.classes = chunk_class(static_cast<uint32_t>((F[p] + 7) / 8));
+                c.rounds = chunk_rounds(c.tiles);
+                c.sync = lane_zero.at<uint32_t>(sync_at);
+                sync_at += chunk_sync_words(c.rounds);
+            }
+            BP_CU(run_step_regalloc(one, in_chunks[p] ? &c : nullptr, s));
         }
         const uint32_t* d_serial = upload_list(1, serial_list);
         batch_serial(progs.at<Prog>(), d_serial, static_cast<uint32_t>(serial_list.size()), s);

@@ -97,7 +97,7 @@ struct ptl_generator {
     DevBuf decl, fn_id, fn_start, fn_size, fn_end, fn_start0, fn_size0, fn_end0;
     DevBuf fn_ra_start, fn_ra_end, fn_ra_size;
     DevBuf instr, rd, rs1, rs2, jt, owner, used, smark, used_instrs;
-    DevBuf tmask, trow, tany, opt_work;
+    DevBuf tmask, trow, tany, lane_zero, lane_rest, opt_work;
     DevBuf symreg, symswp, stamp, defpos, lifetime, trig_min, trig_max, ra_chunks, spill, roffs;
     DevBuf ni, nrd, nr1, nr2, njt, fsz, joffs, out;
     DevBuf sort_a, sort_apos, sort_bpos, sort_seg0, sort_seg1, sort_tile_seg, sort_tile_l, sort_tile_r, sort_stops,
@@ -141,7 +141,7 @@ struct ptl_generator {
         return {&in_type, &in_rtype, &in_parent, &in_depth, &in_child, &in_data, &nt, &rt, &nd1, &nd,
                 &par, &ci, &dep, &fflag, &sizes, &loc0, &loc, &pos, &regs, &decl, &fn_id, &fn_start,
                 &fn_size, &fn_end, &fn_start0, &fn_size0, &fn_end0, &fn_ra_start, &fn_ra_end, &fn_ra_size,
-                &instr, &rd, &rs1, &rs2, &jt, &owner, &used, &smark, &used_instrs, &tmask, &trow, &tany, &opt_work, &symreg, &symswp,
+                &instr, &rd, &rs1, &rs2, &jt, &owner, &used, &smark, &used_instrs, &tmask, &trow, &tany, &lane_zero, &lane_rest, &opt_work, &symreg, &symswp,
                 &stamp, &defpos, &lifetime, &trig_min, &trig_max, &ra_chunks, &spill, &roffs, &ni, &nrd, &nr1, &nr2, &njt,
                 &fsz, &joffs, &out, &sort_a, &sort_apos, &sort_bpos, &sort_seg0, &sort_seg1, &sort_stops,
                 &sort_tile_seg, &sort_tile_l, &sort_tile_r, &sort_leaf, &sort_heap, &sort_counters, &sort_local, &sort_equal,
@@ -660,7 +660,25 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
         if (!prog_ready(P, {P.lifetime, P.rec}))
             return fail(g, PTL_CUDA_ERROR, "internal: unallocated regalloc state");
         RaForm form = RaForm::Serial;
-        PTL_CU(ra_form(P, s, row0_hash, &form));
+        uint32_t items = 0;
+        PTL_CU(ra_form(P, s, row0_hash, &form, &items));
+        ChunkSizes chunk{};
+        ChunkBatch chunks{};
+        const bool in_chunks = form == RaForm::Steps && items != 0 && g->S >= kChunkMinSteps;
+        if (in_chunks) {
+            chunk = chunk_sizes(g->F, g->S, g->W, items);
+            const uint32_t rounds = chunk_rounds(static_cast<uint32_t>(chunk.tiles));
+            const size_t sync = 4ull * chunk_sync_words(rounds);
+            PTL_CU(g->lane_zero.ensure((chunk.zeroed + sync + 15u) / 16u, 16));
+            PTL_CU(g->lane_rest.ensure((chunk.total - chunk.zeroed + 15u) / 16u, 16));
+            PTL_CU(g->lane_zero.zero(s));
+            chunks.n = 1;
+            chunks.runs = static_cast<uint32_t>(chunk.runs);
+            chunks.tiles = static_cast<uint32_t>(chunk.tiles);
+            chunks.classes = chunk_class((g->F + 7u) / 8u);
+            chunks.rounds = rounds;
+            chunks.sync = reinterpret_cast<uint32_t*>(g->lane_zero.at<char>() + chunk.zeroed);
+        }
         if (form == RaForm::Steps) {
             const size_t steps = row_tiles(g->S) * kRowTile;
             PTL_CU(g->tmask.ensure(wb8, 4));
@@ -679,7 +697,8 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
                                   : form == RaForm::General && !prog_ready(P, {P.trig_min, P.trig_max, P.ra_chunks}))
             return fail(g, PTL_CUDA_ERROR, "internal: unallocated regalloc state");
         P.defpos = nullptr;
-        PTL_CU(run_regalloc_steps(P, form, s));
+        if (in_chunks) chunk_bind(P.ch, chunk, g->lane_zero.at<char>(), g->lane_rest.at<char>());
+        PTL_CU(run_regalloc_steps(P, form, in_chunks ? &chunks : nullptr, s));
         g->ra_serial = form == RaForm::Serial;
         PTL_CU(scan_for(wb8, &sc));
         launch_regalloc_count_scan(P, sc, s);

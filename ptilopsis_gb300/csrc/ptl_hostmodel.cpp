@@ -17,13 +17,15 @@
 #include "ptl_sort.cuh"
 #include "ptl_stages.cuh"
 #include "ptl_ra.cuh"
-#include "ptl_steps.cuh"
+#include "ptl_chunks.cuh"
 #include "ptl_scalar.cuh"
 
 using namespace ptl;
 
 namespace {
 
+bool g_last_locked = false;  // the last program's symbols did not fit the slots
+bool g_chunks = true;  // lane-0 functions in chunks (else in lock-step)
 uint32_t g_ring_k = 16;  // words per function in the record form's symbol ring (small: old words too)
 uint32_t g_cache_k = 4;  // entries per function of the lane-0 symbol cache
 bool g_force_hashed = false;  // lane-0 pass finds row-0 values by hashing even when definitions are unique
@@ -215,6 +217,88 @@ struct Model {
         P = Psave;
     }
 
+    // The lane-0 functions in chunks (ptl_chunks.cuh), round by round as its kernel runs
+    // them (the runs of a round one after the other).  False: the rounds ran out.
+    bool chunk_lanes(uint32_t S, uint32_t K) {
+        const uint32_t G0 = (P.F + 7) / 8, tiles = static_cast<uint32_t>(row_tiles(S)), rounds = tiles + 64;
+        const size_t steps = static_cast<size_t>(tiles) * kRowTile;
+        auto size = [&](uint32_t j) { return static_cast<uint32_t>(std::max(s32(P.fn_size0[8 * j]), 0)); };
+        std::vector<uint32_t> off(G0 + 1);
+        for (uint32_t j = 0; j < G0; ++j) off[j + 1] = off[j] + chunks_of(P, j);
+        const size_t items = off[G0];
+        std::vector<uint32_t> last(P.W, 0), slots(G0), need(items + 1, 0), delta(2 * steps, 0), dirty(tiles, 0), moved(tiles, 0);
+        std::vector<unsigned long long> rec(items * kChunk);
+        std::vector<ChunkVec> out(items * kChunk / 2), state((items + 1) * kStateVecs);
+        std::vector<uint32_t> row(steps * kRowPos), mem(kChunkMemWords);
+        std::vector<uint16_t> win(steps * kRowPos);
+        std::vector<ChunkPair> pair(steps);
+        std::vector<uint32_t> touch(tiles, 0);
+        uint32_t lock = 0;
+        P.ch = LaneChunks{last.data(), off.data(), slots.data(), rec.data(), need.data(), out.data(), state.data(), row.data(),
+                          win.data(), pair.data(), touch.data(), nullptr, delta.data(), dirty.data(), moved.data(), &lock};
+        std::vector<uint8_t> ring(K);
+        for (uint32_t j = 0; j < G0; ++j)
+            for (uint32_t i = 0; i < size(j); ++i) chunk_last_read(P, P.fn_start0[8 * j] + i);
+        for (uint32_t j = 0; j < G0; ++j) step_slot_function(P, j, ring.data(), 1, K);
+        g_last_locked = lock != 0;
+        if (lock) return false;
+        const std::vector<uint16_t> no_win(kChunk * kRowPos, 0);
+        for (uint32_t round = 1;; ++round) {
+            const bool first = round == 1;
+            bool changed = false;
+            for (uint32_t c = 0; c < tiles; ++c) {
+                const size_t at = static_cast<size_t>(c) * kChunk;
+                std::vector<ChunkPair> none(kChunk);
+                for (uint32_t t = 0; t < kChunk; ++t) none[t] = ChunkPair{P.tany[at + t], 0};
+                const ChunkRows rows = first ? ChunkRows{P.trow + at * kRowPos, no_win.data(), none.data()}
+                                             : ChunkRows{&row[at * kRowPos], &win[at * kRowPos], &pair[at]};
+                for (uint32_t j = 0; j < G0; ++j) {
+                    if (size(j) <= c * kChunk || !(first || moved[c] == round || need[off[j] + c] >= round)) continue;
+                    const uint32_t r = chunk_run<false>(P, rows, mem.data(), j, c, true, first);
+                    if (r & kChunkNext) { need[off[j] + c + 1] = round + 1; changed = true; }
+                    if (r & kChunkOut) dirty[c] = round;
+                }
+            }
+            for (uint32_t c = 0; c < tiles; ++c) {
+                if (!first && dirty[c] != round) continue;
+                for (uint32_t t = 0; t < kChunk; ++t) {
+                    const size_t i = static_cast<size_t>(c) * kChunk + t;
+                    ChunkPair x{P.tany[i], 0};
+                    std::vector<uint32_t> r(P.trow + i * kRowPos, P.trow + (i + 1) * kRowPos);
+                    uint16_t w[kRowPos] = {};
+                    for (uint32_t j = 0; j < G0; ++j) {
+                        if (size(j) <= c * kChunk) continue;
+                        const uint32_t* o = reinterpret_cast<const uint32_t*>(out.data()) + (static_cast<size_t>(off[j] + c) * kChunk + t) * 2;
+                        x.wr |= o[0];
+                        x.any |= o[1];
+                        for (uint32_t m = o[0]; m; m &= m - 1) w[low_bit(m)] = static_cast<uint16_t>(j + 1);
+                        for (uint32_t m = o[1]; m; m &= m - 1) {
+                            uint32_t& v = r[low_bit(m)];
+                            v = std::min(row_min(v), j + 1) | std::max(row_max(v), j + 1) << 16;
+                        }
+                    }
+                    if (first || !std::equal(r.begin(), r.end(), &row[i * kRowPos]) || !std::equal(w, w + kRowPos, &win[i * kRowPos])) {
+                        moved[c] = round + 1;
+                        changed = true;
+                    }
+                    std::copy(r.begin(), r.end(), &row[i * kRowPos]);
+                    std::copy(w, w + kRowPos, &win[i * kRowPos]);
+                    pair[i] = x;
+                }
+            }
+            if (!changed) break;
+            if (round >= rounds) return false;
+        }
+        for (size_t i = 0; i < steps; ++i) touch[i / kChunk] |= pair[i].any | pair[i].wr;
+        for (uint32_t c = 0; c < tiles; ++c) {
+            const size_t at = static_cast<size_t>(c) * kChunk;
+            for (uint32_t j = 0; j < G0; ++j)
+                if (size(j) > c * kChunk)
+                    chunk_run<true>(P, ChunkRows{&row[at * kRowPos], &win[at * kRowPos], &pair[at]}, mem.data(), j, c, true, false);
+        }
+        return true;
+    }
+
     // The record form's allocation (ptl_steps.cuh), phase by phase as its kernels run it.
     void step_regalloc(uint32_t S, uint32_t K) {
         std::vector<uint8_t> ring(K);
@@ -234,6 +318,7 @@ struct Model {
                 }
             }
         }
+        if (g_chunks && chunk_lanes(S, K)) return;
         LaneShared sh{};
         std::vector<uint8_t> rings(static_cast<size_t>(G0) * K);
         std::vector<LaneSlot> L(G0);
@@ -538,6 +623,8 @@ int ptlhm_gen_desc_ok(void) {
     build_code_tables(&t);
     return gen_desc_ok(&t) ? 1 : 0;
 }
+int ptlhm_last_locked(void) { return g_last_locked ? 1 : 0; }
+void ptlhm_set_chunks(int on) { g_chunks = on != 0; }
 void ptlhm_set_scalar_tiles(int on) { g_force_tiles = on != 0; }
 void ptlhm_set_scalar_serial(int on) { g_force_serial = on != 0; }
 

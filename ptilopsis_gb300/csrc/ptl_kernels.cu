@@ -14,9 +14,29 @@
 
 #include "ptl_kernels.cuh"
 #include "ptl_ra.cuh"
-#include "ptl_steps.cuh"
+#include "ptl_chunks.cuh"
 
 namespace ptl {
+
+cudaError_t launch_cooperative(const void* kernel, uint32_t blocks, uint32_t threads, void** args, size_t smem, cudaStream_t s) {
+    struct Turn {
+        std::mutex m;
+        cudaEvent_t last = nullptr;  // the end of the device's last such launch
+    };
+    static Turn turns[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev >= 64) return cudaErrorInvalidDevice;
+    Turn& t = turns[dev];
+    std::lock_guard<std::mutex> lock(t.m);
+    if (t.last) e = cudaStreamWaitEvent(s, t.last, 0);
+    else e = cudaEventCreateWithFlags(&t.last, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(threads), args, smem, s);
+    if (e == cudaSuccess) e = cudaEventRecord(t.last, s);
+    return e;
+}
+
 
 // A kernel's largest dynamic shared memory is one attribute per function and device,
 // shared by every host thread: batched pipelines on several threads (the compile server's
@@ -1734,12 +1754,19 @@ __global__ void __launch_bounds__(kRaClusterThreads, 1)
 }
 
 // The step records; flags[1]: functions share symbols, flags[2]: a word that a record
-// cannot say, or function ranges that overlap.
+// cannot say, or function ranges that overlap; flags[0]: the lane-0 functions' chunks.
+__device__ void ra_count_chunks(const Prog& P, uint32_t f) {
+    const int32_t size = s32(P.fn_size0[f]);
+    if ((f & 7u) == 0 && size > 0) atomicAdd(P.flags, (static_cast<uint32_t>(size) + kChunk - 1u) / kChunk);
+}
 __global__ void k_ra_records(Prog P) {
     uint32_t any = 0;
     uint32_t hint = 0xFFFFFFFFu;
     PTL_FOR(i, P.W) any |= st_step_record(P, i, &hint);
-    PTL_FOR(f, P.F) any |= st_step_range(P, f);
+    PTL_FOR(f, P.F) {
+        any |= st_step_range(P, f);
+        ra_count_chunks(P, f);
+    }
     if (__syncthreads_or(any & 1u) && threadIdx.x == 0) P.flags[1] = 1;
     if (__syncthreads_or(any & 2u) && threadIdx.x == 0) P.flags[2] = 1;
 }
@@ -2180,8 +2207,7 @@ cudaError_t launch_ra_steps_q(const Prog& P0, const Prog& Pfree, uint32_t G0, ui
         Prog Pl = P0;
         void* args[] = {&Pl, &S, &K, &Kf, &chunks};
         g_launches++;
-        return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_ra_steps<Q>), dim3(1 + free_blocks),
-                                           dim3(T), args, smem, s);
+        return launch_cooperative(reinterpret_cast<const void*>(k_ra_steps<Q>), 1u + free_blocks, T, args, smem, s);
     }
     if (free_fns) {
         g_launches++;
@@ -2284,23 +2310,24 @@ cudaError_t launch_ra_steps(const Prog& P0, const Prog& Pfree, uint32_t G0, cuda
     }
 }
 
-cudaError_t ra_form(const Prog& P, cudaStream_t s, bool general, RaForm* form) {
-    cudaMemsetAsync(P.flags + 1, 0, 2 * sizeof(uint32_t), s);
+cudaError_t ra_form(const Prog& P, cudaStream_t s, bool general, RaForm* form, uint32_t* items) {
+    cudaMemsetAsync(P.flags, 0, 3 * sizeof(uint32_t), s);
     g_launches++;
     k_ra_records<<<grid_for(P.W), kThreads, 0, s>>>(P);
-    uint32_t fl[2] = {0, 0};
-    cudaMemcpyAsync(fl, P.flags + 1, sizeof(fl), cudaMemcpyDeviceToHost, s);
+    uint32_t fl[3] = {};
+    cudaMemcpyAsync(fl, P.flags, sizeof(fl), cudaMemcpyDeviceToHost, s);
     const cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return e;
     // functions that share symbols (or too many lane-0 functions) need the serial order
     const uint32_t G0 = (P.F + 7u) / 8u;
-    if (fl[0] || G0 > 8192u) *form = RaForm::Serial;
-    else if (fl[1] || general || (G0 > kStepBlockMax && (ra_cluster_disabled() || !step_cluster_fits(G0)))) *form = RaForm::General;
+    *items = fl[0];
+    if (fl[1] || G0 > 8192u) *form = RaForm::Serial;
+    else if (fl[2] || general || (G0 > kStepBlockMax && (ra_cluster_disabled() || !step_cluster_fits(G0)))) *form = RaForm::General;
     else *form = RaForm::Steps;
     return cudaSuccess;
 }
 
-cudaError_t run_regalloc_steps(const Prog& P, RaForm form, cudaStream_t s) {
+cudaError_t run_regalloc_steps(const Prog& P, RaForm form, const ChunkBatch* chunks, cudaStream_t s) {
     cudaError_t ce = cudaSuccess;
     if (form == RaForm::Serial) {
         g_launches++;
@@ -2308,7 +2335,7 @@ cudaError_t run_regalloc_steps(const Prog& P, RaForm form, cudaStream_t s) {
     } else if (form == RaForm::General) {
         ce = launch_ra_steps(P, P, (P.F + 7u) / 8u, s);
     } else {
-        ce = run_step_regalloc(P, s);
+        ce = run_step_regalloc(P, chunks, s);
     }
     if (ce != cudaSuccess) return ce;
     g_launches++;
@@ -2562,7 +2589,7 @@ struct BOptMark {
     }
 };
 PTL_BATCH_OP(BOptFinal, P.wb8, st_opt_final(P, i))
-PTL_BATCH_OP(BInitLifetime, P.F, P.lifetime[i] = 0x1Full; if (st_step_range(P, i)) P.flags[2] = 1u)
+PTL_BATCH_OP(BInitLifetime, P.F, P.lifetime[i] = 0x1Full; ra_count_chunks(P, i); if (st_step_range(P, i)) P.flags[2] = 1u)
 // spill flags and cross checks find each word's function from the thread's previous
 // word (the same program, 256 words earlier within a tile)
 struct BSpill {

@@ -46,6 +46,9 @@ uint64_t launch_count();
 void note_launch();
 // Raises a kernel's dynamic shared memory limit to at least bytes (never lowers it).
 cudaError_t allow_dynamic_smem(const void* kernel, size_t bytes);
+// A launch whose blocks wait on one another.  Launches from several streams take turns:
+// two that are each resident in part would wait for good.
+cudaError_t launch_cooperative(const void* kernel, uint32_t blocks, uint32_t threads, void** args, size_t smem, cudaStream_t s);
 
 // Up to kZeroMost memory ranges zeroed by one launch: a compile clears some 45 buffers,
 // and a memset of a small one costs the stream about 2 us whatever its size.  Ranges start
@@ -79,9 +82,56 @@ cudaError_t run_optimize(const Prog& P, void* work, cudaStream_t s, uint32_t* sw
 //   Steps: tmask (one per word), trow and tany (row_tiles(S) tiles of kRowTile steps);
 //   General: trig_min / trig_max (set to none), ra_chunks;
 //   Serial: none.
+struct ChunkBatch;
 enum class RaForm { Steps, General, Serial };
-cudaError_t ra_form(const Prog& P, cudaStream_t s, bool general, RaForm* form);
-cudaError_t run_regalloc_steps(const Prog& P, RaForm form, cudaStream_t s);
+// items: chunks of the lane-0 functions.
+cudaError_t ra_form(const Prog& P, cudaStream_t s, bool general, RaForm* form, uint32_t* items);
+cudaError_t run_regalloc_steps(const Prog& P, RaForm form, const ChunkBatch* chunks, cudaStream_t s);
+
+// The lane-0 functions in chunks of steps (ptl_chunks.cuh): of one program (progs null),
+// or of the programs order[0..n) of a batch, program order[k] having the run tiles
+// run_off[k].. (a chunk of 32 functions each) and the row tiles tile_off[k]..  sync:
+// chunk_sync_words zeroed words.  A program that does not settle, or whose symbols do not
+// fit the slots, has its lock set: the lock-step, launched after, does it.
+struct ChunkSizes {  // offsets in bytes into the program's arrays; [0, zeroed) start as zeros
+    uint64_t last, need, tag, delta, dirty, moved, lock, zeroed, off, slots, rec, out, state, row, win, pair, touch, total;
+    uint64_t runs, tiles;
+};
+ChunkSizes chunk_sizes(uint32_t F, uint32_t S, uint32_t W, uint32_t items);
+void chunk_bind(LaneChunks& ch, const ChunkSizes& z, void* zeroed, void* rest);
+struct ChunkBatch {
+    const Prog* progs;
+    const uint32_t* order;
+    const uint32_t* run_off;   // [n + 1]
+    const uint32_t* tile_off;  // [n + 1]
+    uint32_t n, runs, tiles;
+    uint32_t classes;          // chunk_class of the programs, or'ed
+    uint32_t rounds;           // at most
+    uint32_t* sync;
+};
+// Steps from which on chunks pay.  Their passes and rounds have a cost of their own, about
+// 0.12 ms: with 403 steps (one function) the allocation took 0.36 ms in lock-step and 0.46
+// in chunks, with 1,449 (two functions) 1.46 and 0.82.
+constexpr uint32_t kChunkMinSteps = 768;
+// Lane-0 functions up to which one warp, and four, fold a chunk's rows (else a block).
+constexpr uint32_t kChunkNarrow = 16, kChunkWide = 128;
+inline uint32_t chunk_class(uint32_t G0) { return G0 <= 1u ? 1u : (G0 <= kChunkNarrow ? 2u : (G0 <= kChunkWide ? 4u : 8u)); }
+// Batches: the lock-step runs programs side by side, so it lasts as long as its longest
+// program, where chunks last as long as all their runs.  Measured cycles: a lock-step's
+// step 1,000 with one lane-0 function, 1,450 with up to 32, 2,350 with more; a round, of a
+// sixth of the chunks and some, 20,000 and for each wave of 2,432 runs (16 warps on 152 SMs)
+// 15,000, with more than kChunkNarrow functions (which run again more often, and have folds)
+// four times as much.  64 programs of up to 4,575 steps took 3.0 to 4.3 ms in lock-step and
+// 2.0 to 2.6 in chunks, 512 of up to 4,058 steps and 64 functions 8.4 and 18.5.
+inline uint64_t lock_step_cycles(uint64_t S, uint32_t G0) { return S * (G0 <= 1u ? 1000u : (G0 <= 32u ? 1450u : 2350u)); }
+inline uint64_t chunk_work(uint64_t tiles, uint32_t G0) { return tiles * ((G0 + 31u) / 32u) * (G0 <= kChunkNarrow ? 1u : 4u); }
+inline bool chunk_pays(uint64_t tiles, uint64_t work, uint64_t before, uint64_t after) {
+    return (tiles / 6u + 6u) * (20000u + 15000u * work / 2432u) + after < before;
+}
+// Rounds before the lock-step takes over: they have been a third of the chunks or less.
+inline uint32_t chunk_rounds(uint32_t tiles) { return tiles + 64u; }
+inline uint32_t chunk_sync_words(uint32_t rounds) { return rounds + 4u; }
+cudaError_t run_lane_chunks(const ChunkBatch& b, const Prog& one, cudaStream_t s);
 // The record form of one program, and of the programs order[0..n) of a batch: program
 // order[k] has its independent functions (32 a block) in blocks free_off[k].. and its
 // trigger rows (kRowTile steps a block) in blocks row_off[k]..
@@ -91,7 +141,7 @@ cudaError_t run_regalloc_steps(const Prog& P, RaForm form, cudaStream_t s);
 constexpr uint32_t kStepClusterMin = 256, kStepBlockMax = 1024;
 bool step_cluster_fits(uint32_t G0);
 bool ra_cluster_disabled();
-cudaError_t run_step_regalloc(const Prog& P, cudaStream_t s);
+cudaError_t run_step_regalloc(const Prog& P, const ChunkBatch* chunks, cudaStream_t s);
 struct StepBatch {
     const Prog* progs;
     const uint32_t* order;
@@ -99,6 +149,7 @@ struct StepBatch {
     const uint32_t* row_off;   // [n + 1]
     uint32_t n, free_blocks, row_blocks, max_g0;
     uint32_t per_block;        // batch_step_scalar: functions per block (scalar_per_warp)
+    const ChunkBatch* chunks;  // the programs in chunks (each with blocks for its slots behind its independent functions'), or null
 };
 cudaError_t batch_step_regalloc(const StepBatch& b, cudaStream_t s);
 uint32_t scalar_per_warp(uint64_t functions);

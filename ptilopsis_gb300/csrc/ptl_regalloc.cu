@@ -5,8 +5,8 @@
 
 #include <algorithm>
 
+#include "ptl_chunks.cuh"
 #include "ptl_kernels.cuh"
-#include "ptl_steps.cuh"
 
 namespace ptl {
 namespace {
@@ -58,8 +58,14 @@ __global__ void __launch_bounds__(32) k_step_free(Src src) {
     __shared__ uint8_t ring[kFreeRing * kFreeStride];
     uint32_t local;
     src.take(blockIdx.x, &local, P);
+    const uint32_t G0 = (P.F + 7u) / 8u, free_blocks = (P.F - G0 + 31u) / 32u;
+    if (local >= free_blocks) {  // the lane-0 functions' slots (with chunks only)
+        const uint32_t j = (local - free_blocks) * 32u + threadIdx.x;
+        if (j < G0) step_slot_function(P, j, ring + threadIdx.x, kFreeStride, kFreeRing);
+        return;
+    }
     const uint32_t x = local * 32u + threadIdx.x;
-    if (x >= P.F - (P.F + 7u) / 8u) return;
+    if (x >= P.F - G0) return;
     const uint32_t f = P.ra_order ? P.ra_order[x] : (x / 7u) * 8u + (x % 7u) + 1u;
     step_free_function(P, f, ring + threadIdx.x, kFreeStride, kFreeRing);
 }
@@ -122,6 +128,38 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_step_rows(Src src) {
     for (uint32_t k = threadIdx.x; k < kRowTile * kRowPos; k += 32u * kRowWarps)
         row[k] = lo[k / kRowPos][k % kRowPos] | (hi[k / kRowPos][k % kRowPos] << 16);
     if (threadIdx.x < kRowTile) P.tany[tile * kRowTile + threadIdx.x] = any[threadIdx.x];
+}
+
+// ---- what the lane-0 functions' slots need (ptl_chunks.cuh): each symbol's last reader,
+// with blocks as above, and by a program's first block the functions' items.
+template <class Src>
+__global__ void __launch_bounds__(32 * kRowWarps) k_chunk_prep(Src src) {
+    __shared__ Prog P;
+    __shared__ uint32_t part[32 * kRowWarps];
+    uint32_t tile;
+    src.take(blockIdx.x, &tile, P);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, G0 = (P.F + 7u) / 8u;
+    for (uint32_t j = warp; j < G0; j += kRowWarps)
+        if (s32(P.fn_size0[8u * j]) > s32(tile * kChunk + lane)) chunk_last_read(P, P.fn_start0[8u * j] + tile * kChunk + lane);
+    if (tile != 0) return;
+    constexpr uint32_t T = 32u * kRowWarps;
+    const uint32_t per = (G0 + T - 1u) / T, lo = min(G0, threadIdx.x * per), hi = min(G0, lo + per);
+    uint32_t sum = 0;
+    for (uint32_t j = lo; j < hi; ++j) sum += chunks_of(P, j);
+    part[threadIdx.x] = sum;
+    __syncthreads();
+    for (uint32_t d = 1; d < T; d <<= 1) {
+        const uint32_t y = threadIdx.x >= d ? part[threadIdx.x - d] : 0u;
+        __syncthreads();
+        part[threadIdx.x] += y;
+        __syncthreads();
+    }
+    uint32_t at = part[threadIdx.x] - sum;
+    for (uint32_t j = lo; j < hi; ++j) {
+        P.ch.off[j] = at;
+        at += chunks_of(P, j);
+    }
+    if (hi == G0 && lo < hi) P.ch.off[G0] = at;
 }
 
 // ---- lane-0 functions in lock-step: a thread per slot (slot = group), a block per
@@ -491,6 +529,9 @@ __device__ void lane_pass(const Prog& P, unsigned char* smem, uint32_t T, uint32
     lane_tail(sh, L, tail);
 }
 
+// Whether the lane-0 functions are still to be done.
+__device__ bool lock_step(const Prog& P) { return !P.ch.lock || *P.ch.lock != 0; }
+
 // The block has the threads of the widest listed program; a narrower one's extra warps
 // leave at once.
 template <class Src, int MAXT>
@@ -499,7 +540,7 @@ __global__ void __launch_bounds__(MAXT) k_step_lane0(Src src, uint32_t K) {
     __shared__ Prog P;
     uint32_t local;
     src.take(blockIdx.x, &local, P);
-    if (P.S == 0) return;
+    if (P.S == 0 || !lock_step(P)) return;
     const uint32_t G0 = (P.F + 7u) / 8u;
     const uint32_t T = min(blockDim.x, (G0 + 31u) & ~31u);
     if (threadIdx.x >= T) return;
@@ -513,6 +554,7 @@ __global__ void __launch_bounds__(MAXT) k_step_lane0_cluster(OneProgram src, uin
     __shared__ Prog P;
     uint32_t local;
     src.take(0, &local, P);
+    if (!lock_step(P)) return;  // every CTA alike
     const uint32_t G0 = (P.F + 7u) / 8u, C = gridDim.x;
     const uint32_t rank = cluster_rank();
     const uint32_t j0 = rank * per_cta, j1 = min(G0, j0 + per_cta);
@@ -585,17 +627,27 @@ bool step_cluster_fits(uint32_t G0) {
     return G0 <= kClusterMax * 1024u && launch_lane0_cluster(Prog{}, G0, nullptr, true, &placed) == cudaSuccess && placed;
 }
 
-cudaError_t run_step_regalloc(const Prog& P, cudaStream_t s) {
+cudaError_t run_step_regalloc(const Prog& P, const ChunkBatch* chunks, cudaStream_t s) {
     const OneProgram src{P};
     const uint32_t G0 = (P.F + 7u) / 8u, free_fns = P.F - G0;
-    if (free_fns) {
-        note_launch();
-        k_step_free<<<(free_fns + 31u) / 32u, 32, 0, s>>>(src);
-    }
     const uint32_t tiles = static_cast<uint32_t>(row_tiles(P.S));
+    if (chunks) {
+        note_launch();
+        k_chunk_prep<<<tiles, 32u * kRowWarps, 0, s>>>(src);
+    }
+    const uint32_t blocks = (free_fns + 31u) / 32u + (chunks ? (G0 + 31u) / 32u : 0u);
+    if (blocks) {
+        note_launch();
+        k_step_free<<<blocks, 32, 0, s>>>(src);
+    }
     if (tiles == 0) return cudaGetLastError();
     note_launch();
     k_step_rows<<<tiles, 32u * kRowWarps, 0, s>>>(src);
+    if (chunks) {
+        const cudaError_t e = run_lane_chunks(*chunks, P, s);
+        if (e != cudaSuccess) return e;
+    }
+    // the lock-step, where that has not done it (lock_step)
     if (G0 > kStepClusterMin) {
         bool placed = false;
         const cudaError_t e = launch_lane0_cluster(P, G0, s, false, &placed);
@@ -628,6 +680,10 @@ cudaError_t batch_step_scalar(const StepBatch& b, cudaStream_t s) {
 
 cudaError_t batch_step_regalloc(const StepBatch& b, cudaStream_t s) {
     if (b.n == 0) return cudaSuccess;
+    if (b.chunks) {
+        note_launch();
+        k_chunk_prep<<<b.chunks->tiles, 32u * kRowWarps, 0, s>>>(ManyPrograms{b.progs, b.chunks->tile_off, b.chunks->order, b.chunks->n});
+    }
     if (b.free_blocks) {
         note_launch();
         k_step_free<<<b.free_blocks, 32, 0, s>>>(ManyPrograms{b.progs, b.free_off, b.order, b.n});
@@ -635,6 +691,10 @@ cudaError_t batch_step_regalloc(const StepBatch& b, cudaStream_t s) {
     if (b.row_blocks) {
         note_launch();
         k_step_rows<<<b.row_blocks, 32u * kRowWarps, 0, s>>>(ManyPrograms{b.progs, b.row_off, b.order, b.n});
+    }
+    if (b.chunks) {
+        const cudaError_t e = run_lane_chunks(*b.chunks, Prog{}, s);
+        if (e != cudaSuccess) return e;
     }
     return launch_lane0(ManyPrograms{b.progs, nullptr, b.order, b.n}, b.n, b.max_g0, 128u, s);
 }

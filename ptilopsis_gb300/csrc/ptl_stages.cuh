@@ -120,6 +120,29 @@ struct Tab {
     PTL_HD Slots4 gword(uint32_t type, uint32_t rt) const { return slots4(t->gword, type, rt); }
 };
 
+// Arrays of the lane-0 functions' chunks (ptl_chunks.cuh).
+struct alignas(8) ChunkPair {
+    uint32_t any, wr;
+};
+struct LaneChunks {
+    uint32_t* last;    // per word: the last word that reads its symbol (0: none)
+    uint32_t* off;     // per lane-0 function and at the end: its first item (a chunk of a function)
+    uint32_t* slots;   // per lane-0 function: slots its symbols take
+    unsigned long long* rec;  // [items][kChunk] slot records
+    uint32_t* need;    // per item: the round its start state has changed for
+    void* out;         // [items][kChunk] positions written and triggered
+    void* state;       // [items + 1] state at the chunk's start
+    uint32_t* row;     // [S in whole tiles][kRowPos] P.trow with the lane-0 functions' triggers
+    uint16_t* win;     // [S in whole tiles][kRowPos] greatest lane-0 group + 1 that writes the position
+    ChunkPair* pair;   // [S in whole tiles] positions triggered / written by lane-0 functions at all
+    uint32_t* touch;   // [tiles] positions triggered or written in the tile at all
+    uint32_t* tag;     // [tiles][warps of functions] the round some function's start state has changed for
+    uint32_t* delta;   // [S in whole tiles][2] positions whose writes / triggers have changed since the last fold
+    uint32_t* dirty;   // [tiles] the round some function's output has changed in
+    uint32_t* moved;   // [tiles] the round the rows have changed for
+    uint32_t* lock;    // nonzero: the lock-step has to do it
+};
+
 // ------------------------------------------------------------------ program view
 struct Prog {
     // sizes
@@ -175,6 +198,7 @@ struct Prog {
     uint32_t* tmask;      // per word: positions its step triggers (independent functions)
     uint32_t* trow;       // [S in whole tiles][kRowPos] trigger rows
     uint32_t* tany;       // [S in whole tiles] positions triggered at all
+    LaneChunks ch;
     uint32_t* stamp;      // definitions per virtual register (regalloc cross check)
     uint8_t* defpos;      // row-0 position + 1 of each lane-0 definition; null: use the row-0 hash
     unsigned long long* lifetime;
@@ -197,7 +221,7 @@ struct Prog {
     // tables, errors, scratch flags
     Tab tab;
     ErrorWord* err;
-    uint32_t* flags;      // [0] optimize changed, [1] [2] regalloc checks, [3] a node at max_depth
+    uint32_t* flags;      // [0] optimize changed, then lane-0 chunks; [1] [2] regalloc checks; [3] a node at max_depth
     uint32_t scalar;      // 1: the scalar generator's semantics (ptl_scalar.cuh)
     uint32_t pad_;
     // the scalar generator's register allocation in a batch (null otherwise): per

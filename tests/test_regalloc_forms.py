@@ -100,3 +100,70 @@ def test_gpu_scalar_records(built_cuda, n_functions):
     with BatchCompiler(tiles=None, scalar=True) as b:
         b.compile([_program(5), tree, _program(2)])
         np.testing.assert_array_equal(b.words(1), want)
+
+
+def _long_chain(tree, n):
+    """tree with one literal operand of an addition replaced by n nested additions
+    1 + (1 + (1 + ...)): n symbols that are alive at once."""
+    import dataclasses
+    ADD, LIT, INT = 13, 35, 2
+    t, rt, par = (np.asarray(getattr(tree, k)) for k in ("type", "rtype", "parent"))
+    leaf = [k for k in range(tree.n) if t[k] == LIT and rt[k] == INT and t[par[k]] == ADD][-1]
+    more = 2 * n  # the leaf becomes 1, 1, .., 1 (n + 1 of them), then n additions
+    at = lambda k: k if k < leaf else k + more  # the leaf's place is the outermost addition's
+    cols = {k: np.asarray(getattr(tree, k)) for k in ("type", "rtype", "parent", "depth", "child_idx", "data")}
+    new = {k: np.insert(c, leaf, np.zeros(more, c.dtype)) for k, c in cols.items()}
+    new["parent"] = np.array([at(p) if p >= 0 else p for p in new["parent"]], cols["parent"].dtype)
+    d = int(cols["depth"][leaf])
+    for k in range(n + 1):  # literal k is the left operand of addition k, the last one a right one
+        i = leaf + k
+        new["type"][i], new["rtype"][i], new["data"][i] = LIT, INT, 1
+        new["parent"][i] = leaf + more - min(k, n - 1)
+        new["depth"][i], new["child_idx"][i] = d + min(k, n - 1) + 1, 1 if k == n else 0
+    for k in range(n):  # addition k, the outermost last
+        i = leaf + more - k
+        new["type"][i], new["rtype"][i], new["data"][i] = ADD, INT, 0
+        new["depth"][i] = d + k
+        if k:
+            new["parent"][i], new["child_idx"][i] = i + 1, 1
+    return dataclasses.replace(tree, max_depth=int(new["depth"].max()), **new)
+
+
+@pytest.mark.parametrize("chain", [0, 50, 70])
+@pytest.mark.parametrize("n_functions", [1, 9, 130, 700])
+def test_hostmodel_chunks(built, n_functions, chain):
+    """The lane-0 functions in chunks; 50 nested operands fit the slots, 70 do not (the
+    lock-step then does the program)."""
+    from test_hostmodel import assert_stages_equal, hostmodel
+    L = hostmodel()
+    tree = _program(n_functions, 300.0, max_expr_depth=12, float_frac=0.3)
+    locked = False
+    if chain:
+        tree = _program(1, 900.0, float_frac=0.0) if n_functions == 1 else tree
+        tree = _long_chain(tree, chain)
+    assert_stages_equal(tree_to_ast(tree))
+    locked = bool(L.ptlhm_last_locked())
+    if chain <= 50:
+        assert not locked
+    elif n_functions == 1:
+        assert locked
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("chain", [0, 70])
+@pytest.mark.parametrize("n_functions", [1, 9, 128, 129, 1024, 1025])
+def test_gpu_chunks(built_cuda, n_functions, chain):
+    """Programs long enough for chunks: a lone lane-0 function, and row folds by one warp (2
+    and 16 of them), four warps (17 and 128) and a block (129)."""
+    from oracle import portbind
+    from ptilopsis_gb300 import RvGenerator
+    tree = _program(n_functions, 3000.0 if n_functions < 100 else 500.0, float_frac=0.3)
+    if chain:
+        tree = _long_chain(tree, chain)
+    ref = portbind.compile_ast(tree_to_ast(tree))
+    with RvGenerator(tree) as gen:
+        gen.process()
+        assert gen.function_table()["sizes"].max() > 768
+        np.testing.assert_array_equal(gen.get_instructions(), ref.words)
+        gen.process()  # again, in the same arrays
+        np.testing.assert_array_equal(gen.get_instructions(), ref.words)
