@@ -1042,7 +1042,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
                 hf[k] = nf;
                 hr[k] = nr;
                 nf += static_cast<uint32_t>((nfree[step_list[k]] + 31) / 32);
-                if (in_chunks[step_list[k]]) nf += static_cast<uint32_t>((F[step_list[k]] - nfree[step_list[k]] + 31) / 32);
+                if (in_chunks[step_list[k]]) nf += static_cast<uint32_t>(chunk[step_list[k]].runs);
                 nr += static_cast<uint32_t>(row_tiles(S[step_list[k]]));
             }
             for (size_t k = step_list.size(); k <= B; ++k) {

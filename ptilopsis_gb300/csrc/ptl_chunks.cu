@@ -312,6 +312,8 @@ ChunkSizes chunk_sizes(uint32_t F, uint32_t S, uint32_t W, uint32_t items) {
         return here;
     };
     z.last = take(4ull * W);
+    z.reach = take(4ull * (items + 1ull));
+    z.slots = take(4ull * G0);
     z.need = take(4ull * (items + 1ull));
     z.tag = take(4ull * (z.runs + (G0 + 31u) / 32u));
     z.delta = take(8ull * tiles * kRowTile);
@@ -320,7 +322,6 @@ ChunkSizes chunk_sizes(uint32_t F, uint32_t S, uint32_t W, uint32_t items) {
     z.lock = take(4ull);
     z.zeroed = at;
     z.off = take(4ull * (G0 + 1u));
-    z.slots = take(4ull * G0);
     z.rec = take(static_cast<uint64_t>(items) * kChunk * 8u);
     z.out = take(static_cast<uint64_t>(items) * kChunk * 8u);
     z.state = take((items + 1ull) * kStateVecs * 16u);
@@ -335,6 +336,8 @@ void chunk_bind(LaneChunks& ch, const ChunkSizes& z, void* zeroed, void* rest) {
     char* a = static_cast<char*>(zeroed);
     char* b = static_cast<char*>(rest) - z.zeroed;
     ch.last = reinterpret_cast<uint32_t*>(a + z.last);
+    ch.reach = reinterpret_cast<uint32_t*>(a + z.reach);
+    ch.slots = reinterpret_cast<uint32_t*>(a + z.slots);
     ch.need = reinterpret_cast<uint32_t*>(a + z.need);
     ch.tag = reinterpret_cast<uint32_t*>(a + z.tag);
     ch.delta = reinterpret_cast<uint32_t*>(a + z.delta);
@@ -342,7 +345,6 @@ void chunk_bind(LaneChunks& ch, const ChunkSizes& z, void* zeroed, void* rest) {
     ch.moved = reinterpret_cast<uint32_t*>(a + z.moved);
     ch.lock = reinterpret_cast<uint32_t*>(a + z.lock);
     ch.off = reinterpret_cast<uint32_t*>(b + z.off);
-    ch.slots = reinterpret_cast<uint32_t*>(b + z.slots);
     ch.rec = reinterpret_cast<unsigned long long*>(b + z.rec);
     ch.out = b + z.out;
     ch.state = b + z.state;

@@ -24,8 +24,8 @@
 // a run, and for wide programs the folds (ptl_chunks.cu).  Chunks of 64 steps took fewer
 // rounds but more steps in all (26 x 64 against 32 x 32 for 64 functions), chunks of 16
 // more rounds (41), each with its fold and waits.  Before and after, the whole allocation:
-// 1.46 to 0.82 ms (two lane-0 functions of 1,449 steps), 4.18 to 2.07 (64 of 2,830), 11.7
-// to 4.8 (256 of 8,151), 12.7 to 10.8 (1,229 of 4,072).
+// 1.46 to 0.73 ms (two lane-0 functions of 1,449 steps), 4.18 to 2.05 (64 of 2,830), 11.7
+// to 3.8 (256 of 8,151), 12.7 to 10.2 (1,229 of 4,072).
 #pragma once
 
 #include "ptl_steps.cuh"
@@ -36,7 +36,7 @@ constexpr uint32_t kChunk = kRowTile;  // steps; a row tile per chunk
 constexpr uint32_t kLiveGuess = 0xFFFFFFFEu;
 
 // Symbols live in slots: a symbol takes the lowest free one at its definition and gives it
-// back at its last read (step_slot_function), so a state is a few slots however far apart
+// back at its last read (step_slot_chunk), so a state is a few slots however far apart
 // definition and read are.  Slot 0 always reads as "no symbol".  A program with more than
 // kSlots - 1 symbols alive at once runs in lock-step.
 //
@@ -95,78 +95,80 @@ PTL_HD uint32_t chunks_of(const Prog& P, uint32_t j) {
     return size > 0 ? (static_cast<uint32_t>(size) + kChunk - 1u) / kChunk : 0u;
 }
 
-// The last word that reads each symbol (last, zero before).
-PTL_HD void chunk_last_read(const Prog& P, uint32_t i) {
-    const uint64_t r = P.rec[i];
+PTL_HD void chunk_max(uint32_t* p, uint32_t v) {
+#if defined(__CUDA_ARCH__)
+    atomicMax(p, v);
+#else
+    if (*p < v) *p = v;
+#endif
+}
+// Step i of lane-0 function 8j: the last word that reads each symbol, and for each chunk how
+// far the symbols from before it reach (last, reach: zero before).
+constexpr uint32_t kChunkReach = 256u;  // chunks a symbol may live through (else the lock-step)
+PTL_HD void chunk_last_read(const Prog& P, uint32_t j, uint32_t i) {
+    const uint32_t start = P.fn_start0[8u * j];
+    const uint64_t r = P.rec[start + i];
     const uint32_t d[2] = {step_d1(r), step_d2(r)};
     for (int k = 0; k < 2; ++k) {
         if (!d[k]) continue;
-#if defined(__CUDA_ARCH__)
-        atomicMax(&P.ch.last[i - d[k]], i);
-#else
-        if (P.ch.last[i - d[k]] < i) P.ch.last[i - d[k]] = i;
-#endif
+        chunk_max(&P.ch.last[start + i - d[k]], start + i);
+        const uint32_t to = i / kChunk;
+        uint32_t c = (i - d[k]) / kChunk + 1u;
+        if (to >= c + kChunkReach) {
+            *P.ch.lock = 1u;
+            continue;
+        }
+        for (; c <= to; ++c) chunk_max(&P.ch.reach[P.ch.off[j] + c], start + i);
     }
 }
 
-// Lane-0 function 8j's slot records; a thread each, as the independent functions have
-// (ring: the last words' slots).  Sets *lock if the slots do not suffice.
-PTL_HD void step_slot_function(const Prog& P, uint32_t j, uint8_t* ring, uint32_t stride, uint32_t K) {
-    const uint32_t start = P.fn_start0[8u * j];
-    const int32_t size = s32(P.fn_size0[8u * j]);
-    P.ch.slots[j] = 1;
-    if (size <= 0) return;
+// Slot records.  Between two steps where no symbol is alive (statements mostly) the slots
+// are a matter of their own, so a thread takes the stretches that begin in chunk c of
+// function 8j, from its first such point to the first one behind it (ring: the last words'
+// slots).  One thread per function instead took 528 cycles a step, and as long as the
+// independent functions and more (9,275 steps: the allocation 4.7 ms, now 3.8).  Sets *lock if the
+// slots do not suffice.
+PTL_HD void step_slot_chunk(const Prog& P, uint32_t j, uint32_t c, uint8_t* ring, uint32_t stride, uint32_t K) {
+    const uint32_t start = P.fn_start0[8u * j], n = P.fn_size0[8u * j], base = c * kChunk, mask = K - 1u;
     const unsigned long long* rec = P.rec + start;
     const uint32_t* last = P.ch.last + start;
     unsigned long long* out = P.ch.rec + static_cast<size_t>(P.ch.off[j]) * kChunk;
-    const uint32_t n = static_cast<uint32_t>(size), mask = K - 1u;
+    uint32_t i = base;
+    if (c) {
+        uint32_t alive = P.ch.reach[P.ch.off[j] + c];  // to the last read of any symbol so far
+        for (; i < n && i < base + kChunk && alive >= start + i; ++i) alive = alive > last[i] ? alive : last[i];
+        if (i >= n || i >= base + kChunk) return;
+    }
     uint64_t open = ~1ull;
     uint32_t most = 0;
     bool full = false;
-    unsigned long long next[kStepAhead];
-#pragma unroll
-    for (uint32_t k = 0; k < kStepAhead; ++k) next[k] = k < n ? rec[k] : kStepIdle;
-    for (uint32_t b = 0; b < n; b += kStepAhead) {
-        unsigned long long now[kStepAhead];
-        uint32_t end1[kStepAhead], end2[kStepAhead], read[kStepAhead];
-#pragma unroll
-        for (uint32_t k = 0; k < kStepAhead; ++k) {
-            const uint32_t i = b + k;
-            now[k] = next[k];
-            next[k] = i + kStepAhead < n ? rec[i + kStepAhead] : kStepIdle;
-            end1[k] = i < n ? last[i - step_d1(now[k])] : 0u;
-            end2[k] = i < n ? last[i - step_d2(now[k])] : 0u;
-            read[k] = i < n ? last[i] : 0u;
+    for (; i < n && (i < base + kChunk || open != ~1ull); ++i) {
+        const uint64_t now = rec[i];
+        const uint32_t d1 = step_d1(now), d2 = step_d2(now);
+        uint32_t s1 = ring[((i - d1) & mask) * stride], s2 = ring[((i - d2) & mask) * stride];
+        if (d1 >= K) s1 = slot_of(static_cast<uint32_t>(out[i - d1] >> 32) & 0xFFFFu);
+        if (d2 >= K) s2 = slot_of(static_cast<uint32_t>(out[i - d2] >> 32) & 0xFFFFu);
+        s1 = d1 ? s1 : 0u;
+        s2 = d2 ? s2 : 0u;
+        const bool last1 = !d1 || last[i - d1] == start + i, last2 = !d2 || last[i - d2] == start + i;
+        if (last1) open |= (1ull << s1) & ~1ull;
+        if (last2) open |= (1ull << s2) & ~1ull;
+        uint32_t own = 0;
+        if (last[i]) {
+            const uint32_t low = static_cast<uint32_t>(open), high = static_cast<uint32_t>(open >> 32);
+            if (open) own = low ? low_bit(low) : 32u + low_bit(high);
+            else full = true;
+            open &= ~((1ull << own) & ~1ull);
+            most = own > most ? own : most;
         }
-#pragma unroll
-        for (uint32_t k = 0; k < kStepAhead; ++k) {
-            const uint32_t i = b + k;
-            if (i >= n) break;
-            const uint32_t d1 = step_d1(now[k]), d2 = step_d2(now[k]);
-            uint32_t s1 = ring[((i - d1) & mask) * stride], s2 = ring[((i - d2) & mask) * stride];
-            if (d1 >= K) s1 = slot_of(static_cast<uint32_t>(out[i - d1] >> 32) & 0xFFFFu);
-            if (d2 >= K) s2 = slot_of(static_cast<uint32_t>(out[i - d2] >> 32) & 0xFFFFu);
-            s1 = d1 ? s1 : 0u;
-            s2 = d2 ? s2 : 0u;
-            const bool last1 = !d1 || end1[k] == start + i, last2 = !d2 || end2[k] == start + i;
-            if (last1) open |= (1ull << s1) & ~1ull;
-            if (last2) open |= (1ull << s2) & ~1ull;
-            uint32_t own = 0;
-            if (read[k]) {
-                const uint32_t low = static_cast<uint32_t>(open), high = static_cast<uint32_t>(open >> 32);
-                if (open) own = low ? low_bit(low) : 32u + low_bit(high);
-                else full = true;
-                open &= ~(1ull << own);
-                most = own > most ? own : most;
-            }
-            ring[(i & mask) * stride] = static_cast<uint8_t>(own);
-            // (the fields of rd's code, 6 bits, and the flags are bits 48-56 of both records)
-            out[i] = static_cast<uint64_t>(slot_at(s1)) | static_cast<uint64_t>(slot_at(s2)) << 16 |
-                     static_cast<uint64_t>(slot_at(own)) << 32 | ((now[k] >> 48 & 0x1FFull) << 48) |
-                     static_cast<uint64_t>((last1 ? kStepLast1 : 0u) | (last2 ? kStepLast2 : 0u)) << 32;
-        }
+        ring[(i & mask) * stride] = static_cast<uint8_t>(own);
+        // (rd's code, 6 bits, and the flags are bits 48-56 of both records)
+        out[i] = static_cast<uint64_t>(slot_at(s1)) | static_cast<uint64_t>(slot_at(s2)) << 16 |
+                 static_cast<uint64_t>(slot_at(own)) << 32 | ((now >> 48 & 0x1FFull) << 48) |
+                 static_cast<uint64_t>((last1 ? kStepLast1 : 0u) | (last2 ? kStepLast2 : 0u)) << 32;
+        if (full) break;
     }
-    P.ch.slots[j] = most + 1u;
+    chunk_max(&P.ch.slots[j], most + 1u);
     if (full) *P.ch.lock = 1u;
 }
 

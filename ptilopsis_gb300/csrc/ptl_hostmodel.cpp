@@ -226,7 +226,7 @@ struct Model {
         std::vector<uint32_t> off(G0 + 1);
         for (uint32_t j = 0; j < G0; ++j) off[j + 1] = off[j] + chunks_of(P, j);
         const size_t items = off[G0];
-        std::vector<uint32_t> last(P.W, 0), slots(G0), need(items + 1, 0), delta(2 * steps, 0), dirty(tiles, 0), moved(tiles, 0);
+        std::vector<uint32_t> last(P.W, 0), reach(items + 1, 0), slots(G0, 0), need(items + 1, 0), delta(2 * steps, 0), dirty(tiles, 0), moved(tiles, 0);
         std::vector<unsigned long long> rec(items * kChunk);
         std::vector<ChunkVec> out(items * kChunk / 2), state((items + 1) * kStateVecs);
         std::vector<uint32_t> row(steps * kRowPos), mem(kChunkMemWords);
@@ -234,12 +234,13 @@ struct Model {
         std::vector<ChunkPair> pair(steps);
         std::vector<uint32_t> touch(tiles, 0);
         uint32_t lock = 0;
-        P.ch = LaneChunks{last.data(), off.data(), slots.data(), rec.data(), need.data(), out.data(), state.data(), row.data(),
+        P.ch = LaneChunks{last.data(), reach.data(), off.data(), slots.data(), rec.data(), need.data(), out.data(), state.data(), row.data(),
                           win.data(), pair.data(), touch.data(), nullptr, delta.data(), dirty.data(), moved.data(), &lock};
         std::vector<uint8_t> ring(K);
         for (uint32_t j = 0; j < G0; ++j)
-            for (uint32_t i = 0; i < size(j); ++i) chunk_last_read(P, P.fn_start0[8 * j] + i);
-        for (uint32_t j = 0; j < G0; ++j) step_slot_function(P, j, ring.data(), 1, K);
+            for (uint32_t i = 0; i < size(j); ++i) chunk_last_read(P, j, i);
+        for (uint32_t j = 0; j < G0; ++j)
+            for (uint32_t c = 0; c < chunks_of(P, j); ++c) step_slot_chunk(P, j, c, ring.data(), 1, K);
         g_last_locked = lock != 0;
         if (lock) return false;
         const std::vector<uint16_t> no_win(kChunk * kRowPos, 0);

@@ -94,7 +94,7 @@ cudaError_t run_regalloc_steps(const Prog& P, RaForm form, const ChunkBatch* chu
 // chunk_sync_words zeroed words.  A program that does not settle, or whose symbols do not
 // fit the slots, has its lock set: the lock-step, launched after, does it.
 struct ChunkSizes {  // offsets in bytes into the program's arrays; [0, zeroed) start as zeros
-    uint64_t last, need, tag, delta, dirty, moved, lock, zeroed, off, slots, rec, out, state, row, win, pair, touch, total;
+    uint64_t last, reach, slots, need, tag, delta, dirty, moved, lock, zeroed, off, rec, out, state, row, win, pair, touch, total;
     uint64_t runs, tiles;
 };
 ChunkSizes chunk_sizes(uint32_t F, uint32_t S, uint32_t W, uint32_t items);
@@ -110,8 +110,8 @@ struct ChunkBatch {
     uint32_t* sync;
 };
 // Steps from which on chunks pay.  Their passes and rounds have a cost of their own, about
-// 0.12 ms: with 403 steps (one function) the allocation took 0.36 ms in lock-step and 0.46
-// in chunks, with 1,449 (two functions) 1.46 and 0.82.
+// 0.12 ms: with 403 steps (one function) the allocation took 0.36 ms in lock-step and 0.45
+// in chunks, with 1,449 (two functions) 1.46 and 0.73.
 constexpr uint32_t kChunkMinSteps = 768;
 // Lane-0 functions up to which one warp, and four, fold a chunk's rows (else a block).
 constexpr uint32_t kChunkNarrow = 16, kChunkWide = 128;
@@ -149,7 +149,7 @@ struct StepBatch {
     const uint32_t* row_off;   // [n + 1]
     uint32_t n, free_blocks, row_blocks, max_g0;
     uint32_t per_block;        // batch_step_scalar: functions per block (scalar_per_warp)
-    const ChunkBatch* chunks;  // the programs in chunks (each with blocks for its slots behind its independent functions'), or null
+    const ChunkBatch* chunks;  // the programs in chunks (each with a block per run tile for its slots behind its independent functions'), or null
 };
 cudaError_t batch_step_regalloc(const StepBatch& b, cudaStream_t s);
 uint32_t scalar_per_warp(uint64_t functions);

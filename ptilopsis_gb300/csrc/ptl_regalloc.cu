@@ -59,9 +59,11 @@ __global__ void __launch_bounds__(32) k_step_free(Src src) {
     uint32_t local;
     src.take(blockIdx.x, &local, P);
     const uint32_t G0 = (P.F + 7u) / 8u, free_blocks = (P.F - G0 + 31u) / 32u;
-    if (local >= free_blocks) {  // the lane-0 functions' slots (with chunks only)
-        const uint32_t j = (local - free_blocks) * 32u + threadIdx.x;
-        if (j < G0) step_slot_function(P, j, ring + threadIdx.x, kFreeStride, kFreeRing);
+    if (local >= free_blocks) {  // the lane-0 functions' slots: a block per run tile (with chunks only)
+        const uint32_t NW = (G0 + 31u) / 32u, tile = local - free_blocks;
+        const uint32_t c = tile / NW, j = tile % NW * 32u + threadIdx.x;
+        if (j < G0 && s32(P.fn_size0[8u * j]) > s32(c * kChunk))
+            step_slot_chunk(P, j, c, ring + threadIdx.x, kFreeStride, kFreeRing);
         return;
     }
     const uint32_t x = local * 32u + threadIdx.x;
@@ -130,20 +132,17 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_step_rows(Src src) {
     if (threadIdx.x < kRowTile) P.tany[tile * kRowTile + threadIdx.x] = any[threadIdx.x];
 }
 
-// ---- what the lane-0 functions' slots need (ptl_chunks.cuh): each symbol's last reader,
-// with blocks as above, and by a program's first block the functions' items.
+// ---- what the lane-0 functions' slots need (ptl_chunks.cuh): their items (a block per
+// program), then each symbol's last reader (blocks as above).
 template <class Src>
-__global__ void __launch_bounds__(32 * kRowWarps) k_chunk_prep(Src src) {
+__global__ void __launch_bounds__(32 * kRowWarps) k_chunk_items(Src src) {
     __shared__ Prog P;
     __shared__ uint32_t part[32 * kRowWarps];
-    uint32_t tile;
-    src.take(blockIdx.x, &tile, P);
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, G0 = (P.F + 7u) / 8u;
-    for (uint32_t j = warp; j < G0; j += kRowWarps)
-        if (s32(P.fn_size0[8u * j]) > s32(tile * kChunk + lane)) chunk_last_read(P, P.fn_start0[8u * j] + tile * kChunk + lane);
-    if (tile != 0) return;
+    uint32_t local;
+    src.take(blockIdx.x, &local, P);
     constexpr uint32_t T = 32u * kRowWarps;
-    const uint32_t per = (G0 + T - 1u) / T, lo = min(G0, threadIdx.x * per), hi = min(G0, lo + per);
+    const uint32_t G0 = (P.F + 7u) / 8u, per = (G0 + T - 1u) / T;
+    const uint32_t lo = min(G0, threadIdx.x * per), hi = min(G0, lo + per);
     uint32_t sum = 0;
     for (uint32_t j = lo; j < hi; ++j) sum += chunks_of(P, j);
     part[threadIdx.x] = sum;
@@ -160,6 +159,15 @@ __global__ void __launch_bounds__(32 * kRowWarps) k_chunk_prep(Src src) {
         at += chunks_of(P, j);
     }
     if (hi == G0 && lo < hi) P.ch.off[G0] = at;
+}
+template <class Src>
+__global__ void __launch_bounds__(32 * kRowWarps) k_chunk_last(Src src) {
+    __shared__ Prog P;
+    uint32_t tile;
+    src.take(blockIdx.x, &tile, P);
+    const uint32_t i = tile * kChunk + (threadIdx.x & 31u), G0 = (P.F + 7u) / 8u;
+    for (uint32_t j = threadIdx.x >> 5; j < G0; j += kRowWarps)
+        if (s32(P.fn_size0[8u * j]) > s32(i)) chunk_last_read(P, j, i);
 }
 
 // ---- lane-0 functions in lock-step: a thread per slot (slot = group), a block per
@@ -633,9 +641,11 @@ cudaError_t run_step_regalloc(const Prog& P, const ChunkBatch* chunks, cudaStrea
     const uint32_t tiles = static_cast<uint32_t>(row_tiles(P.S));
     if (chunks) {
         note_launch();
-        k_chunk_prep<<<tiles, 32u * kRowWarps, 0, s>>>(src);
+        k_chunk_items<<<1, 32u * kRowWarps, 0, s>>>(src);
+        note_launch();
+        k_chunk_last<<<tiles, 32u * kRowWarps, 0, s>>>(src);
     }
-    const uint32_t blocks = (free_fns + 31u) / 32u + (chunks ? (G0 + 31u) / 32u : 0u);
+    const uint32_t blocks = (free_fns + 31u) / 32u + (chunks ? chunks->runs : 0u);
     if (blocks) {
         note_launch();
         k_step_free<<<blocks, 32, 0, s>>>(src);
@@ -682,7 +692,10 @@ cudaError_t batch_step_regalloc(const StepBatch& b, cudaStream_t s) {
     if (b.n == 0) return cudaSuccess;
     if (b.chunks) {
         note_launch();
-        k_chunk_prep<<<b.chunks->tiles, 32u * kRowWarps, 0, s>>>(ManyPrograms{b.progs, b.chunks->tile_off, b.chunks->order, b.chunks->n});
+        k_chunk_items<<<b.chunks->n, 32u * kRowWarps, 0, s>>>(ManyPrograms{b.progs, nullptr, b.chunks->order, b.chunks->n});
+        note_launch();
+        k_chunk_last<<<b.chunks->tiles, 32u * kRowWarps, 0, s>>>(
+            ManyPrograms{b.progs, b.chunks->tile_off, b.chunks->order, b.chunks->n});
     }
     if (b.free_blocks) {
         note_launch();

@@ -126,6 +126,7 @@ struct alignas(8) ChunkPair {
 };
 struct LaneChunks {
     uint32_t* last;    // per word: the last word that reads its symbol (0: none)
+    uint32_t* reach;   // per item: the last word from its chunk on that reads a symbol from before it (0: none)
     uint32_t* off;     // per lane-0 function and at the end: its first item (a chunk of a function)
     uint32_t* slots;   // per lane-0 function: slots its symbols take
     unsigned long long* rec;  // [items][kChunk] slot records
