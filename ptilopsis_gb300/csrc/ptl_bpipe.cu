@@ -136,7 +136,7 @@ public:
     DBuf in_type, in_rtype, in_parent, in_depth, in_child, in_data;
     DBuf nt, rt, nd1, nd, par, ci, dep, loc0, loc, pos, decl, fflag, regs;
     DBuf fn_id, fn_start, fn_size, fn_end, fn_start0, fn_size0, ra_order, lifetime;
-    DBuf instr, rd, rs1, rs2, jt, used_instrs, symreg, symswp, stamp, spill, roffs, owner, used, smark, defpos;
+    DBuf instr, rd, rs1, rs2, jt, used_instrs, symreg, symswp, stamp, spill, roffs, owner, used, smark;
     DBuf tmask, trow, tany, lane_zero, lane_rest;
     DBuf trig_min, trig_max, ra_chunks;
     DBuf ni, nrd, nr1, nr2, njt, joffs, out;
@@ -171,7 +171,7 @@ public:
         return {&tab, &in_type, &in_rtype, &in_parent, &in_depth, &in_child, &in_data, &nt, &rt, &nd1, &nd, &par,
                 &ci, &dep, &loc0, &loc, &pos, &decl, &fflag, &regs, &fn_id, &fn_start, &fn_size,
                 &fn_end, &fn_start0, &fn_size0, &ra_order, &lifetime, &instr, &rd, &rs1, &rs2, &jt, &used_instrs, &symreg,
-                &symswp, &stamp, &spill, &roffs, &owner, &used, &smark, &defpos, &tmask, &trow, &tany, &lane_zero, &lane_rest, &trig_min, &trig_max, &ra_chunks, &ni, &nrd,
+                &symswp, &stamp, &spill, &roffs, &owner, &used, &smark, &tmask, &trow, &tany, &lane_zero, &lane_rest, &trig_min, &trig_max, &ra_chunks, &ni, &nrd,
                 &nr1, &nr2, &njt, &joffs, &out, &errw, &flags, &meta, &progs, &tabs, &lists, &changed,
                 &sort_err, &a_off, &dirty, &ra_sync, &sa, &sapos, &sbpos, &seg0, &seg1, &tile_seg, &tile_l, &tile_r,
                 &sort_stops, &leaf, &heap, &counters, &scan_status, &scan_counter, &sort_local, &sort_equal,
@@ -704,7 +704,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
         BP_CU(family(Lw, {&instr, &rd, &rs1, &rs2, &jt, &symreg, &symswp, &stamp}, 4));
         BP_CU(family_written(Lw, {&used_instrs, &spill, &roffs}, 4));
         BP_CU(family(Lw, {&owner}, 8));
-        BP_CU(family(Lw, {&used, &smark, &defpos}, 1));
+        BP_CU(family(Lw, {&used, &smark}, 1));
         for (size_t p = 0; p < B; ++p) {
             Prog& P = hp[p];
             P.W = static_cast<uint32_t>(W[p]);
@@ -726,7 +726,6 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
             P.rec = P.owner;  // done with after isn_gen
             P.used = used.at<uint8_t>(e);
             P.smark = smark.at<uint8_t>(e);
-            P.defpos = defpos.at<uint8_t>(e);
         }
         upload_progs();
         {
@@ -925,7 +924,6 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
                 }
             } else {
                 general[p] = 1;
-                hp[p].defpos = nullptr;
                 if (g0 > kRaClusterMin && ra_cluster_fits(static_cast<uint32_t>(g0))) {
                     wide_list.push_back(static_cast<uint32_t>(p));  // its own launches, on a cluster
                 } else {
@@ -964,9 +962,11 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
         std::vector<ChunkSizes> chunk(B);
         std::vector<uint8_t> in_chunks(B, 0);
         ChunkBatch chunks{};
+        chunks.share = ra_share;
         uint64_t zero_bytes = 0, rest_bytes = 0, sync_words = 0;
         auto groups = [&](uint32_t p) { return static_cast<uint32_t>((F[p] + 7) / 8); };
-        auto long_enough = [&](uint32_t p) { return S[p] >= kChunkMinSteps && hfl[4 * p] != 0; };
+        const bool can = chunks_fit();
+        auto long_enough = [&](uint32_t p) { return can && S[p] >= kChunkMinSteps && hfl[4 * p] != 0; };
         auto put_in_chunks = [&](uint32_t p) {
             in_chunks[p] = 1;
             chunk[p] = chunk_sizes(static_cast<uint32_t>(F[p]), static_cast<uint32_t>(S[p]), static_cast<uint32_t>(W[p]), hfl[4 * p]);
@@ -1103,6 +1103,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
             Prog one = hp[p];
             one.ra_order = nullptr;
             ChunkBatch c{};
+            c.share = ra_share;
             if (in_chunks[p]) {
                 c.n = 1;
                 c.runs = static_cast<uint32_t>(chunk[p].runs);

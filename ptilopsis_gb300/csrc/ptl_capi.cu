@@ -98,7 +98,7 @@ struct ptl_generator {
     DevBuf fn_ra_start, fn_ra_end, fn_ra_size;
     DevBuf instr, rd, rs1, rs2, jt, owner, used, smark, used_instrs;
     DevBuf tmask, trow, tany, lane_zero, lane_rest, opt_work;
-    DevBuf symreg, symswp, stamp, defpos, lifetime, trig_min, trig_max, ra_chunks, spill, roffs;
+    DevBuf symreg, symswp, stamp, lifetime, trig_min, trig_max, ra_chunks, spill, roffs;
     DevBuf ni, nrd, nr1, nr2, njt, fsz, joffs, out;
     DevBuf sort_a, sort_apos, sort_bpos, sort_seg0, sort_seg1, sort_tile_seg, sort_tile_l, sort_tile_r, sort_stops,
         sort_leaf, sort_heap, sort_counters, sort_local, sort_equal;
@@ -142,7 +142,7 @@ struct ptl_generator {
                 &par, &ci, &dep, &fflag, &sizes, &loc0, &loc, &pos, &regs, &decl, &fn_id, &fn_start,
                 &fn_size, &fn_end, &fn_start0, &fn_size0, &fn_end0, &fn_ra_start, &fn_ra_end, &fn_ra_size,
                 &instr, &rd, &rs1, &rs2, &jt, &owner, &used, &smark, &used_instrs, &tmask, &trow, &tany, &lane_zero, &lane_rest, &opt_work, &symreg, &symswp,
-                &stamp, &defpos, &lifetime, &trig_min, &trig_max, &ra_chunks, &spill, &roffs, &ni, &nrd, &nr1, &nr2, &njt,
+                &stamp, &lifetime, &trig_min, &trig_max, &ra_chunks, &spill, &roffs, &ni, &nrd, &nr1, &nr2, &njt,
                 &fsz, &joffs, &out, &sort_a, &sort_apos, &sort_bpos, &sort_seg0, &sort_seg1, &sort_stops,
                 &sort_tile_seg, &sort_tile_l, &sort_tile_r, &sort_leaf, &sort_heap, &sort_counters, &sort_local, &sort_equal,
                 &scan_status, &meta, &flags, &errw, &tables, &preserve, &sregs, &ssteps,
@@ -330,7 +330,6 @@ Prog make_prog(ptl_generator* g) {
     P.symreg = g->symreg.at<uint32_t>();
     P.symswp = g->symswp.at<uint32_t>();
     P.stamp = g->stamp.at<uint32_t>();
-    P.defpos = g->defpos.at<uint8_t>();
     P.lifetime = g->lifetime.at<unsigned long long>();
     P.trig_min = g->trig_min.at<uint32_t>();
     P.trig_max = g->trig_max.at<uint32_t>();
@@ -612,10 +611,9 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
             b->zero(z);
         PTL_CU(launch_zero(z, s));
     }
-    PTL_CU(g->defpos.ensure(wb8, 1));
     P = make_prog(g);
     if (!prog_ready(P, {P.instr, P.rd, P.rs1, P.rs2, P.jt, P.used_instrs, P.symreg, P.symswp, P.stamp, P.spill,
-                        P.defpos, P.roffs, P.owner, P.used, P.smark, P.pos, P.regs}))
+                        P.roffs, P.owner, P.used, P.smark, P.pos, P.regs}))
         return fail(g, PTL_CUDA_ERROR, "internal: unallocated word arrays");
     PTL_CU(run_depth_sort(P, ss, s, &g->sort_rounds, &g->sort_graph));
     if (g->scalar) launch_gen_scalar(P, s);
@@ -664,7 +662,7 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
         PTL_CU(ra_form(P, s, row0_hash, &form, &items));
         ChunkSizes chunk{};
         ChunkBatch chunks{};
-        const bool in_chunks = form == RaForm::Steps && items != 0 && g->S >= kChunkMinSteps;
+        const bool in_chunks = form == RaForm::Steps && items != 0 && g->S >= kChunkMinSteps && chunks_fit();
         if (in_chunks) {
             chunk = chunk_sizes(g->F, g->S, g->W, items);
             const uint32_t rounds = chunk_rounds(static_cast<uint32_t>(chunk.tiles));
@@ -696,7 +694,6 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
         if (form == RaForm::Steps ? !prog_ready(P, {P.tmask, P.trow, P.tany})
                                   : form == RaForm::General && !prog_ready(P, {P.trig_min, P.trig_max, P.ra_chunks}))
             return fail(g, PTL_CUDA_ERROR, "internal: unallocated regalloc state");
-        P.defpos = nullptr;
         if (in_chunks) chunk_bind(P.ch, chunk, g->lane_zero.at<char>(), g->lane_rest.at<char>());
         PTL_CU(run_regalloc_steps(P, form, in_chunks ? &chunks : nullptr, s));
         g->ra_serial = form == RaForm::Serial;

@@ -354,6 +354,15 @@ void chunk_bind(LaneChunks& ch, const ChunkSizes& z, void* zeroed, void* rest) {
     ch.touch = reinterpret_cast<uint32_t*>(b + z.touch);
 }
 
+bool chunks_fit() {
+    int dev = 0, coop = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
+        return false;
+    constexpr size_t bytes = kWarps * kWarpBytes;
+    if (allow_dynamic_smem(reinterpret_cast<const void*>(&k_lane_chunks), bytes) != cudaSuccess) return false;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lane_chunks, kThreads, bytes) == cudaSuccess && per_sm >= 1;
+}
+
 cudaError_t run_lane_chunks(const ChunkBatch& b, const Prog& one, cudaStream_t s) {
     if (b.n == 0 || b.runs == 0) return cudaSuccess;
     constexpr size_t bytes = kWarps * kWarpBytes;
@@ -364,7 +373,8 @@ cudaError_t run_lane_chunks(const ChunkBatch& b, const Prog& one, cudaStream_t s
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // small programs leave most SMs out: four warps fill an SM's schedulers
-    const uint32_t grid = std::max(1u, std::min<uint32_t>(sms, (b.runs + 3u) / 4u));
+    const uint32_t most = b.share > 0.0 && b.share < 1.0 ? static_cast<uint32_t>(sms * b.share) : static_cast<uint32_t>(sms);
+    const uint32_t grid = std::max(1u, std::min(most, (b.runs + 3u) / 4u));
     note_launch();
     ChunkBatch arg = b;
     Prog p = one;

@@ -52,7 +52,7 @@ struct Model {
     CodeTables tab;
     ErrorWord err{};
     uint32_t flags[4] = {0, 0, 0, 0};
-    HBuf<uint8_t> in_type, in_rtype, fflag, used, smark, defpos, nt, rt;
+    HBuf<uint8_t> in_type, in_rtype, fflag, used, smark, nt, rt;
     HBuf<int32_t> in_parent, in_depth, in_child, par, ci, dep;
     HBuf<uint32_t> in_data, nd1, nd, sizes, loc0, loc, regs, pos, decl, fn_id, fn_start, fn_size,
         fn_end, fn_start0, fn_size0, fn_end0, fn_ra_start, fn_ra_end, fn_ra_size, instr, rd, rs1, rs2, jt,
@@ -71,7 +71,6 @@ struct Model {
         P.fn_end = fn_end.p; P.fn_start0 = fn_start0.p; P.fn_size0 = fn_size0.p; P.instr = instr.p;
         P.rd = rd.p; P.rs1 = rs1.p; P.rs2 = rs2.p; P.jt = jt.p; P.used = used.p; P.smark = smark.p;
         P.used_instrs = used_instrs.p; P.symreg = symreg.p; P.symswp = symswp.p; P.stamp = stamp.p;
-        P.defpos = defpos.p;
         P.lifetime = lifetime.p; P.trig_min = trig_min.p; P.trig_max = trig_max.p; P.spill = spill.p;
         P.roffs = roffs.p; P.ni = ni.p; P.nrd = nrd.p; P.nr1 = nr1.p; P.nr2 = nr2.p; P.njt = njt.p;
         P.fsz = fsz.p; P.joffs = joffs.p; P.out = out.p;
@@ -161,10 +160,8 @@ struct Model {
     uint32_t hm_cache_k = g_cache_k;
 
     // The lane-0 pass with the same phase functions as k_ra_lane0_cached.
-    void lane0_cached(uint32_t S, uint32_t K, bool hashed) {
+    void lane0_cached(uint32_t S, uint32_t K) {
         const uint32_t G0 = (P.F + 7) / 8;
-        const Prog Psave = P;
-        if (hashed) P.defpos = nullptr;
         Ra2Shared sh{};
         std::vector<uint32_t> cur(4 * G0), tag(static_cast<size_t>(G0) * K);
         std::vector<uint32_t> val(static_cast<size_t>(G0) * K);
@@ -176,7 +173,7 @@ struct Model {
             ra2_slot_init(P, c, L[j], j, j);
         }
         for (int p = 0; p < 64; ++p) { sh.R0[p] = 0xFFFFFFFFu; sh.R0own[p] = 0xFFFFFFFFu; }
-        if (S > 0) for (uint32_t p = 0; p < 64; ++p) ra2_begin_p(sh, 0, p, P.trig_min[p], P.trig_max[p], hashed);
+        if (S > 0) for (uint32_t p = 0; p < 64; ++p) ra2_begin_p(sh, 0, p, P.trig_min[p], P.trig_max[p]);
         uint32_t s0 = 0;  // steps with a lane-0 function still running
         for (uint32_t j = 0; j < G0; ++j) s0 = std::max(s0, ra2_lane0_size(L[j]));
         s0 = std::min(s0, S);
@@ -200,21 +197,20 @@ struct Model {
                 }
                 for (uint32_t j = 0; j < G0; ++j) ra2_apply(P, c, sh, L[j], j, i, cur.data() + 4 * j);
             }
-            if (hashed) for (uint32_t p = 0; p < 64; ++p) snap_clear_next(sh, i, p);
+            for (uint32_t p = 0; p < 64; ++p) snap_clear_next(sh, i, p);
             for (uint32_t p = 0; p < 64; ++p) {
                 ra2_end_p(P, c, sh, p, cur.data());
             }
             if (i + 1 < S) {
                 for (uint32_t p = 0; p < 64; ++p) {
                     ra2_begin_p(sh, i + 1, p, P.trig_min[static_cast<size_t>(i + 1) * 64 + p],
-                                P.trig_max[static_cast<size_t>(i + 1) * 64 + p], hashed);
+                                P.trig_max[static_cast<size_t>(i + 1) * 64 + p]);
                 }
             }
         }
         {  // the steps after the last lane-0 function only mark row 0's symbols
             for (uint32_t p = 0; p < 64; ++p) ra2_tail_p(P, c, sh, p, s0, S);
         }
-        P = Psave;
     }
 
     // The lane-0 functions in chunks (ptl_chunks.cuh), round by round as its kernel runs
@@ -507,8 +503,6 @@ struct Model {
         trig_min.ensure(static_cast<size_t>(std::max<uint32_t>(S, 1)) * 64, 0xFFFFFFFFu);
         trig_max.ensure(static_cast<size_t>(std::max<uint32_t>(S, 1)) * 64, 0u);
         bind();
-        defpos.ensure(wb8);
-        bind();
         if (scalar) {
             scalar_regalloc(F, W, wb8);
             if (!check()) return err.code;
@@ -523,10 +517,8 @@ struct Model {
             } else if (flagbits & 2u) {
                 std::vector<uint32_t> tag(64), val(64);
                 const SymCache c1{tag.data(), val.data(), 64};
-                Prog Pfree = P;
-                Pfree.defpos = nullptr;
-                for (uint32_t f = 0; f < F; ++f) if (f & 7u) ra_free_function_cached(Pfree, c1, 0, f);
-                lane0_cached(S, hm_cache_k, true);
+                for (uint32_t f = 0; f < F; ++f) if (f & 7u) ra_free_function_cached(P, c1, 0, f);
+                lane0_cached(S, hm_cache_k);
             } else {
                 tmask.ensure(wb8);
                 bind();

@@ -108,6 +108,7 @@ struct ChunkBatch {
     uint32_t classes;          // chunk_class of the programs, or'ed
     uint32_t rounds;           // at most
     uint32_t* sync;
+    double share;              // part of the SMs the launch may take (0: all)
 };
 // Steps from which on chunks pay.  Their passes and rounds have a cost of their own, about
 // 0.12 ms: with 403 steps (one function) the allocation took 0.36 ms in lock-step and 0.45
@@ -132,6 +133,7 @@ inline bool chunk_pays(uint64_t tiles, uint64_t work, uint64_t before, uint64_t 
 inline uint32_t chunk_rounds(uint32_t tiles) { return tiles + 64u; }
 inline uint32_t chunk_sync_words(uint32_t rounds) { return rounds + 4u; }
 cudaError_t run_lane_chunks(const ChunkBatch& b, const Prog& one, cudaStream_t s);
+bool chunks_fit();  // whether the current device can run its blocks together (else the lock-step)
 // The record form of one program, and of the programs order[0..n) of a batch: program
 // order[k] has its independent functions (32 a block) in blocks free_off[k].. and its
 // trigger rows (kRowTile steps a block) in blocks row_off[k]..
@@ -160,7 +162,7 @@ cudaError_t batch_step_scalar(const StepBatch& b, cudaStream_t s);
 // Lane-0 passes too wide for one block: programs with more than kRaClusterMin lane-0
 // groups (at most 8,192) run theirs on a thread-block cluster when the device can place
 // it.  ra_cluster_fits tells whether it can; launch_ra_wide launches the program's
-// independent functions (Pfree: no definition positions), then the cluster pass (P0),
+// independent functions (Pfree), then the cluster pass (P0),
 // and sets *launched, or launches nothing.
 constexpr uint32_t kRaClusterMin = 1024;
 bool ra_cluster_fits(uint32_t G0);

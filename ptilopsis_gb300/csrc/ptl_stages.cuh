@@ -201,7 +201,6 @@ struct Prog {
     uint32_t* tany;       // [S in whole tiles] positions triggered at all
     LaneChunks ch;
     uint32_t* stamp;      // definitions per virtual register (regalloc cross check)
-    uint8_t* defpos;      // row-0 position + 1 of each lane-0 definition; null: use the row-0 hash
     unsigned long long* lifetime;
     uint32_t* trig_min;   // [S][64] min group+1 of non-lane-0 triggers, 0xFFFFFFFF = none
     uint32_t* trig_max;   // [S][64] max group+1, 0 = none
@@ -843,20 +842,6 @@ PTL_HD uint32_t function_of(const Prog& P, uint32_t i, uint32_t hint = 0xFFFFFFF
         if (P.fn_start0[mid] <= i) lo = mid; else hi = mid;
     }
     return lo;
-}
-
-PTL_HD uint32_t st_ra_cross(const Prog& P, uint32_t i, uint32_t* defcnt, uint32_t* hint = nullptr) {
-    const uint32_t lo = function_of(P, i, hint ? *hint : 0xFFFFFFFFu);
-    if (hint) *hint = lo;
-    const uint32_t rd = P.rd[i];
-    if (!ra_own(P, lo, P.rs1[i]) || !ra_own(P, lo, P.rs2[i]) || !ra_own(P, lo, rd)) return 1u;
-    if ((lo & 7u) != 0 || !(s32(rd) > 63)) return 0u;
-#if defined(__CUDA_ARCH__)
-    const uint32_t before = atomicAdd(&defcnt[rd - 64u], 1u);
-#else
-    const uint32_t before = defcnt[rd - 64u]++;
-#endif
-    return before != 0 ? 2u : 0u;
 }
 
 // The reference's step loop as written (rv_generator_avx.cpp:1400-1413 with one worker):
