@@ -112,7 +112,7 @@ struct ChunkBatch {
 };
 // Steps from which on chunks pay.  Their passes and rounds have a cost of their own, about
 // 0.12 ms: with 403 steps (one function) the allocation took 0.36 ms in lock-step and 0.45
-// in chunks, with 1,449 (two functions) 1.46 and 0.73.
+// in chunks, with 1,449 (two functions) 1.46 and 0.65.
 constexpr uint32_t kChunkMinSteps = 768;
 // Lane-0 functions up to which one warp, and four, fold a chunk's rows (else a block).
 constexpr uint32_t kChunkNarrow = 16, kChunkWide = 128;
