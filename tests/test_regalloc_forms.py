@@ -167,3 +167,20 @@ def test_gpu_chunks(built_cuda, n_functions, chain):
         np.testing.assert_array_equal(gen.get_instructions(), ref.words)
         gen.process()  # again, in the same arrays
         np.testing.assert_array_equal(gen.get_instructions(), ref.words)
+
+
+@pytest.mark.gpu
+def test_gpu_batch_chunks(built_cuda):
+    """A batch with programs in chunks beside short ones in lock-step, one with more symbols
+    alive than there are slots, and one too wide for a block (its own launches)."""
+    from oracle import portbind
+    from ptilopsis_gb300.batch import BatchCompiler
+    trees = [_program(n, m, float_frac=0.3) for n, m in ((1, 6000.0), (9, 4000.0), (140, 900.0), (3, 40.0), (20, 60.0))]
+    trees.append(_long_chain(_program(1, 6000.0, seed=0x50544D90, float_frac=0.0), 70))
+    trees.append(_program(8200, 60.0, sigma=1.5, max_fn_nodes=4000))
+    with BatchCompiler(tiles=None) as b:
+        for _ in range(2):
+            b.compile(trees)
+            for k, tree in enumerate(trees):
+                np.testing.assert_array_equal(b.words(k), portbind.compile_ast(tree_to_ast(tree)).words, err_msg=str(k))
+        assert max(int(b.function_table(6)["sizes"].max()), 0) > 768
