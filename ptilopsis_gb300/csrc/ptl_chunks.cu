@@ -45,6 +45,7 @@ struct GridBarrier {
 constexpr uint32_t kRowsAt = 0, kWinsAt = kChunk * kRowPos * 4u, kPairsAt = kWinsAt + kChunk * kRowPos * 2u,
                    kMemAt = kPairsAt + kChunk * 8u, kRunBytes = kMemAt + kChunkMemWords * 4u;
 constexpr uint32_t kFoldStride = kRowPos + 1u, kFoldBytes = 3u * kChunk * kFoldStride * 4u + kChunk * 8u;
+constexpr uint32_t kListMost = 512u, kListBytes = kListMost * 6u;  // a folding warp's functions (8,192 groups, a block)
 constexpr uint32_t kWarpBytes = ((kRunBytes > kFoldBytes ? kRunBytes : kFoldBytes) + 15u) & ~15u;
 
 // The rows of chunk c again from its functions' outputs, at the positions where some
@@ -89,19 +90,43 @@ __device__ bool fold(const Prog& P, uint32_t c, uint32_t* smem, uint32_t warp, b
     // costs an operation per slice, where a loop over its positions diverges (and took up
     // to 450,000 cycles).
     uint32_t lo_s[kBits + kHigh] = {}, hi_s[kBits + kHigh] = {}, win_s[kBits + kHigh] = {}, trigs = 0, wrote_s = 0;
-    for (uint32_t j0 = warp, nb = 0; j0 < G0; j0 += kBatch * kTeam, ++nb) {
+    // This warp's functions that reach the chunk, in order: how many they are, and where the
+    // k-th one's outputs are.  Few reach a wide program's last chunks (1,229 functions: the
+    // allocation 10.2 to 9.1 ms).
+    uint32_t count = (G0 - min(G0, warp) + kTeam - 1u) / kTeam;
+    uint32_t* items = nullptr;
+    uint16_t* numbers = nullptr;
+    if constexpr (kTeam > 1) {
+        items = smem + (kWarpBytes + warp * kListBytes) / 4u;
+        numbers = reinterpret_cast<uint16_t*>(items + kListMost);
+        uint32_t all = count, n = 0;
+        for (uint32_t x0 = 0; x0 < all; x0 += 32u) {
+            const uint32_t x = x0 + lane, j = min(warp + x * kTeam, G0 - 1u), item = off[j] + c;
+            const bool has = x < all && item < off[j + 1u];
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, has), at = n + __popc(mask & ((1u << lane) - 1u));
+            if (has) {
+                items[at] = item;
+                numbers[at] = static_cast<uint16_t>(x);
+            }
+            n += __popc(mask);
+        }
+        count = n;
+        __syncwarp();
+    }
+    for (uint32_t x0 = 0, nb = 0; x0 < count; x0 += kBatch, ++nb) {
         uint2 x[kBatch];
-        uint32_t item[kBatch], end[kBatch];
 #pragma unroll
         for (uint32_t k = 0; k < kBatch; ++k) {  // no branches, so that all loads are in flight
-            const uint32_t j = min(j0 + k * kTeam, G0 - 1u);
-            item[k] = off[j] + c;
-            end[k] = j0 + k * kTeam < G0 ? off[j + 1u] : 0u;
-        }
-#pragma unroll
-        for (uint32_t k = 0; k < kBatch; ++k) {
-            const bool has = item[k] < end[k];
-            x[k] = __ldcg(out + static_cast<size_t>(has ? item[k] : 0u) * kChunk + lane);
+            bool has = x0 + k < count;
+            uint32_t item;
+            if constexpr (kTeam > 1) {
+                item = items[has ? x0 + k : 0u];
+            } else {
+                const uint32_t j = min(warp + (x0 + k) * kTeam, G0 - 1u);
+                item = off[j] + c;
+                has = has && item < off[j + 1u];
+            }
+            x[k] = __ldcg(out + static_cast<size_t>(has ? item : 0u) * kChunk + lane);
             if (!has) x[k] = make_uint2(0, 0);
         }
         uint32_t lo_b[kBits] = {}, hi_b[kBits] = {}, win_b[kBits] = {}, t = 0, w = 0;  // of the batch
@@ -136,6 +161,11 @@ __device__ bool fold(const Prog& P, uint32_t c, uint32_t* smem, uint32_t warp, b
             l |= (lo_s[i] >> p & 1u) << i;
             h |= (hi_s[i] >> p & 1u) << i;
             v |= (win_s[i] >> p & 1u) << i;
+        }
+        if constexpr (kTeam > 1) {
+            l = numbers[l];
+            h = numbers[h];
+            v = numbers[v];
         }
         const uint32_t group = warp + 1u;
         if (trigs >> p & 1u) {
@@ -199,6 +229,7 @@ __device__ bool fold(const Prog& P, uint32_t c, uint32_t* smem, uint32_t warp, b
 __global__ void __launch_bounds__(kThreads, 1)
     k_lane_chunks(const __grid_constant__ ChunkBatch b, const __grid_constant__ Prog one) {
     static_assert(kChunkNarrow <= 8u << 1 && kChunkWide <= 4u * 16u << 1 && 8192u <= kWarps * 16u << 5, "folds");
+    static_assert(kWarps * kListBytes <= (kWarps - 1u) * kWarpBytes && 4u * kListBytes <= 3u * kWarpBytes, "fold lists");
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     uint32_t* changed = b.sync + 2;  // [round]

@@ -25,7 +25,7 @@
 // rounds but more steps in all (26 x 64 against 32 x 32 for 64 functions), chunks of 16
 // more rounds (41), each with its fold and waits.  Before and after, the whole allocation:
 // 1.46 to 0.65 ms (two lane-0 functions of 1,449 steps), 4.18 to 1.80 (64 of 2,830), 11.7
-// to 3.5 (256 of 8,151), 12.7 to 10.2 (1,229 of 4,072).
+// to 3.5 (256 of 8,151), 12.7 to 9.1 (1,229 of 4,072).
 #pragma once
 
 #include "ptl_steps.cuh"
