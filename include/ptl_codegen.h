@@ -86,6 +86,12 @@ ptl_status ptl_generator_create_scalar(const ptl_ast_view* tree, int device, ptl
  * output). */
 ptl_status ptl_generator_process(ptl_generator* gen, int profile);
 
+/* Limits after which register allocation's chunks of steps give up, lower than the
+ * built-in ones: rounds (then its lock-step form allocates; same output), and clock cycles
+ * of one wait of a block for the others (then PTL_DEVICE_TIMEOUT).  0: the built-in limit.
+ * They hold for the following compiles; for tests of what comes after a limit. */
+ptl_status ptl_generator_set_chunk_limits(ptl_generator* gen, uint32_t rounds, uint64_t wait_cycles);
+
 /* Replaces get_instructions() (rv_generator_avx.cpp:82-84): the encoded RV words, in a
  * host buffer owned by the generator, valid until the next process or destroy. */
 ptl_status ptl_generator_instructions(ptl_generator* gen, const uint32_t** words, size_t* count);
@@ -217,6 +223,8 @@ ptl_status ptl_batch_tiles(const ptl_batch* batch, uint32_t tiles[2]);
  * launch may take (default 1).  Batches compiled at the same time on other handles of the
  * same device run beside it when it takes less. */
 ptl_status ptl_batch_set_regalloc_share(ptl_batch* batch, double share);
+/* ptl_generator_set_chunk_limits for the batch's following compiles. */
+ptl_status ptl_batch_set_chunk_limits(ptl_batch* batch, uint32_t rounds, uint64_t wait_cycles);
 /* scalar != 0: the following compiles give every program the scalar generator's output
  * (rv_generator_st, the reference's -s; ptl_generator_create_scalar one program at a
  * time); 0 (the default): the AVX generator's. */

@@ -43,6 +43,7 @@ def _bind(L):
     L.ptl_batch_tiles.argtypes = [vp, ctypes.POINTER(ctypes.c_uint32)]
     L.ptl_batch_set_regalloc_share.argtypes = [vp, ctypes.c_double]
     L.ptl_batch_set_scalar.argtypes = [vp, ctypes.c_int]
+    L.ptl_batch_set_chunk_limits.argtypes = [vp, ctypes.c_uint32, u64]
     L.ptl_batch_device_ns.argtypes = [vp]
     L.ptl_batch_device_ns.restype = u64
     L.ptl_batch_depth_sort_ns.argtypes = [vp]
@@ -67,7 +68,7 @@ def _bind(L):
     L.ptl_clock_ns.restype = u64
     for fn in ("ptl_batch_create", "ptl_batch_compile", "ptl_batch_status", "ptl_batch_words", "ptl_batch_stage_ns",
                "ptl_batch_copied_bytes", "ptl_batch_sizes", "ptl_batch_host_ns", "ptl_batch_set_tiles", "ptl_batch_tiles",
-               "ptl_batch_set_regalloc_share", "ptl_batch_set_scalar",
+               "ptl_batch_set_regalloc_share", "ptl_batch_set_scalar", "ptl_batch_set_chunk_limits",
                "ptl_batch_function_table", "ptl_server_create", "ptl_server_submit", "ptl_server_submit_flags", "ptl_server_poll",
                "ptl_server_result", "ptl_server_times", "ptl_server_release", "ptl_server_stats", "ptl_server_memory"):
         getattr(L, fn).restype = ctypes.c_int
@@ -190,6 +191,12 @@ class BatchCompiler:
         st = self._lib.ptl_batch_set_regalloc_share(self._h, float(share))
         if st != 0:
             raise PtlError(st, f"ptl_batch_set_regalloc_share({share})")
+
+    def set_chunk_limits(self, rounds: int = 0, wait_cycles: int = 0) -> None:
+        """RvGenerator.set_chunk_limits for the following compiles."""
+        st = self._lib.ptl_batch_set_chunk_limits(self._h, rounds, wait_cycles)
+        if st != 0:
+            raise PtlError(st, f"ptl_batch_set_chunk_limits({rounds}, {wait_cycles})")
 
     def tiles(self) -> tuple:
         v = (ctypes.c_uint32 * 2)()

@@ -134,6 +134,7 @@ def lib():
         L.ptl_generator_create.argtypes = [ctypes.POINTER(_AstView), ctypes.c_int, ctypes.POINTER(vp)]
         L.ptl_generator_create_scalar.argtypes = [ctypes.POINTER(_AstView), ctypes.c_int, ctypes.POINTER(vp)]
         L.ptl_generator_process.argtypes = [vp, ctypes.c_int]
+        L.ptl_generator_set_chunk_limits.argtypes = [vp, ctypes.c_uint32, ctypes.c_uint64]
         L.ptl_generator_upload.argtypes = [vp, ctypes.POINTER(_AstView)]
         L.ptl_kernel_launches.argtypes = []
         L.ptl_kernel_launches.restype = ctypes.c_uint64
@@ -155,7 +156,8 @@ def lib():
         L.ptl_code_table.restype = ctypes.c_size_t
         L.ptl_device_info.argtypes = [ctypes.c_int, ctypes.c_char_p, sz, ctypes.POINTER(ctypes.c_int),
                                       ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
-        for fn in ("ptl_generator_create", "ptl_generator_create_scalar", "ptl_generator_process", "ptl_generator_upload", "ptl_generator_instructions", "ptl_generator_copy_instructions",
+        for fn in ("ptl_generator_create", "ptl_generator_create_scalar", "ptl_generator_process",
+                   "ptl_generator_set_chunk_limits", "ptl_generator_upload", "ptl_generator_instructions", "ptl_generator_copy_instructions",
                    "ptl_generator_device_instructions", "ptl_generator_function_table",
                    "ptl_generator_stage_ns", "ptl_generator_snapshot", "ptl_compile", "ptl_device_info"):
             getattr(L, fn).restype = ctypes.c_int
@@ -253,6 +255,12 @@ class RvGenerator:
         the scalar generator's serial register allocation (both: same output)."""
         flags = (1 if profile else 0) | (0 if to_host else 2) | (4 if row0_hash else 0) | (8 if serial else 0)
         self._check(self._lib.ptl_generator_process(self._h, flags), "process")
+
+    def set_chunk_limits(self, rounds: int = 0, wait_cycles: int = 0) -> None:
+        """Lower limits (0: the built-in ones) after which register allocation's chunks give
+        up: rounds, after which its lock-step form allocates (same output), and cycles of one
+        wait, after which process raises a device timeout.  For tests."""
+        self._check(self._lib.ptl_generator_set_chunk_limits(self._h, rounds, wait_cycles), "set_chunk_limits")
 
     def get_instructions(self) -> np.ndarray:
         # A copy of the generator's host words.  (Fetching from the device straight into a

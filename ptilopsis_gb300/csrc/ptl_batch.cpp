@@ -157,6 +157,12 @@ extern "C" ptl_status ptl_batch_set_regalloc_share(ptl_batch* b, double share) {
     return PTL_OK;
 }
 
+extern "C" ptl_status ptl_batch_set_chunk_limits(ptl_batch* b, uint32_t rounds, uint64_t wait_cycles) {
+    if (!b || wait_cycles > (uint64_t(1) << 31)) return PTL_BAD_ARGUMENT;
+    b->pipe->set_chunk_limits(rounds, static_cast<long long>(wait_cycles));
+    return PTL_OK;
+}
+
 extern "C" ptl_status ptl_batch_set_scalar(ptl_batch* b, int scalar) {
     if (!b) return PTL_BAD_ARGUMENT;
     b->pipe->set_scalar(scalar != 0);

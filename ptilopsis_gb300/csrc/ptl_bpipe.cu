@@ -201,6 +201,7 @@ public:
         for (DBuf* b : all()) b->release();
         d_gp.release();
     }
+    void set_chunk_limits(uint32_t rounds, long long wait) override { chunk_limits = ChunkLimits{rounds, wait}; }
     void set_regalloc_share(double share) override { ra_share = std::min(1.0, std::max(0.05, share)); }
     void set_scalar(bool on) override { scalar_mode = on; }
     ptl_status scalar_regalloc(const std::vector<uint64_t>& F, const std::vector<uint64_t>& W,
@@ -267,6 +268,7 @@ public:
     }
     // tile sizes: element-wise stages, optimize sweeps (chosen by the autotuner or the defaults)
     uint32_t elem_tile = batch_tile(), sweep_tile = 1024;
+    ChunkLimits chunk_limits;
     double ra_share = 1.0;  // part of the resident blocks the persistent regalloc launch takes
     SortRoundGraph sort_graph;  // a pair of depth-sort rounds, replayed
     uint32_t slot_tile[32] = {};
@@ -1071,6 +1073,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
                 chunks.n = static_cast<uint32_t>(chunk_list.size());
                 chunks.sync = lane_zero.at<uint32_t>(sync_at);
                 sync_at += chunk_sync_words(chunks.rounds);
+                chunk_limits.apply(chunks);
             }
             const uint32_t* d_steps = upload_list(0, step_list);
             const uint32_t count = static_cast<uint32_t>(step_list.size());
@@ -1112,6 +1115,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
                 c.rounds = chunk_rounds(c.tiles);
                 c.sync = lane_zero.at<uint32_t>(sync_at);
                 sync_at += chunk_sync_words(c.rounds);
+                chunk_limits.apply(c);
             }
             BP_CU(run_step_regalloc(one, in_chunks[p] ? &c : nullptr, s));
         }

@@ -105,6 +105,7 @@ struct ptl_generator {
     DevBuf scan_status, meta, flags, errw, tables;
     DevBuf preserve, sregs, ssteps, sextra, sclaim;  // scalar register allocation
     bool scalar = false;  // the scalar generator's semantics (rv_generator_st)
+    ChunkLimits chunk_limits;
 
     // Pinned host memory for read-backs (a copy to pageable memory waits for the stream by
     // itself, so several of them are several waits): the error word and a few sizes, then
@@ -676,6 +677,7 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
             chunks.classes = chunk_class((g->F + 7u) / 8u);
             chunks.rounds = rounds;
             chunks.sync = reinterpret_cast<uint32_t*>(g->lane_zero.at<char>() + chunk.zeroed);
+            g->chunk_limits.apply(chunks);
         }
         if (form == RaForm::Steps) {
             const size_t steps = row_tiles(g->S) * kRowTile;
@@ -846,6 +848,12 @@ ptl_status ptl_generator_process(ptl_generator* g, int profile) {
         run_pipeline(g, (profile & 1) != 0, (profile & 2) == 0, (profile & 4) != 0, (profile & 8) != 0);
     if (st == PTL_OK) g->last_error.clear();
     return st;
+}
+
+ptl_status ptl_generator_set_chunk_limits(ptl_generator* g, uint32_t rounds, uint64_t wait_cycles) {
+    if (!g || wait_cycles > static_cast<uint64_t>(kChunkWait)) return PTL_BAD_ARGUMENT;
+    g->chunk_limits = ChunkLimits{rounds, static_cast<long long>(wait_cycles)};
+    return PTL_OK;
 }
 
 namespace {

@@ -14,9 +14,10 @@ namespace {
 constexpr uint32_t kWarps = 16, kThreads = 32 * kWarps;
 
 // Every block waits for all (the launch is cooperative: they are resident together).
-// False after a second without them.
+// False after `most` cycles without them.
 struct GridBarrier {
     uint32_t* count;
+    long long most;
     uint32_t goal = 0;
     __device__ bool wait() {
         __shared__ uint32_t lost;
@@ -26,13 +27,12 @@ struct GridBarrier {
             __threadfence();
             atomicAdd(count, 1u);
             const long long since = clock64();
-            bool late = false;
-            uint32_t seen;
-            do {
+            for (;;) {
+                uint32_t seen;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
-                late = clock64() - since > (1ll << 31);
-            } while (static_cast<int32_t>(seen - goal) < 0 && !late);
-            lost = late;
+                lost = static_cast<int32_t>(seen - goal) < 0;
+                if (!lost || clock64() - since > most) break;
+            }
             __threadfence();
         }
         __syncthreads();
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     uint32_t* changed = b.sync + 2;  // [round]
-    GridBarrier grid{b.sync};
+    GridBarrier grid{b.sync, b.wait};
     auto prog = [&](uint32_t k) -> const Prog& { return b.progs ? b.progs[b.order[k]] : one; };
     auto first_of = [&](const uint32_t* off, uint32_t k) { return b.progs ? off[k] : 0u; };
     auto owner = [&](const uint32_t* off, uint32_t q) {  // off[lo] <= q < off[lo + 1]
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         return lo;
     };
     auto late = [&](uint32_t round) {
-        if (threadIdx.x == 0) record_error(prog(0).err, ST_DEVICE_TIMEOUT, W_RA2, round);
+        chunks_lost(prog, b.n, threadIdx.x, kThreads, round);
     };
     // Rows of the chunks with new outputs (or of all), of programs with least < groups <=
     // most, by teams of kTeam warps.  A program with one lane-0 function needs none: what

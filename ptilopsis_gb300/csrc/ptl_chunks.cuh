@@ -363,4 +363,12 @@ PTL_HD uint32_t chunk_run(const Prog& P, const ChunkRows& rows, uint32_t* mem, u
     return result;
 }
 
+// What a launch whose blocks have lost one another leaves: none of its programs has its
+// lane-0 functions allocated, so the error is every program's (one without it would go on,
+// with registers that nothing allocated).  Done by thread `thread` of `threads`.
+template <class ProgramOf>
+PTL_HD void chunks_lost(const ProgramOf& program, uint32_t n, uint32_t thread, uint32_t threads, uint32_t round) {
+    for (uint32_t k = thread; k < n; k += threads) record_error(program(k).err, ST_DEVICE_TIMEOUT, W_RA2, round);
+}
+
 }  // namespace ptl

@@ -617,6 +617,14 @@ int ptlhm_gen_desc_ok(void) {
     return gen_desc_ok(&t) ? 1 : 0;
 }
 int ptlhm_last_locked(void) { return g_last_locked ? 1 : 0; }
+// The error codes of n programs after a lost chunk launch of `threads` threads a block.
+void ptlhm_chunks_lost(uint32_t n, uint32_t threads, uint32_t* codes) {
+    std::vector<ErrorWord> err(n);
+    std::vector<Prog> progs(n);
+    for (uint32_t k = 0; k < n; ++k) progs[k].err = &err[k];
+    for (uint32_t t = 0; t < threads; ++t) chunks_lost([&](uint32_t k) -> const Prog& { return progs[k]; }, n, t, threads, 3u);
+    for (uint32_t k = 0; k < n; ++k) codes[k] = err[k].code;
+}
 void ptlhm_set_chunks(int on) { g_chunks = on != 0; }
 void ptlhm_set_scalar_tiles(int on) { g_force_tiles = on != 0; }
 void ptlhm_set_scalar_serial(int on) { g_force_serial = on != 0; }

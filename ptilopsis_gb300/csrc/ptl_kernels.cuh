@@ -99,6 +99,7 @@ struct ChunkSizes {  // offsets in bytes into the program's arrays; [0, zeroed) 
 };
 ChunkSizes chunk_sizes(uint32_t F, uint32_t S, uint32_t W, uint32_t items);
 void chunk_bind(LaneChunks& ch, const ChunkSizes& z, void* zeroed, void* rest);
+constexpr long long kChunkWait = 1ll << 31;  // about a second
 struct ChunkBatch {
     const Prog* progs;
     const uint32_t* order;
@@ -109,6 +110,7 @@ struct ChunkBatch {
     uint32_t rounds;           // at most
     uint32_t* sync;
     double share;              // part of the SMs the launch may take (0: all)
+    long long wait = kChunkWait;  // cycles that a block waits for the others
 };
 // Steps from which on chunks pay.  Their passes and rounds have a cost of their own, about
 // 0.12 ms: with 403 steps (one function) the allocation took 0.36 ms in lock-step and 0.45
@@ -131,6 +133,15 @@ inline bool chunk_pays(uint64_t tiles, uint64_t work, uint64_t before, uint64_t 
 }
 // Rounds before the lock-step takes over: they have been a third of the chunks or less.
 inline uint32_t chunk_rounds(uint32_t tiles) { return tiles + 64u; }
+// Other limits of a generator or a batch (0: the above), so that tests see what comes after.
+struct ChunkLimits {
+    uint32_t rounds = 0;
+    long long wait = 0;
+    void apply(ChunkBatch& b) const {
+        if (rounds) b.rounds = rounds < b.rounds ? rounds : b.rounds;  // b.sync has words for no more
+        if (wait) b.wait = wait;
+    }
+};
 inline uint32_t chunk_sync_words(uint32_t rounds) { return rounds + 4u; }
 cudaError_t run_lane_chunks(const ChunkBatch& b, const Prog& one, cudaStream_t s);
 bool chunks_fit();  // whether the current device can run its blocks together (else the lock-step)

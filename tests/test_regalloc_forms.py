@@ -184,3 +184,41 @@ def test_gpu_batch_chunks(built_cuda):
             for k, tree in enumerate(trees):
                 np.testing.assert_array_equal(b.words(k), portbind.compile_ast(tree_to_ast(tree)).words, err_msg=str(k))
         assert max(int(b.function_table(6)["sizes"].max()), 0) > 768
+
+
+@pytest.mark.parametrize("programs, threads", [(1, 512), (3, 512), (512, 512), (1000, 512), (7, 1)])
+def test_hostmodel_lost_launch_fails_every_program(built, programs, threads):
+    """A chunk launch that gives up a wait holds many programs: each has the error (5), so
+    that none passes on words whose registers nothing allocated."""
+    from test_hostmodel import hostmodel
+    codes = np.zeros(programs, np.uint32)
+    hostmodel().ptlhm_chunks_lost(ctypes.c_uint32(programs), ctypes.c_uint32(threads), ctypes.c_void_p(codes.ctypes.data))
+    assert (codes == 5).all()
+
+
+@pytest.mark.gpu
+def test_gpu_chunk_wait_gives_up(built_cuda):
+    """A wait of one cycle runs out: a device timeout of every program in chunks, plain and
+    batched, and of no other; with the built-in wait the same objects compile again."""
+    from oracle import portbind
+    from ptilopsis_gb300 import PtlError, RvGenerator
+    from ptilopsis_gb300.batch import BatchCompiler
+    trees = [_program(n, m, float_frac=0.3) for n, m in ((9, 4000.0), (3, 40.0), (3, 6000.0), (140, 900.0))]
+    refs = [portbind.compile_ast(tree_to_ast(t)).words for t in trees]
+    with RvGenerator(trees[0]) as gen:
+        gen.set_chunk_limits(wait_cycles=1)
+        with pytest.raises(PtlError) as e:
+            gen.process()
+        assert e.value.status == 5
+        gen.set_chunk_limits()
+        gen.process()
+        np.testing.assert_array_equal(gen.get_instructions(), refs[0])
+    with BatchCompiler(tiles=None) as b:
+        b.set_chunk_limits(wait_cycles=1)
+        b.compile(trees, check=False)
+        assert [b.status(k) for k in range(4)] == [5, 0, 5, 5]
+        np.testing.assert_array_equal(b.words(1), refs[1])
+        b.set_chunk_limits()
+        b.compile(trees)
+        for k, want in enumerate(refs):
+            np.testing.assert_array_equal(b.words(k), want, err_msg=str(k))
