@@ -22,9 +22,6 @@
 namespace ptl {
 namespace {
 
-constexpr size_t kFrontPad = 16;  // elements before index 0 (the reference reads [-1])
-constexpr size_t kBackPad = 80;   // elements after the last 8-lane block
-
 // A device buffer with the reference's padding around it.  Allocated and freed in the
 // order of its generator's stream (cudaMallocAsync / cudaFreeAsync): growing or freeing
 // it does not wait for the whole device, so generators on other threads keep running.
@@ -39,7 +36,7 @@ struct DevBuf {
     T* at() const { return base ? reinterpret_cast<T*>(static_cast<char*>(base) + kFrontPad * elem) : nullptr; }
 
     cudaError_t ensure(size_t n, size_t esize) {
-        const size_t need = (n + kFrontPad + kBackPad) * esize;
+        const size_t need = buffer_bytes(n, esize);
         if (base && bytes >= need && elem == esize) {
             count = n;
             return cudaSuccess;
@@ -47,7 +44,7 @@ struct DevBuf {
         if (base) cudaFreeAsync(base, s);
         base = nullptr;
         bytes = 0;
-        const size_t grow = need + need / 4;  // room to grow without reallocating
+        const size_t grow = allocated_bytes(need);
         cudaError_t e = cudaMallocAsync(&base, grow, s);
         if (e != cudaSuccess) { base = nullptr; return e; }
         bytes = grow;
@@ -55,9 +52,9 @@ struct DevBuf {
         count = n;
         return cudaSuccess;
     }
-    cudaError_t zero(cudaStream_t s) const { return base ? cudaMemsetAsync(base, 0, (count + kFrontPad + kBackPad) * elem, s) : cudaSuccess; }
-    void zero(ZeroList& z) const { if (base) z.add(base, (count + kFrontPad + kBackPad) * elem); }
-    cudaError_t fill(cudaStream_t s, int byte) const { return base ? cudaMemsetAsync(base, byte, (count + kFrontPad + kBackPad) * elem, s) : cudaSuccess; }
+    cudaError_t zero(cudaStream_t s) const { return base ? cudaMemsetAsync(base, 0, buffer_bytes(count, elem), s) : cudaSuccess; }
+    void zero(ZeroList& z) const { if (base) z.add(base, buffer_bytes(count, elem)); }
+    cudaError_t fill(cudaStream_t s, int byte) const { return base ? cudaMemsetAsync(base, byte, buffer_bytes(count, elem), s) : cudaSuccess; }
     void release() { if (base) cudaFreeAsync(base, s); base = nullptr; bytes = 0; }
     // elements the allocation holds (at least the last ensure's n)
     size_t capacity() const { return base ? bytes / elem - kFrontPad - kBackPad : 0; }

@@ -86,6 +86,16 @@ bool gen_desc_ok(const CodeTables* t);
 PTL_HD int32_t s32(uint32_t v) { return static_cast<int32_t>(v); }
 PTL_HD uint32_t u32(int32_t v) { return static_cast<uint32_t>(v); }
 
+// ---------------------------------------------------------------- device buffers
+constexpr size_t kFrontPad = 16;  // elements before index 0 (the reference reads [-1])
+constexpr size_t kBackPad = 80;   // elements after the last 8-lane block
+// Bytes of a buffer of n elements with its pads, what clearing it writes (whole 16-byte
+// words), and what is allocated for it: room to grow without reallocating, in whole words,
+// so that whatever size fits the allocation can be cleared inside it.
+constexpr size_t buffer_bytes(size_t n, size_t elem) { return (n + kFrontPad + kBackPad) * elem; }
+constexpr size_t cleared_bytes(size_t bytes) { return (bytes + 15u) & ~size_t(15); }
+constexpr size_t allocated_bytes(size_t bytes) { return cleared_bytes(bytes + bytes / 4); }
+
 // ---------------------------------------------------------------- status
 enum Status : int {
     ST_OK = 0,

@@ -617,6 +617,13 @@ int ptlhm_gen_desc_ok(void) {
     return gen_desc_ok(&t) ? 1 : 0;
 }
 int ptlhm_last_locked(void) { return g_last_locked ? 1 : 0; }
+// Of a buffer of n elements: the bytes it needs, those that clearing it writes, and those
+// allocated for it.
+void ptlhm_buffer_bytes(size_t n, size_t elem, size_t out[3]) {
+    out[0] = buffer_bytes(n, elem);
+    out[1] = cleared_bytes(out[0]);
+    out[2] = allocated_bytes(out[0]);
+}
 // The error codes of n programs after a lost chunk launch of `threads` threads a block.
 void ptlhm_chunks_lost(uint32_t n, uint32_t threads, uint32_t* codes) {
     std::vector<ErrorWord> err(n);

@@ -1841,6 +1841,7 @@ void note_launch() { g_launches++; }
 
 // ====================================================================== launchers
 cudaError_t launch_zero(const ZeroList& z, cudaStream_t s) {
+    if (z.count > kZeroMost) return cudaErrorInvalidValue;
     uint64_t most = 0;
     for (int b = 0; b < z.count; ++b) most = std::max(most, z.n16[b]);
     if (most == 0) return cudaSuccess;

@@ -52,15 +52,19 @@ cudaError_t launch_cooperative(const void* kernel, uint32_t blocks, uint32_t thr
 
 // Up to kZeroMost memory ranges zeroed by one launch: a compile clears some 45 buffers,
 // and a memset of a small one costs the stream about 2 us whatever its size.  Ranges start
-// on 16-byte boundaries; their lengths round up to 16 bytes.
+// on 16-byte boundaries; their lengths round up to 16 bytes (allocations are in whole 16-byte
+// words).  launch_zero refuses a list that was given more.
 constexpr int kZeroMost = 24;
 struct ZeroList {
     uint4* p[kZeroMost];
     uint64_t n16[kZeroMost];
     int count = 0;
     void add(void* q, size_t bytes) {
-        p[count] = static_cast<uint4*>(q);
-        n16[count++] = (bytes + 15u) / 16u;
+        if (count < kZeroMost) {
+            p[count] = static_cast<uint4*>(q);
+            n16[count] = cleared_bytes(bytes) / 16u;
+        }
+        ++count;
     }
 };
 cudaError_t launch_zero(const ZeroList& z, cudaStream_t s);

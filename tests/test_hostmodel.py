@@ -158,3 +158,25 @@ def test_packed_gen_tables_decode_to_the_code_tables(built):
     """isn_gen reads each node type's four slots from one packed 16-byte record; every
     field must fit and decode to the table it was packed from."""
     assert hostmodel().ptlhm_gen_desc_ok() == 1
+
+
+@pytest.mark.parametrize("elem", [1, 4, 8, 12, 16, 40])
+def test_cleared_buffers_stay_inside_their_allocation(built, elem):
+    """A generator's buffer is kept while a later size fits its allocation, and cleared in
+    16-byte words: for every size that fits, inside what the first size allocated."""
+    L = hostmodel()
+    L.ptlhm_buffer_bytes.argtypes = [ctypes.c_size_t, ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)]
+    L.ptlhm_buffer_bytes.restype = None
+
+    def sizes(n):
+        out = (ctypes.c_size_t * 3)()
+        L.ptlhm_buffer_bytes(n, elem, out)
+        return list(out)
+
+    for first in range(0, 400, 8):
+        need, _, allocated = sizes(first)
+        assert allocated >= need + need // 4 and allocated % 16 == 0
+        n = first
+        while sizes(n)[0] <= allocated:
+            assert sizes(n)[1] <= allocated, (first, n)
+            n += 1
