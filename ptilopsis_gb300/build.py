@@ -30,7 +30,7 @@ SYNTH_LIB = os.path.join(LIBDIR, "libptlsynth.so")
 HOSTMODEL_LIB = os.path.join(LIBDIR, "libptl_hostmodel.so")
 
 HEADERS = ["ptl_device.h", "ptl_common.cuh", "ptl_stages.cuh", "ptl_sort.cuh", "ptl_ra.cuh", "ptl_steps.cuh", "ptl_chunks.cuh", "ptl_scalar.cuh", "ptl_kernels.cuh",
-           "ptl_bpipe.h"]
+           "ptl_flatten.cuh", "ptl_bpipe.h"]
 
 
 def _nvcc() -> str:
@@ -92,7 +92,7 @@ def build_synth(force: bool = False) -> str:
 
 def build_hostmodel(force: bool = False) -> str:
     srcs = _src("ptl_hostmodel.cpp", "ptl_tables.cpp", "ptl_common.cuh", "ptl_stages.cuh", "ptl_sort.cuh", "ptl_ra.cuh", "ptl_steps.cuh",
-                "ptl_chunks.cuh", "ptl_scalar.cuh")
+                "ptl_chunks.cuh", "ptl_flatten.cuh", "ptl_scalar.cuh")
     if not force and _newer(HOSTMODEL_LIB, srcs):
         return HOSTMODEL_LIB
     os.makedirs(LIBDIR, exist_ok=True)

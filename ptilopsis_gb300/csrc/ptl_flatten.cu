@@ -15,11 +15,11 @@
 //   2. the tour: events enter(v) = 2v and exit(v) = 2v+1, and an end event 2n.  enter(v)
 //      goes to enter(first child) or exit(v); exit(v) to enter(next sibling), exit(parent)
 //      or, for the root, the end;
-//   3. the ranking by splitters: one enter in 8 or 16 (by a hash of the node) and the root's.
-//      A thread per splitter walks the tour to the next splitter and sums two weights --
-//      1 per exit (post-order: v's index is n minus the exits from exit(v) on) and +1 per
-//      enter / -1 per exit (depth); pointer jumping sums them over the splitters to the
-//      end; a second walk gives every node its index and depth;
+//   3. the ranking by splitters: one event in 16 or 32 (ptl_flatten.cuh) and the root's
+//      enter.  A thread per splitter walks the tour to the next splitter and sums two
+//      weights -- 1 per exit (post-order: v's index is n minus the exits from exit(v) on)
+//      and +1 per enter / -1 per exit (depth); pointer jumping sums them over the splitters
+//      to the end; a second walk gives every node its index and depth;
 //   4. the six arrays in post-order.
 // The root's enter must see all n exits; fewer means nodes the root does not reach (a
 // cycle of parents), an INVALID_AST.  No kernel waits on another block.
@@ -28,7 +28,8 @@
 // some 16 to 32 events (the longest, about ln(splitters) times that, ends last).  4.3M
 // nodes on the device: 0.90 ms; pointer jumping over all events, which read and wrote 32
 // bytes per event in each of 24 rounds, with a same-address atomic per node for the depth
-// and per child for the counts, took 4.1 ms.
+// and per child for the counts, took 4.1 ms.  Where some walk is longer than walk_most (the
+// nodes' numbers follow the hash), that ranking is done after all.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,8 +37,11 @@
 
 #include "../../include/ptl_codegen.h"
 #include "ptl_device.h"
+#include "ptl_flatten.cuh"
 
 namespace {
+
+using namespace ptl;
 
 constexpr int kThreads = 256;
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
@@ -57,14 +61,18 @@ struct NodeRec {
     uint32_t data, types;
 };
 
-// Whether enter(v) is a splitter (besides the root's): one node in 2^lg, spread evenly over
-// any run of consecutive nodes (multiplicative hashing by the golden ratio).
-__host__ __device__ __forceinline__ bool is_splitter(uint32_t v, uint32_t lg) {
-    return ((v * 0x9E3779B1u) >> (32u - lg)) == 0;
-}
+// An event of the ranking by pointer jumping over all of them.
+struct Event {
+    uint32_t next;   // event further on (2n: the end)
+    uint32_t exits;  // exits from here up to there
+    int32_t level;   // enters minus exits
+    uint32_t pad;
+};
+
+constexpr uint32_t kFar = 2;  // some walk is longer than walk_most: the ranking is still to be done
 
 struct FlatErr {
-    uint32_t code;     // 0 ok, 1 invalid
+    uint32_t code;     // 0 ok, 1 invalid, kFar
     uint32_t detail;   // the first node found bad
     uint32_t roots;    // nodes with parent -1
     uint32_t max_depth;
@@ -207,7 +215,7 @@ __global__ void k_fl_place(const NodeRec* rec, uint32_t n, const uint32_t* deg, 
 }
 
 // The tour (successors of enter(v) and exit(v)), and the splitters in any order: split[k]
-// is splitter k's node, sidx its k.  From here on the input is flagged or every slot holds
+// is splitter k's event, sidx of its node is k.  From here on the input is flagged or every slot holds
 // one child, so no two events have the same successor but the end.
 __global__ void k_fl_tour(const NodeRec* rec, uint32_t n, const uint32_t* deg, const uint32_t* off,
                           const uint32_t* kids, uint32_t lg, uint2* succ, uint32_t* split, uint32_t cap, uint32_t* sidx,
@@ -232,26 +240,31 @@ __global__ void k_fl_tour(const NodeRec* rec, uint32_t n, const uint32_t* deg, c
             }
         }
         succ[v] = make_uint2(s, x);
-        if (r.x < 0 || is_splitter(v, lg)) {
+        auto add = [&](uint32_t event) {
             const uint32_t k = atomicAdd(&e->splitters, 1u);
             if (k < cap) {
-                split[k] = v;
+                split[k] = event;
                 sidx[v] = k;
             } else {
                 flag(e, v);  // several roots
             }
-        }
+        };
+        // The root's enter, which follows nothing, is always one, and its exit may be too:
+        // sidx is the latter's.  (One add for both kinds: the counter's atomics are 0.1 ms
+        // of 4.3M nodes' as it is.)
+        const bool enter = r.x < 0 || is_splitter(2u * v, lg), exit = is_splitter(2u * v + 1u, lg);
+        if (enter || exit) add(enter ? 2u * v : 2u * v + 1u);
+        if (r.x < 0 && exit) add(2u * v + 1u);
     }
 }
 
-// From each splitter to the next: how far, and to which.  The walk ends: no two events
-// share a successor, so it leads to the end or back to a splitter.
+// From each splitter to the next: how far, and to which.
 __global__ void k_fl_walk(const uint32_t* succ, const uint32_t* split, const uint32_t* sidx,
                           uint32_t n, uint32_t lg, Rank* rank, FlatErr* e) {
     if (bad(e)) return;
     const uint32_t count = e->splitters, end = 2u * n;
     FL_FOR(k, count) {
-        uint32_t x = 2u * split[k], exits = 0;
+        uint32_t x = split[k], exits = 0, steps = 0;
         int32_t level = 0;
         uint32_t next = count;
         for (;;) {
@@ -259,8 +272,12 @@ __global__ void k_fl_walk(const uint32_t* succ, const uint32_t* split, const uin
             level += (x & 1u) ? -1 : 1;
             x = succ[x];
             if (x == end) break;
-            if (!(x & 1u) && is_splitter(x >> 1, lg)) {  // the root's enter follows nothing
+            if (is_splitter(x, lg)) {
                 next = sidx[x >> 1];
+                break;
+            }
+            if (++steps == walk_most(lg)) {
+                e->code = kFar;
                 break;
             }
         }
@@ -279,18 +296,18 @@ __global__ void k_fl_jump(const Rank* __restrict__ in, Rank* __restrict__ out, c
     }
 }
 
-// The walks again, with what lies behind each splitter known: every node's post-order
-// index (post), and by index its node and depth (at).
+// The walks again (all within walk_most), with what lies behind each splitter known: every
+// node's post-order index (post), and by index its node and depth (at).
 __global__ void k_fl_number(const uint32_t* succ, const NodeRec* rec, const uint32_t* split, uint32_t n, uint32_t lg,
                             const Rank* rank, int32_t* post, uint2* at, FlatErr* e) {
     if (bad(e)) return;
     const uint32_t count = e->splitters, end = 2u * n;
     uint32_t deepest = 0;
     FL_FOR(k, count) {
-        uint32_t x = 2u * split[k];
+        uint32_t x = split[k];
         uint32_t exits = rank[k].exits;  // from x to the end
         int32_t level = rank[k].level;
-        if (rec[x >> 1].parent == -1) e->reached = exits;
+        if (!(x & 1u) && rec[x >> 1].parent == -1) e->reached = exits;
         for (;;) {
             if (x & 1u) {
                 const uint32_t v = x >> 1, q = n - exits;
@@ -306,8 +323,40 @@ __global__ void k_fl_number(const uint32_t* succ, const NodeRec* rec, const uint
                 --level;
             }
             x = succ[x];
-            if (x == end || (!(x & 1u) && is_splitter(x >> 1, lg))) break;
+            if (x == end || is_splitter(x, lg)) break;
         }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) deepest = max(deepest, __shfl_down_sync(0xFFFFFFFFu, deepest, d));
+    if ((threadIdx.x & 31u) == 0 && deepest) atomicMax(&e->max_depth, deepest);
+}
+
+// The ranking without splitters, of a tour with a walk longer than walk_most: pointer
+// jumping over all events, as many rounds whatever the nodes' numbers (n = 117k: 0.35 ms,
+// where the longest walks took 37).
+__global__ void k_fl_events(const uint32_t* succ, uint32_t n, Event* ev) {
+    const uint64_t end = 2ull * n;
+    FL_FOR(x, end) ev[x] = Event{succ[x], x & 1u, (x & 1u) ? -1 : 1, 0u};
+    if (blockIdx.x == 0 && threadIdx.x == 0) ev[end] = Event{static_cast<uint32_t>(end), 0u, 0, 0u};
+}
+__global__ void k_fl_event_jump(const Event* __restrict__ in, Event* __restrict__ out, uint64_t events) {
+    FL_FOR(x, events) {
+        const uint4 a = reinterpret_cast<const uint4*>(in)[x];
+        const uint4 b = reinterpret_cast<const uint4*>(in)[a.x];
+        reinterpret_cast<uint4*>(out)[x] = make_uint4(b.x, a.y + b.y, a.z + b.z, 0u);
+    }
+}
+__global__ void k_fl_event_number(const Event* ev, const NodeRec* rec, uint32_t n, int32_t* post, uint2* at, FlatErr* e) {
+    uint32_t deepest = 0;
+    FL_FOR(v, n) {
+        const uint32_t q = n - ev[2ull * v + 1u].exits;
+        const int32_t depth = -ev[2ull * v].level;
+        if (q < n) {  // else a node the root does not reach
+            post[v] = static_cast<int32_t>(q);
+            at[q] = make_uint2(v, static_cast<uint32_t>(depth));
+        }
+        if (depth > 0) deepest = max(deepest, static_cast<uint32_t>(depth));
+        if (rec[v].parent == -1) e->reached = ev[2ull * v].exits;
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) deepest = max(deepest, __shfl_down_sync(0xFFFFFFFFu, deepest, d));
@@ -368,13 +417,11 @@ extern "C" ptl_status ptl_flatten(const ptl_tree_view* in, ptl_depth_tree_out* o
     uint2 *succ = nullptr, *at = nullptr;
     uint32_t *split = nullptr, *sidx = nullptr;
     Rank *rank0 = nullptr, *rank1 = nullptr;
+    Event *ev0 = nullptr, *ev1 = nullptr;
     FlatErr* err = nullptr;
     FlatErr herr{};
     const uint32_t tiles = static_cast<uint32_t>((n64 + 1 + kScanTile - 1) / kScanTile);
-    // A splitter per 16 nodes of a large tree, per 8 of a small one (whose walks are over
-    // sooner than the jumps between more splitters cost).
-    const uint32_t lg = n >= (1u << 20) ? 4u : 3u;
-    const uint32_t cap = (n >> lg) + (n >> (lg + 2u)) + 64u;
+    const uint32_t lg = splitter_lg(n), cap = splitters_most(n);
     ptl_status st = PTL_OK;
     cudaError_t ce = cudaSuccess;
 #define FL_CU(x)                       \
@@ -442,6 +489,29 @@ extern "C" ptl_status ptl_flatten(const ptl_tree_view* in, ptl_depth_tree_out* o
                                               o_order, err);
     FL_CU(cudaGetLastError());
     FL_CU(cudaMemcpyAsync(&herr, err, sizeof(herr), cudaMemcpyDeviceToHost, s));
+    FL_CU(cudaStreamSynchronize(s));
+    if (herr.code == kFar) {
+        const uint64_t events = 2 * n64 + 1;
+        for (void* p : {static_cast<void*>(deg), static_cast<void*>(off), static_cast<void*>(kids),
+                        static_cast<void*>(split), static_cast<void*>(sidx), static_cast<void*>(rank0),
+                        static_cast<void*>(rank1)})  // done with; the events take 64 bytes a node
+            cudaFreeAsync(p, s);
+        deg = off = kids = split = sidx = nullptr;
+        rank0 = rank1 = nullptr;
+        FL_CU(cudaMemsetAsync(&err->code, 0, sizeof(err->code), s));
+        FL_CU(dev_alloc(&ev0, events, s));
+        FL_CU(dev_alloc(&ev1, events, s));
+        k_fl_events<<<grid_of(events), kThreads, 0, s>>>(reinterpret_cast<const uint32_t*>(succ), n, ev0);
+        for (uint32_t r = 0; (1ull << r) < events; ++r) {
+            k_fl_event_jump<<<grid_of(events), kThreads, 0, s>>>(ev0, ev1, events);
+            std::swap(ev0, ev1);
+        }
+        k_fl_event_number<<<grid_of(n), kThreads, 0, s>>>(ev0, rec, n, post, at, err);
+        k_fl_emit<<<grid_of(n), kThreads, 0, s>>>(rec, n, post, at, o_type, o_rtype, o_parent, o_depth, o_child, o_data,
+                                                  o_order, err);
+        FL_CU(cudaGetLastError());
+        FL_CU(cudaMemcpyAsync(&herr, err, sizeof(herr), cudaMemcpyDeviceToHost, s));
+    }
     if (!out->on_device) {
         FL_CU(cudaMemcpyAsync(out->parent, o_parent, 4 * n64, cudaMemcpyDeviceToHost, s));
         FL_CU(cudaMemcpyAsync(out->depth, o_depth, 4 * n64, cudaMemcpyDeviceToHost, s));
@@ -460,7 +530,8 @@ done:
                     static_cast<void*>(off), static_cast<void*>(kids), static_cast<void*>(tsum),
                     static_cast<void*>(post), static_cast<void*>(rec), static_cast<void*>(succ),
                     static_cast<void*>(at), static_cast<void*>(split), static_cast<void*>(sidx),
-                    static_cast<void*>(rank0), static_cast<void*>(rank1), static_cast<void*>(err)})
+                    static_cast<void*>(rank0), static_cast<void*>(rank1), static_cast<void*>(ev0),
+                    static_cast<void*>(ev1), static_cast<void*>(err)})
         if (p) cudaFreeAsync(p, s);
     if (ce != cudaSuccess) {
         cudaStreamSynchronize(s);

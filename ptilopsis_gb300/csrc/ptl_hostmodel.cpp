@@ -18,6 +18,7 @@
 #include "ptl_stages.cuh"
 #include "ptl_ra.cuh"
 #include "ptl_chunks.cuh"
+#include "ptl_flatten.cuh"
 #include "ptl_scalar.cuh"
 
 using namespace ptl;
@@ -617,6 +618,38 @@ int ptlhm_gen_desc_ok(void) {
     return gen_desc_ok(&t) ? 1 : 0;
 }
 int ptlhm_last_locked(void) { return g_last_locked ? 1 : 0; }
+// The flattening's walks over a valid tree's tour: the longest, its limit, the splitters
+// and their limit.
+void ptlhm_flatten_walks(const int32_t* parent, const int32_t* child, uint32_t n, uint32_t out[4]) {
+    std::vector<uint32_t> deg(n, 0), off(n + 1, 0), kids(n), succ(2 * static_cast<size_t>(n));
+    for (uint32_t v = 0; v < n; ++v)
+        if (parent[v] >= 0) ++deg[parent[v]];
+    for (uint32_t v = 0; v < n; ++v) off[v + 1] = off[v] + deg[v];
+    uint32_t root = 0;
+    for (uint32_t v = 0; v < n; ++v) {
+        if (parent[v] >= 0) kids[off[parent[v]] + child[v]] = v;
+        else root = v;
+    }
+    const uint32_t lg = splitter_lg(n), end = 2 * n;
+    for (uint32_t v = 0; v < n; ++v) {
+        const uint32_t p = static_cast<uint32_t>(parent[v]), c = static_cast<uint32_t>(child[v]) + 1u;
+        succ[2 * v] = deg[v] ? 2 * kids[off[v]] : 2 * v + 1;
+        succ[2 * v + 1] = v == root ? end : (c < deg[p] ? 2 * kids[off[p] + c] : 2 * p + 1);
+    }
+    uint32_t longest = 0, steps = 0, splitters = 1;  // the root's enter
+    for (uint32_t x = succ[2 * root]; x != end; x = succ[x]) {
+        ++steps;
+        if (is_splitter(x, lg)) {
+            ++splitters;
+            steps = 0;
+        }
+        longest = std::max(longest, steps);
+    }
+    out[0] = longest;
+    out[1] = walk_most(lg);
+    out[2] = splitters;
+    out[3] = splitters_most(n);
+}
 // Of a buffer of n elements: the bytes it needs, those that clearing it writes, and those
 // allocated for it.
 void ptlhm_buffer_bytes(size_t n, size_t elem, size_t out[3]) {

@@ -219,3 +219,74 @@ def test_gpu_flatten_splitter_walks(built_cuda, n):
         np.testing.assert_array_equal(tree.depth, want_depth)
         np.testing.assert_array_equal(order[at], np.arange(n))
         assert tree.max_depth == depth.max()
+
+
+# ---------------------------------------------------------------- walks of any numbering
+def renumbered(arrs, at):
+    """The tree with node k as node at[k]."""
+    out = []
+    for a in (arrs[0], arrs[1], np.where(arrs[2] >= 0, at[np.maximum(arrs[2], 0)], -1).astype(np.int32), arrs[3], arrs[4]):
+        b = np.empty_like(a)
+        b[at] = a
+        out.append(b)
+    return out
+
+
+def splitters_last(n):
+    """A numbering of n nodes that gives the first of them the numbers that are no splitters
+    (ptl_flatten.cuh's rule, enters and exits)."""
+    lg = 5 if n >= 1 << 20 else 4
+    top = ((np.arange(2 * n, dtype=np.uint64) * np.uint64(0x9E3779B1)) & np.uint64(0xFFFFFFFF)) >> np.uint64(32 - lg)
+    splitter = (top.reshape(n, 2) == 0).any(axis=1)
+    return np.concatenate([np.flatnonzero(~splitter), np.flatnonzero(splitter)])
+
+
+def _walks(arrs):
+    import ctypes
+    from test_hostmodel import hostmodel
+    parent, child = np.ascontiguousarray(arrs[2], np.int32), np.ascontiguousarray(arrs[3], np.int32)
+    out = (ctypes.c_uint32 * 4)()
+    hostmodel().ptlhm_flatten_walks(ctypes.c_void_p(parent.ctypes.data), ctypes.c_void_p(child.ctypes.data),
+                                    ctypes.c_uint32(len(parent)), out)
+    longest, most, splitters, cap = list(out)
+    assert splitters <= cap
+    return longest, most
+
+
+def test_flatten_walks_stay_short(built):
+    """A walk from one splitter to the next is bounded by the splitters' spacing, not by the
+    depth or width of the tree; only numbers that follow the splitters' hash make longer
+    ones (pointer jumping then ranks the tour)."""
+    rng = np.random.default_rng(11)
+    t = synth_tree(0x50544E70, fns=60, median=900.0)
+    for arrs in (chain(1000), chain(100_000), star(100_000), (t.type, t.rtype, t.parent, t.child_idx, t.data)):
+        n = len(arrs[2])
+        for at in (np.arange(n), np.arange(n)[::-1], rng.permutation(n)):
+            longest, most = _walks(renumbered(arrs, at))
+            assert longest < most, n
+    for arrs in (chain(5000), star(5000)):
+        longest, most = _walks(renumbered(arrs, splitters_last(len(arrs[2]))))
+        assert longest > most
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [700, 5000, 30_000])
+def test_gpu_flatten_any_numbering(built_cuda, n):
+    """Deep, wide and ordinary trees whose numbers keep the splitters to the tour's end, so
+    that walks reach their limit (700 nodes: just below it), and malformed ones."""
+    from oracle import portbind
+    from ptilopsis_gb300 import PtlError, flatten
+    t = synth_tree(0x50544E80 + n, fns=max(1, n // 900), median=900.0)
+    for arrs in (chain(n), star(n - 1), (t.type, t.rtype, t.parent, t.child_idx, t.data)):
+        arrs = renumbered(arrs, splitters_last(len(arrs[2])))
+        want, want_order = portbind.flatten(*arrs)
+        got, order = flatten(*arrs)
+        assert_tree(got, want)
+        np.testing.assert_array_equal(order, want_order)
+    arrs = renumbered(chain(n), splitters_last(n))  # a cycle away from the root
+    leaf = int(np.flatnonzero(np.bincount(arrs[2][arrs[2] >= 0], minlength=n) == 0)[0])
+    above = int(arrs[2][int(arrs[2][leaf])])
+    arrs[2][above] = leaf
+    with pytest.raises(PtlError) as e:
+        flatten(*arrs)
+    assert e.value.status == 1
