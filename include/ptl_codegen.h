@@ -78,10 +78,10 @@ ptl_status ptl_generator_create_scalar(const ptl_ast_view* tree, int device, ptl
  * the seven stages.  Unlike the reference, which mutates its arrays and cannot be run
  * twice, process may be called again and recompiles from the copied tree.
  * profile bits: 1 = per-stage device times (ptl_generator_stage_ns); 2 = leave the words
- * on the device (ptl_generator_device_instructions); 4 = the register allocator finds
- * row-0 values through its hash table even when every virtual register has one
- * definition (the general path, normally taken only when one has two; same output);
- * 8 = a scalar generator allocates registers in the reference's serial order for every
+ * on the device (ptl_generator_device_instructions); 16 = the register allocator takes
+ * its general form (normally only for programs that its packed records cannot say; same
+ * output); 4 = that form, which finds row-0 values through its hash table even when every
+ * virtual register has one definition (same output); 8 = a scalar generator allocates registers in the reference's serial order for every
  * program (normally only for programs whose functions name each other's words; same
  * output). */
 ptl_status ptl_generator_process(ptl_generator* gen, int profile);

@@ -249,11 +249,13 @@ class RvGenerator:
         self.n = tree.n
 
     def process(self, profile: bool = False, to_host: bool = True, row0_hash: bool = False,
-                serial: bool = False) -> None:
+                serial: bool = False, general: bool = False) -> None:
         """rv_generator_avx::process.  to_host=False leaves the words on the device;
-        row0_hash=True takes the register allocator's general row-0 lookup, serial=True
-        the scalar generator's serial register allocation (both: same output)."""
-        flags = (1 if profile else 0) | (0 if to_host else 2) | (4 if row0_hash else 0) | (8 if serial else 0)
+        general=True takes the register allocator's general form, row0_hash=True that form
+        with its general row-0 lookup, serial=True the scalar generator's serial register
+        allocation (all: same output)."""
+        flags = ((1 if profile else 0) | (0 if to_host else 2) | (4 if row0_hash else 0) | (8 if serial else 0) |
+                 (16 if general else 0))
         self._check(self._lib.ptl_generator_process(self._h, flags), "process")
 
     def set_chunk_limits(self, rounds: int = 0, wait_cycles: int = 0) -> None:

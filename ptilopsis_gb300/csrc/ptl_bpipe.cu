@@ -137,7 +137,7 @@ public:
     DBuf nt, rt, nd1, nd, par, ci, dep, loc0, loc, pos, decl, fflag, regs;
     DBuf fn_id, fn_start, fn_size, fn_end, fn_start0, fn_size0, ra_order, lifetime;
     DBuf instr, rd, rs1, rs2, jt, used_instrs, symreg, symswp, stamp, spill, roffs, owner, used, smark;
-    DBuf tmask, trow, tany, lane_zero, lane_rest;
+    DBuf tmask, trow, tany, lane_zero, lane_rest, defpos;
     DBuf trig_min, trig_max, ra_chunks;
     DBuf ni, nrd, nr1, nr2, njt, joffs, out;
     DBuf errw, flags, meta, progs, tabs, lists, changed, sort_err, a_off, dirty, ra_sync;
@@ -171,7 +171,7 @@ public:
         return {&tab, &in_type, &in_rtype, &in_parent, &in_depth, &in_child, &in_data, &nt, &rt, &nd1, &nd, &par,
                 &ci, &dep, &loc0, &loc, &pos, &decl, &fflag, &regs, &fn_id, &fn_start, &fn_size,
                 &fn_end, &fn_start0, &fn_size0, &ra_order, &lifetime, &instr, &rd, &rs1, &rs2, &jt, &used_instrs, &symreg,
-                &symswp, &stamp, &spill, &roffs, &owner, &used, &smark, &tmask, &trow, &tany, &lane_zero, &lane_rest, &trig_min, &trig_max, &ra_chunks, &ni, &nrd,
+                &symswp, &stamp, &spill, &roffs, &owner, &used, &smark, &tmask, &trow, &tany, &lane_zero, &lane_rest, &defpos, &trig_min, &trig_max, &ra_chunks, &ni, &nrd,
                 &nr1, &nr2, &njt, &joffs, &out, &errw, &flags, &meta, &progs, &tabs, &lists, &changed,
                 &sort_err, &a_off, &dirty, &ra_sync, &sa, &sapos, &sbpos, &seg0, &seg1, &tile_seg, &tile_l, &tile_r,
                 &sort_stops, &leaf, &heap, &counters, &scan_status, &scan_counter, &sort_local, &sort_equal,
@@ -427,7 +427,7 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
     for (auto& x : hns) x = 0;
 
     // ---- small per-program state and the pinned small area
-    constexpr int kTables = 27, kLists = 6;  // table slots 0..26 are used
+    constexpr int kTables = 29, kLists = 6;  // table slots 0..28 are used
     small_progs_off = static_cast<size_t>(kTables) * (B + 1) * 4;
     small_meta_off = small_progs_off + B * sizeof(Prog);
     small_err_off = small_meta_off + B * 16;
@@ -1034,6 +1034,20 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
                 hp[p].trig_max = trig_max.at<uint32_t>(Lt.elem(p));
                 hp[p].ra_chunks = ra_chunks.at<uint32_t>(Lc.elem(p));
             }
+            // definition positions, where they tell (ra_positions_tell)
+            BP_CU(cudaMemsetAsync(flags.p, 0, B * 16, s));
+            const uint32_t t_def = tiles(27, W, elem_tile, &general), t_range = tiles(28, F, elem_tile, &general);
+            batch_stage(BatchStage::Definitions, bl(27), t_def, nullptr);
+            batch_stage(BatchStage::Ranges, bl(28), t_range, nullptr);
+            std::vector<uint32_t> more(4 * B);
+            BP_CU(cudaMemcpyAsync(more.data(), flags.p, B * 16, cudaMemcpyDeviceToHost, s));
+            BP_CU(cudaStreamSynchronize(s));
+            Layout Lp;
+            Lp.build(wb8, general);
+            BP_CU(family(Lp, {&defpos}, 1));
+            for (size_t p = 0; p < B; ++p)
+                if (general[p] && !more[4 * p + 2] && ra_positions_pay(static_cast<uint32_t>((F[p] + 7) / 8)))
+                    hp[p].defpos = defpos.at<uint8_t>(Lp.elem(p));
         }
         upload_progs();
         if (!step_list.empty()) {  // blocks of program order[k], longest program first
@@ -1122,8 +1136,10 @@ ptl_status Pipeline::compile(const ptl_ast_view* trees, size_t count, std::vecto
         const uint32_t* d_serial = upload_list(1, serial_list);
         batch_serial(progs.at<Prog>(), d_serial, static_cast<uint32_t>(serial_list.size()), s);
         for (const uint32_t p : wide_list) {
+            Prog Pfree = hp[p];
+            Pfree.defpos = nullptr;  // the independent functions never need definition positions
             bool launched = false;
-            BP_CU(launch_ra_wide(hp[p], hp[p], static_cast<uint32_t>((F[p] + 7) / 8), s, &launched));
+            BP_CU(launch_ra_wide(hp[p], Pfree, static_cast<uint32_t>((F[p] + 7) / 8), s, &launched));
             if (!launched) return cuda_fail(cudaErrorLaunchFailure, "lane-0 cluster pass");
         }
         }  // the AVX generator's allocation

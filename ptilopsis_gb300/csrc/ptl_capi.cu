@@ -95,7 +95,7 @@ struct ptl_generator {
     DevBuf fn_ra_start, fn_ra_end, fn_ra_size;
     DevBuf instr, rd, rs1, rs2, jt, owner, used, smark, used_instrs;
     DevBuf tmask, trow, tany, lane_zero, lane_rest, opt_work;
-    DevBuf symreg, symswp, stamp, lifetime, trig_min, trig_max, ra_chunks, spill, roffs;
+    DevBuf symreg, symswp, stamp, defpos, lifetime, trig_min, trig_max, ra_chunks, spill, roffs;
     DevBuf ni, nrd, nr1, nr2, njt, fsz, joffs, out;
     DevBuf sort_a, sort_apos, sort_bpos, sort_seg0, sort_seg1, sort_tile_seg, sort_tile_l, sort_tile_r, sort_stops,
         sort_leaf, sort_heap, sort_counters, sort_local, sort_equal;
@@ -140,7 +140,7 @@ struct ptl_generator {
                 &par, &ci, &dep, &fflag, &sizes, &loc0, &loc, &pos, &regs, &decl, &fn_id, &fn_start,
                 &fn_size, &fn_end, &fn_start0, &fn_size0, &fn_end0, &fn_ra_start, &fn_ra_end, &fn_ra_size,
                 &instr, &rd, &rs1, &rs2, &jt, &owner, &used, &smark, &used_instrs, &tmask, &trow, &tany, &lane_zero, &lane_rest, &opt_work, &symreg, &symswp,
-                &stamp, &lifetime, &trig_min, &trig_max, &ra_chunks, &spill, &roffs, &ni, &nrd, &nr1, &nr2, &njt,
+                &stamp, &defpos, &lifetime, &trig_min, &trig_max, &ra_chunks, &spill, &roffs, &ni, &nrd, &nr1, &nr2, &njt,
                 &fsz, &joffs, &out, &sort_a, &sort_apos, &sort_bpos, &sort_seg0, &sort_seg1, &sort_stops,
                 &sort_tile_seg, &sort_tile_l, &sort_tile_r, &sort_leaf, &sort_heap, &sort_counters, &sort_local, &sort_equal,
                 &scan_status, &meta, &flags, &errw, &tables, &preserve, &sregs, &ssteps,
@@ -510,9 +510,10 @@ cudaError_t sort_scratch(ptl_generator* g, size_t n, SortScratch* ss) {
     return cudaSuccess;
 }
 
-// row0_hash: the AVX allocator's general row-0 lookup; serial: the scalar allocator in
-// the reference's order for every program.  Both leave the output unchanged.
-ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_hash, bool serial) {
+// general: the AVX allocator's general form for every program; row0_hash: that form with
+// its general row-0 lookup; serial: the scalar allocator in the reference's order for every
+// program.  All leave the output unchanged.
+ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_hash, bool serial, bool general) {
     cudaStream_t s = g->stream;
     const size_t n = g->n;
     const size_t nb8 = r8(n);
@@ -657,7 +658,14 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
             return fail(g, PTL_CUDA_ERROR, "internal: unallocated regalloc state");
         RaForm form = RaForm::Serial;
         uint32_t items = 0;
-        PTL_CU(ra_form(P, s, row0_hash, &form, &items));
+        PTL_CU(ra_form(P, s, general || row0_hash, &form, &items));
+        bool positions = false;
+        if (form == RaForm::General && !row0_hash && ra_positions_pay((g->F + 7u) / 8u))
+            PTL_CU(ra_positions_tell(P, s, &positions));
+        if (positions) {
+            PTL_CU(g->defpos.ensure(wb8, 1));
+            PTL_CU(g->defpos.zero(s));
+        }
         ChunkSizes chunk{};
         ChunkBatch chunks{};
         const bool in_chunks = form == RaForm::Steps && items != 0 && g->S >= kChunkMinSteps && chunks_fit();
@@ -693,6 +701,7 @@ ptl_status run_pipeline(ptl_generator* g, bool profile, bool to_host, bool row0_
         if (form == RaForm::Steps ? !prog_ready(P, {P.tmask, P.trow, P.tany})
                                   : form == RaForm::General && !prog_ready(P, {P.trig_min, P.trig_max, P.ra_chunks}))
             return fail(g, PTL_CUDA_ERROR, "internal: unallocated regalloc state");
+        P.defpos = positions ? g->defpos.at<uint8_t>() : nullptr;
         if (in_chunks) chunk_bind(P.ch, chunk, g->lane_zero.at<char>(), g->lane_rest.at<char>());
         PTL_CU(run_regalloc_steps(P, form, in_chunks ? &chunks : nullptr, s));
         g->ra_serial = form == RaForm::Serial;
@@ -842,7 +851,7 @@ ptl_status ptl_generator_process(ptl_generator* g, int profile) {
     const DeviceScope on_device(g->device);
     if (!on_device.ok()) return fail(g, PTL_CUDA_ERROR, "cudaSetDevice");
     const ptl_status st =
-        run_pipeline(g, (profile & 1) != 0, (profile & 2) == 0, (profile & 4) != 0, (profile & 8) != 0);
+        run_pipeline(g, (profile & 1) != 0, (profile & 2) == 0, (profile & 4) != 0, (profile & 8) != 0, (profile & 16) != 0);
     if (st == PTL_OK) g->last_error.clear();
     return st;
 }

@@ -29,8 +29,9 @@ bool g_last_locked = false;  // the last program's symbols did not fit the slots
 bool g_chunks = true;  // lane-0 functions in chunks (else in lock-step)
 uint32_t g_ring_k = 16;  // words per function in the record form's symbol ring (small: old words too)
 uint32_t g_cache_k = 4;  // entries per function of the lane-0 symbol cache
-bool g_force_hashed = false;  // lane-0 pass finds row-0 values by hashing even when definitions are unique
-bool g_last_hashed = false;   // the last compile had a lane-0 virtual register with two definitions
+bool g_force_general = false; // the general form for every program
+bool g_force_hashed = false;  // ... which finds row-0 values by hashing even when definitions are unique
+bool g_last_hashed = false;   // the last compile did
 bool g_last_cross = false;    // the last scalar compile took the serial register allocation
 bool g_force_tiles = false;   // scalar register allocation by word tiles for every program
 bool g_force_serial = false;  // scalar register allocation in the reference's order for every program
@@ -53,7 +54,7 @@ struct Model {
     CodeTables tab;
     ErrorWord err{};
     uint32_t flags[4] = {0, 0, 0, 0};
-    HBuf<uint8_t> in_type, in_rtype, fflag, used, smark, nt, rt;
+    HBuf<uint8_t> in_type, in_rtype, fflag, used, smark, defpos, nt, rt;
     HBuf<int32_t> in_parent, in_depth, in_child, par, ci, dep;
     HBuf<uint32_t> in_data, nd1, nd, sizes, loc0, loc, regs, pos, decl, fn_id, fn_start, fn_size,
         fn_end, fn_start0, fn_size0, fn_end0, fn_ra_start, fn_ra_end, fn_ra_size, instr, rd, rs1, rs2, jt,
@@ -72,6 +73,7 @@ struct Model {
         P.fn_end = fn_end.p; P.fn_start0 = fn_start0.p; P.fn_size0 = fn_size0.p; P.instr = instr.p;
         P.rd = rd.p; P.rs1 = rs1.p; P.rs2 = rs2.p; P.jt = jt.p; P.used = used.p; P.smark = smark.p;
         P.used_instrs = used_instrs.p; P.symreg = symreg.p; P.symswp = symswp.p; P.stamp = stamp.p;
+        P.defpos = defpos.p;
         P.lifetime = lifetime.p; P.trig_min = trig_min.p; P.trig_max = trig_max.p; P.spill = spill.p;
         P.roffs = roffs.p; P.ni = ni.p; P.nrd = nrd.p; P.nr1 = nr1.p; P.nr2 = nr2.p; P.njt = njt.p;
         P.fsz = fsz.p; P.joffs = joffs.p; P.out = out.p;
@@ -161,8 +163,10 @@ struct Model {
     uint32_t hm_cache_k = g_cache_k;
 
     // The lane-0 pass with the same phase functions as k_ra_lane0_cached.
-    void lane0_cached(uint32_t S, uint32_t K) {
+    void lane0_cached(uint32_t S, uint32_t K, bool hashed) {
         const uint32_t G0 = (P.F + 7) / 8;
+        const Prog Psave = P;
+        if (hashed) P.defpos = nullptr;
         Ra2Shared sh{};
         std::vector<uint32_t> cur(4 * G0), tag(static_cast<size_t>(G0) * K);
         std::vector<uint32_t> val(static_cast<size_t>(G0) * K);
@@ -174,7 +178,7 @@ struct Model {
             ra2_slot_init(P, c, L[j], j, j);
         }
         for (int p = 0; p < 64; ++p) { sh.R0[p] = 0xFFFFFFFFu; sh.R0own[p] = 0xFFFFFFFFu; }
-        if (S > 0) for (uint32_t p = 0; p < 64; ++p) ra2_begin_p(sh, 0, p, P.trig_min[p], P.trig_max[p]);
+        if (S > 0) for (uint32_t p = 0; p < 64; ++p) ra2_begin_p(sh, 0, p, P.trig_min[p], P.trig_max[p], hashed);
         uint32_t s0 = 0;  // steps with a lane-0 function still running
         for (uint32_t j = 0; j < G0; ++j) s0 = std::max(s0, ra2_lane0_size(L[j]));
         s0 = std::min(s0, S);
@@ -198,20 +202,21 @@ struct Model {
                 }
                 for (uint32_t j = 0; j < G0; ++j) ra2_apply(P, c, sh, L[j], j, i, cur.data() + 4 * j);
             }
-            for (uint32_t p = 0; p < 64; ++p) snap_clear_next(sh, i, p);
+            if (hashed) for (uint32_t p = 0; p < 64; ++p) snap_clear_next(sh, i, p);
             for (uint32_t p = 0; p < 64; ++p) {
                 ra2_end_p(P, c, sh, p, cur.data());
             }
             if (i + 1 < S) {
                 for (uint32_t p = 0; p < 64; ++p) {
                     ra2_begin_p(sh, i + 1, p, P.trig_min[static_cast<size_t>(i + 1) * 64 + p],
-                                P.trig_max[static_cast<size_t>(i + 1) * 64 + p]);
+                                P.trig_max[static_cast<size_t>(i + 1) * 64 + p], hashed);
                 }
             }
         }
         {  // the steps after the last lane-0 function only mark row 0's symbols
             for (uint32_t p = 0; p < 64; ++p) ra2_tail_p(P, c, sh, p, s0, S);
         }
+        P = Psave;
     }
 
     // The lane-0 functions in chunks (ptl_chunks.cuh), round by round as its kernel runs
@@ -503,23 +508,29 @@ struct Model {
         for (uint32_t f = 0; f < F; ++f) lifetime.p[f] = 0x1Full;
         trig_min.ensure(static_cast<size_t>(std::max<uint32_t>(S, 1)) * 64, 0xFFFFFFFFu);
         trig_max.ensure(static_cast<size_t>(std::max<uint32_t>(S, 1)) * 64, 0u);
+        defpos.ensure(wb8);
         bind();
         if (scalar) {
             scalar_regalloc(F, W, wb8);
             if (!check()) return err.code;
         } else {
-            uint32_t flagbits = g_force_hashed ? 2u : 0u;
+            uint32_t flagbits = g_force_general || g_force_hashed ? 2u : 0u;
             for (uint32_t f = 0; f < F; ++f) flagbits |= st_step_range(P, f);
             for (uint32_t i = 0; i < W; ++i) flagbits |= st_step_record(P, i);
-            g_last_hashed = (flagbits & 2u) != 0;
+            g_last_hashed = false;
             const uint32_t G0 = (F + 7) / 8;
             if ((flagbits & 1u) || G0 > 8192u) {
                 st_ra_serial(P, stamp.p);
             } else if (flagbits & 2u) {
                 std::vector<uint32_t> tag(64), val(64);
                 const SymCache c1{tag.data(), val.data(), 64};
-                for (uint32_t f = 0; f < F; ++f) if (f & 7u) ra_free_function_cached(P, c1, 0, f);
-                lane0_cached(S, hm_cache_k);
+                Prog Pfree = P;
+                Pfree.defpos = nullptr;
+                for (uint32_t f = 0; f < F; ++f) if (f & 7u) ra_free_function_cached(Pfree, c1, 0, f);
+                g_last_hashed = g_force_hashed;
+                for (uint32_t f = 0; f < F; ++f) g_last_hashed |= st_step_range(P, f) != 0;
+                for (uint32_t i = 0; i < W; ++i) g_last_hashed |= st_ra_definition(P, i);
+                lane0_cached(S, hm_cache_k, g_last_hashed);
             } else {
                 tmask.ensure(wb8);
                 bind();
@@ -671,6 +682,7 @@ void ptlhm_set_scalar_serial(int on) { g_force_serial = on != 0; }
 
 void ptlhm_set_cache_entries(uint32_t k) { g_cache_k = k; }
 void ptlhm_set_ring_words(uint32_t k) { g_ring_k = k; }  // a power of two
+void ptlhm_set_general(int on) { g_force_general = on != 0; }
 void ptlhm_set_hashed(int on) { g_force_hashed = on != 0; }
 int ptlhm_last_hashed(void) { return g_last_hashed ? 1 : 0; }
 

@@ -1163,6 +1163,117 @@ __device__ bool ra_wait_chunk(const uint32_t* done, uint32_t c, uint32_t need, E
     }
 }
 
+// The lane-0 pass of a program with one lane-0 function (at most 8 functions) whose
+// registers are each defined once.  Every other function is in group 0, so no mark of an
+// earlier group exists (the check and the Jacobi rounds never act), no later group
+// triggers a position the slot reads (no swapped rewrites), and the slot wins every row-0
+// position it writes.  Lane 0 of warp 0 runs the slot; the warp turns each step's trigger
+// records into a 64-bit mask by ballot.  Row 0 stays in shared memory beside a mask of
+// the positions that hold virtual registers.  No block barrier: the other warps return.
+__device__ void ra_lane0_single(const Prog& P, uint32_t S, uint32_t K, uint32_t chunks, unsigned char* smem) {
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    constexpr unsigned full = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x;  // warp 0 only
+    const uint32_t* hist = P.ra_chunks;
+    const uint32_t* done = P.ra_chunks + chunks;
+    Ra2Shared& sh = *reinterpret_cast<Ra2Shared*>(smem);
+    uint32_t* cur = reinterpret_cast<uint32_t*>(smem + sizeof(Ra2Shared));
+    uint32_t* ctag = cur + 4u;
+    uint32_t* cval = ctag + K;
+    const SymCache c{ctag, cval, K};
+    uint32_t need = 0, wc = 0, waited = 0;  // lane 0: progress of the other functions
+    auto wait_for = [&](uint32_t chunk) -> int {
+        while (wc < chunk) need -= hist[wc++];
+        waited = chunk + 1;
+        return ra_wait_chunk(done, chunk, need, P.err) ? 0 : 1;
+    };
+    int abort = 0;
+    Ra2Slot L;
+    L.act = false;
+    L.have_next = false;
+    uint32_t s0 = 0;
+    if (lane == 0) {
+        for (uint32_t x = 0; x < chunks; ++x) need += hist[x];
+        if (chunks > 0 && S > 0) abort = wait_for(0);
+        ra2_slot_init(P, c, L, 0, 0);
+        s0 = min(ra2_lane0_size(L), S);
+    }
+    sh.R0[lane] = sh.R0[lane + 32] = kNone;
+    sh.R0own[lane] = sh.R0own[lane + 32] = kNone;
+    s0 = __shfl_sync(full, s0, 0);
+    if (__shfl_sync(full, abort, 0)) return;
+    unsigned long long occ = 0;  // lane 0: positions whose row-0 entry is a virtual register
+    uint32_t t0 = 0, t1 = 0;     // this step's records at positions lane and lane + 32
+    if (s0 > 0) {
+        t0 = __ldcg(&P.trig_max[lane]);
+        t1 = __ldcg(&P.trig_max[32u + lane]);
+    }
+    __syncwarp();
+    for (uint32_t i = 0; i < s0; ++i) {
+        if (chunks > 0 && i + 2 < S && (i + 2) % kRaChunk == 0) {
+            int ab = 0;
+            if (lane == 0) ab = wait_for((i + 2) / kRaChunk);
+            if (__shfl_sync(full, ab, 0)) return;
+        }
+        const unsigned long long others = static_cast<unsigned long long>(__ballot_sync(full, t0 != 0)) |
+                                          (static_cast<unsigned long long>(__ballot_sync(full, t1 != 0)) << 32);
+        if (i + 1 < S) {  // records of the next step (its chunk is complete: waited above)
+            t0 = __ldcg(&P.trig_max[static_cast<size_t>(i + 1) * 64u + lane]);
+            t1 = __ldcg(&P.trig_max[static_cast<size_t>(i + 1) * 64u + 32u + lane]);
+        }
+        if (lane == 0) {
+            ra2_load(P, L, i, cur);
+            RaStep& St = L.S;
+            unsigned long long marks = others & occ;
+            if (L.act) {
+                uint32_t r1reg = 0, r2reg = 0;
+                bool r1s = false, r2s = false;
+                if (s32(St.r1) > 63) sym_read(P, c, 0, St.r1, &r1reg, &r1s);
+                if (s32(St.r2) > 63) sym_read(P, c, 0, St.r2, &r2reg, &r2s);
+                ra_compute(St, L.lifetime, r1reg, r1s, r2reg, r2s);
+                L.lt_new = St.cleared | St.rdm;
+                if (s32(St.ord) > 63) sym_write(P, c, 0, St.ord, St.rdr, false, (St.rdr & 63u) + 1u);
+                if (s32(St.r1) > 63) sym_write(P, c, 0, St.r1, St.r1r, false);
+                if (s32(St.r2) > 63) sym_write(P, c, 0, St.r2, St.r2r, false);
+                marks = (others | St.trig) & occ;
+            }
+            // marks on the symbols row 0 held at the step's start, unless the slot updated them
+            for (unsigned long long m = marks; m; m &= m - 1) {
+                const uint32_t v = sh.R0[ctz64(m)];
+                const bool updated = L.act && ((s32(St.ord) > 63 && St.ord == v) || (s32(St.r1) > 63 && St.r1 == v) ||
+                                               (s32(St.r2) > 63 && St.r2 == v));
+                if (!updated) sym_mark(P, c, 0, v);
+            }
+            // row 0: the defined register at its position, cleared entries at rs1 / rs2
+            if (L.act) {
+                if (St.ord != 0) {
+                    const uint32_t q = St.rdr & 63u;
+                    sh.R0[q] = St.ord;
+                    sh.R0own[q] = 0;
+                    occ = s32(St.ord - 64u) >= 0 ? (occ | (1ull << q)) : (occ & ~(1ull << q));
+                }
+                for (const uint32_t r : {St.r1r, St.r2r}) {
+                    if (r != St.rdr && s32(r) >= 0 && r < 64u) {
+                        sh.R0[r] = kNone;
+                        sh.R0own[r] = 0;
+                        occ &= ~(1ull << r);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+    if (s0 >= S) return;
+    // the steps after the slot's last one only mark row 0's symbols
+    int ab = 0;
+    if (lane == 0)
+        for (uint32_t x = waited; x < chunks && !ab; ++x) ab = wait_for(x);
+    if (__shfl_sync(full, ab, 0)) return;
+    __syncwarp();
+    ra2_tail_p(P, c, sh, lane, s0, S);
+    ra2_tail_p(P, c, sh, lane + 32u, s0, S);
+}
+
 // Register allocation steps in one launch.  Block 0 runs the lane-0 functions (f % 8 ==
 // 0) in lock-step; thread t runs slots t, t+T, ... (Q per thread), slot = group index.
 // Blocks 1.. run the independent functions, one per thread, and count finished chunks
@@ -1182,6 +1293,10 @@ __device__ bool ra_wait_chunk(const uint32_t* done, uint32_t c, uint32_t need, E
 // function in smem.  With chunks > 0 it waits on the independent functions' progress.
 template <int Q>
 __device__ void ra_lane0_block(const Prog& P, uint32_t S, uint32_t K, uint32_t chunks, unsigned char* smem) {
+    if (P.F <= 8u && P.defpos) {  // one lane-0 function: warp 0 alone, no block barriers
+        if (threadIdx.x < 32) ra_lane0_single(P, S, K, chunks, smem);
+        return;
+    }
     const uint32_t tid = threadIdx.x, T = blockDim.x;
     __shared__ uint32_t s_abort, s_s0;
     const uint32_t* hist = P.ra_chunks;
@@ -1192,6 +1307,7 @@ __device__ void ra_lane0_block(const Prog& P, uint32_t S, uint32_t K, uint32_t c
     uint32_t* ctag = cur + 4u * G0;
     uint32_t* cval = ctag + G0 * K;
     const SymCache c{ctag, cval, K};
+    const bool hashed = P.defpos == nullptr;
     // Row-0 phases: thread tid handles physical registers tid, tid + T, ... (two each in a
     // one-warp block, which small programs get: its barriers cost next to nothing).
     constexpr uint32_t kRow = 64;
@@ -1238,7 +1354,7 @@ __device__ void ra_lane0_block(const Prog& P, uint32_t S, uint32_t K, uint32_t c
         for (uint32_t r = 0; r < 2; ++r) {  // T >= 32: at most two positions per thread
             const uint32_t p = tid + r * T;
             if (p >= kRow) continue;
-            ra2_begin_p(sh, 0, p, __ldcg(&P.trig_min[p]), __ldcg(&P.trig_max[p]));
+            ra2_begin_p(sh, 0, p, __ldcg(&P.trig_min[p]), __ldcg(&P.trig_max[p]), hashed);
             if (S > 1) { tmin[r] = __ldcg(&P.trig_min[kRow + p]); tmax[r] = __ldcg(&P.trig_max[kRow + p]); }
         }
     }
@@ -1275,7 +1391,8 @@ __device__ void ra_lane0_block(const Prog& P, uint32_t S, uint32_t K, uint32_t c
             const uint32_t j = tid + static_cast<uint32_t>(q) * T;
             if (j < G0) ra2_apply(P, c, sh, L[q], j, i, cur + 4u * j);
         }
-        for (uint32_t p = tid; p < kRow; p += T) snap_clear_next(sh, i, p);
+        if (hashed)
+            for (uint32_t p = tid; p < kRow; p += T) snap_clear_next(sh, i, p);
         if (__syncthreads_or(flag)) {
             for (uint32_t p = tid; p < kRow; p += T) sh.r0grp[p] = 0;
             for (uint32_t round = 0;; ++round) {
@@ -1306,7 +1423,7 @@ __device__ void ra_lane0_block(const Prog& P, uint32_t S, uint32_t K, uint32_t c
             if (p < kRow) {
                 ra2_end_p(P, c, sh, p, cur);
                 if (i + 1 < S) {
-                    ra2_begin_p(sh, i + 1, p, tmin[r], tmax[r]);
+                    ra2_begin_p(sh, i + 1, p, tmin[r], tmax[r], hashed);
                     if (i + 2 < S) {
                         tmin[r] = __ldcg(&P.trig_min[static_cast<size_t>(i + 2) * kRow + p]);
                         tmax[r] = __ldcg(&P.trig_max[static_cast<size_t>(i + 2) * kRow + p]);
@@ -1333,8 +1450,11 @@ __global__ void __launch_bounds__(1024) k_ra_steps(Prog P, uint32_t S, uint32_t 
     if (blockIdx.x > 0) {
         uint32_t* tag = reinterpret_cast<uint32_t*>(smem);
         const SymCache cf{tag, tag + T * Kf, Kf};
+        // the independent functions never need definition positions
+        Prog Pf = P;
+        Pf.defpos = nullptr;
         const uint32_t f = free_function_of((blockIdx.x - 1u) * T + tid);
-        if (f < P.F) ra_free_function_cached(P, cf, tid, f, P.ra_chunks + chunks);
+        if (f < P.F) ra_free_function_cached(Pf, cf, tid, f, P.ra_chunks + chunks);
         return;
     }
     ra_lane0_block<Q>(P, S, K, chunks, smem);
@@ -1398,12 +1518,14 @@ __device__ bool c_compute0(const Prog& P, const SymCache& c, const Ra2Shared& lo
     L.r1stored = L.r2stored = false;
     L.m1 = L.m2 = 0;
     if (s32(S.r1) > 63) {
-        sym_read(P, c, slot, S.r1, &L.r1reg, &L.r1stored);
-        L.m1 = snap_positions(loc, i, S.r1);
+        uint32_t d;
+        sym_read(P, c, slot, S.r1, &L.r1reg, &L.r1stored, &d);
+        L.m1 = snap_positions(P, loc, i, S.r1, d);
     }
     if (s32(S.r2) > 63) {
-        sym_read(P, c, slot, S.r2, &L.r2reg, &L.r2stored);
-        L.m2 = snap_positions(loc, i, S.r2);
+        uint32_t d;
+        sym_read(P, c, slot, S.r2, &L.r2reg, &L.r2stored, &d);
+        L.m2 = snap_positions(P, loc, i, S.r2, d);
     }
     L.r1m = c_marked_before(loc, ag, L.m1, L.j, false);
     L.r2m = c_marked_before(loc, ag, L.m2, L.j, false);
@@ -1446,10 +1568,10 @@ __device__ void c_apply(const Prog& P, const SymCache& c, const Ra2Shared& loc, 
         }
         return false;
     };
-    const bool l_ord = s32(S.ord) > 63 && later(snap_positions(loc, i, S.ord));
+    const bool l_ord = !P.defpos && s32(S.ord) > 63 && later(snap_positions_hashed(loc, i, S.ord));
     const bool l_r1 = s32(S.r1) > 63 && later(L.m1);
     const bool l_r2 = s32(S.r2) > 63 && later(L.m2);
-    if (s32(S.ord) > 63) sym_write(P, c, slot, S.ord, S.rdr, false);
+    if (s32(S.ord) > 63) sym_write(P, c, slot, S.ord, S.rdr, false, (S.rdr & 63u) + 1u);
     if (s32(S.r1) > 63) sym_write(P, c, slot, S.r1, S.r1r, false);
     if (s32(S.r2) > 63) sym_write(P, c, slot, S.r2, S.r2r, false);
     const bool r2v = s32(S.r2) > 63, r1v = s32(S.r1) > 63;
@@ -1503,6 +1625,7 @@ __global__ void __launch_bounds__(kRaClusterThreads, 1)
     uint32_t* cval = ctag + per_cta * K;
     const SymCache c{ctag, cval, K};  // this CTA's slots, by local index
     const bool row = tid < 64u;       // the CTA's row-0 threads (T >= 64)
+    const bool hashed = P.defpos == nullptr;
     if (tid == 0) {
         s_s0 = 0;
         s_or[0] = s_or[1] = s_or[2] = 0;
@@ -1553,7 +1676,7 @@ __global__ void __launch_bounds__(kRaClusterThreads, 1)
     __syncthreads();
     uint32_t tmin = 0xFFFFFFFFu, tmax = 0;  // a row-0 thread's trigger records, one step ahead
     if (row && S > 0) {
-        ra2_begin_p(loc, 0, tid, __ldcg(&P.trig_min[tid]), __ldcg(&P.trig_max[tid]));
+        ra2_begin_p(loc, 0, tid, __ldcg(&P.trig_min[tid]), __ldcg(&P.trig_max[tid]), hashed);
         if (S > 1) {
             tmin = __ldcg(&P.trig_min[64u + tid]);
             tmax = __ldcg(&P.trig_max[64u + tid]);
@@ -1588,7 +1711,7 @@ __global__ void __launch_bounds__(kRaClusterThreads, 1)
                 c_apply(P, c, loc, a, L[q], l, i, curp + 4u * l);
             }
         }
-        if (row) snap_clear_next(loc, i, tid);
+        if (hashed && row) snap_clear_next(loc, i, tid);
         if (cluster_or(flag)) {
             if (rank == 0 && row) a.r0grp[tid] = 0;
             for (uint32_t round = 0;; ++round) {
@@ -1615,7 +1738,7 @@ __global__ void __launch_bounds__(kRaClusterThreads, 1)
         if (row) {
             c_end_p(P, c, loc, a, tid, rank, per_cta, curp);
             if (i + 1 < S) {
-                ra2_begin_p(loc, i + 1, tid, tmin, tmax);
+                ra2_begin_p(loc, i + 1, tid, tmin, tmax, hashed);
                 if (i + 2 < S) {
                     tmin = __ldcg(&P.trig_min[static_cast<size_t>(i + 2) * 64u + tid]);
                     tmax = __ldcg(&P.trig_max[static_cast<size_t>(i + 2) * 64u + tid]);
@@ -1838,6 +1961,14 @@ struct SRaCountLoad {
 
 uint64_t launch_count() { return g_launches.load(); }
 void note_launch() { g_launches++; }
+
+__global__ void k_ra_definitions(Prog P) {
+    bool any = false;
+    uint32_t hint = 0xFFFFFFFFu;
+    PTL_FOR(i, P.W) any |= st_ra_definition(P, i, &hint);
+    PTL_FOR(f, P.F) any |= st_step_range(P, f) != 0;
+    if (__syncthreads_or(any) && threadIdx.x == 0) P.flags[2] = 1;
+}
 
 // ====================================================================== launchers
 cudaError_t launch_zero(const ZeroList& z, cudaStream_t s) {
@@ -2205,13 +2336,28 @@ cudaError_t ra_form(const Prog& P, cudaStream_t s, bool general, RaForm* form, u
     return cudaSuccess;
 }
 
+bool ra_positions_pay(uint32_t G0) { return G0 <= kRaClusterMin || ra_cluster_fits(G0); }
+
+cudaError_t ra_positions_tell(const Prog& P, cudaStream_t s, bool* tell) {
+    cudaMemsetAsync(P.flags + 2, 0, sizeof(uint32_t), s);
+    g_launches++;
+    k_ra_definitions<<<grid_for(P.W), kThreads, 0, s>>>(P);
+    uint32_t more = 0;
+    cudaMemcpyAsync(&more, P.flags + 2, sizeof(more), cudaMemcpyDeviceToHost, s);
+    const cudaError_t e = cudaStreamSynchronize(s);
+    *tell = more == 0;
+    return e;
+}
+
 cudaError_t run_regalloc_steps(const Prog& P, RaForm form, const ChunkBatch* chunks, cudaStream_t s) {
     cudaError_t ce = cudaSuccess;
     if (form == RaForm::Serial) {
         g_launches++;
         k_ra_serial<<<1, 1, 0, s>>>(P);
     } else if (form == RaForm::General) {
-        ce = launch_ra_steps(P, P, (P.F + 7u) / 8u, s);
+        Prog Pfree = P;
+        Pfree.defpos = nullptr;  // the independent functions never need definition positions
+        ce = launch_ra_steps(P, Pfree, (P.F + 7u) / 8u, s);
     } else {
         ce = run_step_regalloc(P, chunks, s);
     }
@@ -2511,6 +2657,16 @@ struct BScalarRecords {
         if (r & 2u) P.flags[2] = 1u;
     }
 };
+struct BDefinitions {
+    static constexpr bool kViewInShared = true;
+    uint32_t hint = 0xFFFFFFFFu, hp = 0xFFFFFFFFu;
+    __device__ static uint32_t count(const Prog& P) { return P.W; }
+    __device__ void operator()(const Prog& P, uint32_t i, uint32_t p) {
+        if (p != hp) { hp = p; hint = 0xFFFFFFFFu; }
+        if (st_ra_definition(P, i, &hint)) P.flags[2] = 1u;
+    }
+};
+PTL_BATCH_OP(BRanges, P.F, if (st_step_range(P, i)) P.flags[2] = 1u)
 PTL_BATCH_OP(BScalarRange, P.F, if (st_scalar_range(P, i)) P.flags[2] = 1u)
 
 // per program: word count and longest function (meta[4p + 1], meta[4p + 2])
@@ -2863,7 +3019,8 @@ __global__ void __launch_bounds__(MAXT) k_batch_ra(BatchRa ra) {
         const uint32_t local = item - ra.item_off[pos];
         const uint32_t free_tiles = ra.item_off[pos + 1] - ra.item_off[pos] - 1u;
         if (local < free_tiles) {
-            const Prog Pf = ra.progs[p];
+            Prog Pf = ra.progs[p];
+            Pf.defpos = nullptr;  // the independent functions never need definition positions
             uint32_t* tag = reinterpret_cast<uint32_t*>(smem);
             const SymCache cf{tag, tag + T * ra.Kf, ra.Kf};
             const uint32_t x = local * T + tid;
@@ -2984,6 +3141,8 @@ void batch_stage(BatchStage st, const BatchLaunch& bl, uint32_t total, uint32_t*
         case BatchStage::InitLifetime: batch_launch(bl, total, BInitLifetime{}); break;
         case BatchStage::ScalarRecords: batch_launch(bl, total, BScalarRecords{}); break;
         case BatchStage::ScalarRange: batch_launch(bl, total, BScalarRange{}); break;
+        case BatchStage::Definitions: batch_launch(bl, total, BDefinitions{}); break;
+        case BatchStage::Ranges: batch_launch(bl, total, BRanges{}); break;
         case BatchStage::Records: batch_launch(bl, total, BRecords{}); break;
         case BatchStage::RaHist: batch_launch(bl, total, BRaHist{}); break;
         case BatchStage::Spill: batch_launch(bl, total, BSpill{}); break;

@@ -84,12 +84,21 @@ cudaError_t run_optimize(const Prog& P, void* work, cudaStream_t s, uint32_t* sw
 // Register allocation of one program.  ra_form builds the step records (P.rec) and tells
 // which form the program takes; the caller then provides that form's arrays:
 //   Steps: tmask (one per word), trow and tany (row_tiles(S) tiles of kRowTile steps);
-//   General: trig_min / trig_max (set to none), ra_chunks;
+//   General: trig_min / trig_max (set to none), ra_chunks, and defpos (ra_positions_tell);
 //   Serial: none.
 struct ChunkBatch;
 enum class RaForm { Steps, General, Serial };
 // items: chunks of the lane-0 functions.
 cudaError_t ra_form(const Prog& P, cudaStream_t s, bool general, RaForm* form, uint32_t* items);
+// General form: whether definition positions (P.defpos, zeroed) tell where row 0 has a
+// symbol: no virtual register of a lane-0 function has two definitions, and no word is in
+// two functions.  P.stamp: zeroed.
+cudaError_t ra_positions_tell(const Prog& P, cudaStream_t s, bool* tell);
+// Where positions pay, measured through the general form, positions and hash, ms: one lane-0
+// function (which then has a form of its own) 132 and 364 with 111k nodes, 9 and 300 functions
+// 24.8 and 29.3, 15.6 and 18.1, 1,025 on a cluster 10.45 and 10.88; several groups a thread
+// of one block 3.95 and 3.80 (1,025 groups), 19.7 and 18.8 (4,125).
+bool ra_positions_pay(uint32_t G0);
 cudaError_t run_regalloc_steps(const Prog& P, RaForm form, const ChunkBatch* chunks, cudaStream_t s);
 
 // The lane-0 functions in chunks of steps (ptl_chunks.cuh): of one program (progs null),
@@ -177,7 +186,7 @@ cudaError_t batch_step_scalar(const StepBatch& b, cudaStream_t s);
 // Lane-0 passes too wide for one block: programs with more than kRaClusterMin lane-0
 // groups (at most 8,192) run theirs on a thread-block cluster when the device can place
 // it.  ra_cluster_fits tells whether it can; launch_ra_wide launches the program's
-// independent functions (Pfree), then the cluster pass (P0),
+// independent functions (Pfree: no definition positions), then the cluster pass (P0),
 // and sets *launched, or launches nothing.
 constexpr uint32_t kRaClusterMin = 1024;
 bool ra_cluster_fits(uint32_t G0);
@@ -239,7 +248,7 @@ struct BatchLaunch {
     uint32_t tile;
 };
 enum class BatchStage {
-    Ingest, Preprocess, Fix, Functab, Gen, OptMark, OptFinal, InitLifetime, Records, ScalarRecords, ScalarRange, RaHist, Spill,
+    Ingest, Preprocess, Fix, Functab, Gen, OptMark, OptFinal, InitLifetime, Records, ScalarRecords, ScalarRange, Definitions, Ranges, RaHist, Spill,
     Scatter, RaFunctab, FjEmit, FjFunctab,
     // the scalar generator's (ptl_scalar.cuh): preprocess, isn_gen, preserve counts
     // (per function), scatter (per word), the function table after regalloc (per

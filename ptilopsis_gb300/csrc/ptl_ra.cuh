@@ -25,28 +25,42 @@ PTL_HD void cache_reset(const SymCache& c, uint32_t slot) {
     for (uint32_t k = 0; k < c.K; ++k) c.tag[slot * c.K + k] = 0;
 }
 
-// Looks up v (> 63); returns physical register and swapped flag.
-PTL_HD void sym_read(const Prog& P, const SymCache& c, uint32_t slot, uint32_t v, uint32_t* reg, bool* swp) {
+// Looks up v (> 63); returns physical register, swapped flag and (through defp, when
+// given) the row-0 position + 1 of v's definition.
+PTL_HD void sym_read(const Prog& P, const SymCache& c, uint32_t slot, uint32_t v, uint32_t* reg, bool* swp,
+                     uint32_t* defp = nullptr) {
     const uint32_t e = slot * c.K + ((v - 64u) & (c.K - 1u));
     uint32_t x;
     if (c.tag[e] == v) {
         x = c.val[e];
     } else {
-        x = (P.symreg[v - 64u] & 0xFFu) | (P.symswp[v - 64u] != 0 ? 0x100u : 0u);
+        x = (P.symreg[v - 64u] & 0xFFu) | (P.symswp[v - 64u] != 0 ? 0x100u : 0u) |
+            (P.defpos ? static_cast<uint32_t>(P.defpos[v - 64u]) << 16 : 0u);
         c.tag[e] = v;
         c.val[e] = x;
     }
     *reg = x & 0xFFu;
     *swp = ((x >> 8) & 1u) != 0;
+    if (defp) *defp = x >> 16;
 }
 
-// Owner update of v.
-PTL_HD void sym_write(const Prog& P, const SymCache& c, uint32_t slot, uint32_t v, uint32_t reg, bool swp) {
+// Owner update of v.  defp = row-0 position + 1 of a definition, 0 for a use (kept).
+PTL_HD void sym_write(const Prog& P, const SymCache& c, uint32_t slot, uint32_t v, uint32_t reg, bool swp,
+                      uint32_t defp = 0) {
     P.symreg[v - 64u] = reg;
     P.symswp[v - 64u] = swp ? 0xFFFFFFFFu : 0u;
     const uint32_t e = slot * c.K + ((v - 64u) & (c.K - 1u));
+    uint32_t keep = 0;
+    if (defp) {
+        if (P.defpos) P.defpos[v - 64u] = static_cast<uint8_t>(defp);
+        keep = defp << 16;
+    } else if (c.tag[e] == v) {
+        keep = c.val[e] & 0xFFFF0000u;
+    } else if (P.defpos) {
+        keep = static_cast<uint32_t>(P.defpos[v - 64u]) << 16;
+    }
     c.tag[e] = v;
-    c.val[e] = (reg & 0xFFu) | (swp ? 0x100u : 0u);
+    c.val[e] = (reg & 0xFFu) | (swp ? 0x100u : 0u) | keep;
 }
 
 // A swap mark: global memory, plus the owner's cached copy if it holds v.
@@ -152,7 +166,7 @@ struct Ra2Slot {
 PTL_HD uint32_t snap_hash(uint32_t v) { return (v * 2654435761u) >> 25; }
 
 // Row-0 positions holding v at the start of step i (v > 63), from the hash of row 0.
-PTL_HD uint64_t snap_positions(const Ra2Shared& sh, uint32_t i, uint32_t v) {
+PTL_HD uint64_t snap_positions_hashed(const Ra2Shared& sh, uint32_t i, uint32_t v) {
     const uint32_t t = i & 1u;
     uint32_t h = snap_hash(v);
     for (uint32_t probe = 0; probe < kSnapHash; ++probe) {
@@ -195,6 +209,15 @@ PTL_HD void snap_clear_next(Ra2Shared& sh, uint32_t i, uint32_t p) {
     }
 }
 
+// Row-0 positions holding v: a lane-0 value enters row 0 only where its definition put
+// it, so one compare answers the question -- unless two instructions define the same
+// virtual register, for which the row-0 hash is built instead (P.defpos == null).
+PTL_HD uint64_t snap_positions(const Prog& P, const Ra2Shared& sh, uint32_t i, uint32_t v, uint32_t d) {
+    if (!P.defpos) return snap_positions_hashed(sh, i, v);
+    if (d == 0) return 0;
+    return sh.snap[d - 1u] == v ? (1ull << (d - 1u)) : 0ull;
+}
+
 // Whether a symbol at row-0 positions m is marked by a group before j (g1 <= j).
 PTL_HD bool marked_before(const Ra2Shared& sh, uint64_t m, uint32_t j, bool with_lane0) {
     for (; m; m &= m - 1) {
@@ -217,10 +240,10 @@ PTL_HD void ra2_slot_init(const Prog& P, const SymCache& c, Ra2Slot& L, uint32_t
 
 // Step start for row-0 position p (64 threads); tmin/tmax are the step's trigger
 // records of the other functions (loaded a step ahead).
-PTL_HD void ra2_begin_p(Ra2Shared& sh, uint32_t i, uint32_t p, uint32_t tmin, uint32_t tmax) {
+PTL_HD void ra2_begin_p(Ra2Shared& sh, uint32_t i, uint32_t p, uint32_t tmin, uint32_t tmax, bool hashed) {
     sh.snap[p] = sh.R0[p];
     sh.snapown[p] = sh.R0own[p];
-    if (s32(sh.R0[p] - 64u) >= 0) snap_insert(sh, i, sh.R0[p], p);
+    if (hashed && s32(sh.R0[p] - 64u) >= 0) snap_insert(sh, i, sh.R0[p], p);
     sh.omin[p] = tmin;
     sh.omax[p] = tmax;
     sh.lcur[p] = 0xFFFFFFFFu;
@@ -273,12 +296,14 @@ PTL_HD bool ra2_compute0(const Prog& P, const SymCache& c, Ra2Shared& sh, Ra2Slo
     L.r1stored = L.r2stored = false;
     L.m1 = L.m2 = 0;
     if (s32(S.r1) > 63) {
-        sym_read(P, c, slot, S.r1, &L.r1reg, &L.r1stored);
-        L.m1 = snap_positions(sh, i, S.r1);
+        uint32_t d;
+        sym_read(P, c, slot, S.r1, &L.r1reg, &L.r1stored, &d);
+        L.m1 = snap_positions(P, sh, i, S.r1, d);
     }
     if (s32(S.r2) > 63) {
-        sym_read(P, c, slot, S.r2, &L.r2reg, &L.r2stored);
-        L.m2 = snap_positions(sh, i, S.r2);
+        uint32_t d;
+        sym_read(P, c, slot, S.r2, &L.r2reg, &L.r2stored, &d);
+        L.m2 = snap_positions(P, sh, i, S.r2, d);
     }
     L.r1m = marked_before(sh, L.m1, L.j, false);
     L.r2m = marked_before(sh, L.m2, L.j, false);
@@ -336,14 +361,14 @@ PTL_HD void ra2_apply(const Prog& P, const SymCache& c, Ra2Shared& sh, Ra2Slot& 
         return false;
     };
     // The swap flags need the row-0 positions at the step start: m1/m2 from the round-0
-    // lookups.  The defined register sits in row 0 before its definition when it has
-    // two definitions.
-    const bool l_ord = s32(S.ord) > 63 && later(snap_positions(sh, i, S.ord));
+    // lookups.  The defined register sits in row 0 before its definition only when it
+    // has two definitions, i.e. in hashed mode.
+    const bool l_ord = !P.defpos && s32(S.ord) > 63 && later(snap_positions_hashed(sh, i, S.ord));
     const bool l_r1 = s32(S.r1) > 63 && later(L.m1);
     const bool l_r2 = s32(S.r2) > 63 && later(L.m2);
     // the reference's order: rd, rs1, rs2 (a later write of the same symbol wins); a
     // definition records the row-0 position it writes (when it writes row 0 at all)
-    if (s32(S.ord) > 63) sym_write(P, c, slot, S.ord, S.rdr, false);
+    if (s32(S.ord) > 63) sym_write(P, c, slot, S.ord, S.rdr, false, (S.rdr & 63u) + 1u);
     if (s32(S.r1) > 63) sym_write(P, c, slot, S.r1, S.r1r, false);
     if (s32(S.r2) > 63) sym_write(P, c, slot, S.r2, S.r2r, false);
     // a swapped symbol keeps the register just written for it (the last of the three

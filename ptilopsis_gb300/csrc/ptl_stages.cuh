@@ -200,7 +200,8 @@ struct Prog {
     uint32_t* trow;       // [S in whole tiles][kRowPos] trigger rows
     uint32_t* tany;       // [S in whole tiles] positions triggered at all
     LaneChunks ch;
-    uint32_t* stamp;      // definitions per virtual register (regalloc cross check)
+    uint32_t* stamp;      // general form: definitions per virtual register; serial form: its scratch
+    uint8_t* defpos;      // general form: row-0 position + 1 of each lane-0 definition; null: use the row-0 hash
     unsigned long long* lifetime;
     uint32_t* trig_min;   // [S][64] min group+1 of non-lane-0 triggers, 0xFFFFFFFF = none
     uint32_t* trig_max;   // [S][64] max group+1, 0 = none
@@ -842,6 +843,20 @@ PTL_HD uint32_t function_of(const Prog& P, uint32_t i, uint32_t hint = 0xFFFFFFF
         if (P.fn_start0[mid] <= i) lo = mid; else hi = mid;
     }
     return lo;
+}
+
+// Counts word i's definition of a virtual register by a lane-0 function; whether the
+// register has another one (the general form then looks row 0 up by hash).
+PTL_HD bool st_ra_definition(const Prog& P, uint32_t i, uint32_t* hint = nullptr) {
+    const uint32_t lo = function_of(P, i, hint ? *hint : 0xFFFFFFFFu);
+    if (hint) *hint = lo;
+    const uint32_t rd = P.rd[i];
+    if ((lo & 7u) != 0 || !(s32(rd) > 63) || rd - 64u >= P.W) return false;
+#if defined(__CUDA_ARCH__)
+    return atomicAdd(&P.stamp[rd - 64u], 1u) != 0;
+#else
+    return P.stamp[rd - 64u]++ != 0;
+#endif
 }
 
 // The reference's step loop as written (rv_generator_avx.cpp:1400-1413 with one worker):

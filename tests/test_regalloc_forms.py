@@ -222,3 +222,38 @@ def test_gpu_chunk_wait_gives_up(built_cuda):
         b.compile(trees)
         for k, want in enumerate(refs):
             np.testing.assert_array_equal(b.words(k), want, err_msg=str(k))
+
+
+@pytest.mark.parametrize("hashed", [0, 1])
+@pytest.mark.parametrize("entries", [1, 64])
+@pytest.mark.parametrize("n_functions", [1, 9, 130])
+def test_hostmodel_general_form(built, n_functions, entries, hashed):
+    """The general form, which the programs of the front end take no more: row 0 by
+    definition positions where every register has one definition, and by hash, with a symbol
+    cache of one entry and of many."""
+    from test_hostmodel import assert_stages_equal, hostmodel
+    L = hostmodel()
+    L.ptlhm_set_general(1)
+    L.ptlhm_set_hashed(hashed)
+    L.ptlhm_set_cache_entries(ctypes.c_uint32(entries))
+    try:
+        assert_stages_equal(tree_to_ast(_program(n_functions, 200.0, max_expr_depth=12, float_frac=0.5)))
+        assert L.ptlhm_last_hashed() == hashed
+    finally:
+        L.ptlhm_set_general(0)
+        L.ptlhm_set_hashed(0)
+        L.ptlhm_set_cache_entries(ctypes.c_uint32(4))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_functions", [1, 8, 9, 300, 2100])
+def test_gpu_general_form(built_cuda, n_functions):
+    """By definition positions (with up to 8 functions one warp does it alone) and by hash."""
+    from oracle import portbind
+    from ptilopsis_gb300 import RvGenerator
+    tree = _program(n_functions, 200.0, max_expr_depth=12, float_frac=0.5)
+    want = portbind.compile_ast(tree_to_ast(tree)).words
+    with RvGenerator(tree) as gen:
+        for how in ({"general": True}, {"row0_hash": True}, {"general": True}):
+            gen.process(**how)
+            np.testing.assert_array_equal(gen.get_instructions(), want)
