@@ -127,7 +127,9 @@ struct ChunkBatch {
 };
 // Steps from which on chunks pay.  Their passes and rounds have a cost of their own, about
 // 0.12 ms: with 403 steps (one function) the allocation took 0.36 ms in lock-step and 0.45
-// in chunks, with 1,449 (two functions) 1.46 and 0.65.
+// in chunks, with 1,449 (two functions) 1.46 and 0.65.  At other widths, lock-step below and
+// chunks above the line, ms: 8 lane-0 functions of 605 steps 0.75, of 1,093 0.91; 64 of 614
+// 1.03, of 1,176 1.46; 512 of 591 2.76, of 1,210 2.88; 1,024 of 613 3.85, of 1,175 4.54.
 constexpr uint32_t kChunkMinSteps = 768;
 // Lane-0 functions up to which one warp, and four, fold a chunk's rows (else a block).
 constexpr uint32_t kChunkNarrow = 16, kChunkWide = 128;
@@ -139,12 +141,18 @@ inline uint32_t chunk_class(uint32_t G0) { return G0 <= 1u ? 1u : (G0 <= kChunkN
 // 15,000, with more than kChunkNarrow functions (which run again more often, and have folds)
 // four times as much.  64 programs of up to 4,575 steps took 3.0 to 4.3 ms in lock-step and
 // 2.0 to 2.6 in chunks, 512 of up to 4,058 steps and 64 functions 8.4 and 18.5.
+//
+// The rule counts all SMs also for a batch held to a share of them.  At half of them that is
+// right for the few large programs of a compile server's lane (16 of 100k to 2M nodes 7.1 ms
+// in chunks, 13.0 in lock-step) and wrong for many middling ones (128 of 70k nodes 9.7 and
+// 7.4); with the waves of the share the first would go the wrong way.
 inline uint64_t lock_step_cycles(uint64_t S, uint32_t G0) { return S * (G0 <= 1u ? 1000u : (G0 <= 32u ? 1450u : 2350u)); }
 inline uint64_t chunk_work(uint64_t tiles, uint32_t G0) { return tiles * ((G0 + 31u) / 32u) * (G0 <= kChunkNarrow ? 1u : 4u); }
 inline bool chunk_pays(uint64_t tiles, uint64_t work, uint64_t before, uint64_t after) {
     return (tiles / 6u + 6u) * (20000u + 15000u * work / 2432u) + after < before;
 }
-// Rounds before the lock-step takes over: they have been a third of the chunks or less.
+// Rounds before the lock-step takes over: they have been 10 for 18 chunks, 30 for 148 and 100
+// for 175.
 inline uint32_t chunk_rounds(uint32_t tiles) { return tiles + 64u; }
 // Other limits of a generator or a batch (0: the above), so that tests see what comes after.
 struct ChunkLimits {
