@@ -27,6 +27,8 @@ namespace {
 
 bool g_last_locked = false;  // the last program's symbols did not fit the slots
 bool g_chunks = true;  // lane-0 functions in chunks (else in lock-step)
+uint32_t g_chunk_rounds = 0;  // rounds of the chunks at most (0: the kernel's limit)
+bool g_last_lock_step = false;  // the last program's lane-0 functions went in lock-step
 uint32_t g_ring_k = 16;  // words per function in the record form's symbol ring (small: old words too)
 uint32_t g_cache_k = 4;  // entries per function of the lane-0 symbol cache
 bool g_force_general = false; // the general form for every program
@@ -222,7 +224,7 @@ struct Model {
     // The lane-0 functions in chunks (ptl_chunks.cuh), round by round as its kernel runs
     // them (the runs of a round one after the other).  False: the rounds ran out.
     bool chunk_lanes(uint32_t S, uint32_t K) {
-        const uint32_t G0 = (P.F + 7) / 8, tiles = static_cast<uint32_t>(row_tiles(S)), rounds = tiles + 64;
+        const uint32_t G0 = (P.F + 7) / 8, tiles = static_cast<uint32_t>(row_tiles(S)), rounds = g_chunk_rounds ? g_chunk_rounds : tiles + 64;
         const size_t steps = static_cast<size_t>(tiles) * kRowTile;
         auto size = [&](uint32_t j) { return static_cast<uint32_t>(std::max(s32(P.fn_size0[8 * j]), 0)); };
         std::vector<uint32_t> off(G0 + 1);
@@ -321,7 +323,8 @@ struct Model {
                 }
             }
         }
-        if (g_chunks && chunk_lanes(S, K)) return;
+        g_last_lock_step = !(g_chunks && chunk_lanes(S, K));
+        if (!g_last_lock_step) return;
         LaneShared sh{};
         std::vector<uint8_t> rings(static_cast<size_t>(G0) * K);
         std::vector<LaneSlot> L(G0);
@@ -676,7 +679,9 @@ void ptlhm_chunks_lost(uint32_t n, uint32_t threads, uint32_t* codes) {
     for (uint32_t t = 0; t < threads; ++t) chunks_lost([&](uint32_t k) -> const Prog& { return progs[k]; }, n, t, threads, 3u);
     for (uint32_t k = 0; k < n; ++k) codes[k] = err[k].code;
 }
+int ptlhm_last_lock_step(void) { return g_last_lock_step ? 1 : 0; }
 void ptlhm_set_chunks(int on) { g_chunks = on != 0; }
+void ptlhm_set_chunk_rounds(uint32_t rounds) { g_chunk_rounds = rounds; }
 void ptlhm_set_scalar_tiles(int on) { g_force_tiles = on != 0; }
 void ptlhm_set_scalar_serial(int on) { g_force_serial = on != 0; }
 

@@ -257,3 +257,134 @@ def test_gpu_general_form(built_cuda, n_functions):
         for how in ({"general": True}, {"row0_hash": True}, {"general": True}):
             gen.process(**how)
             np.testing.assert_array_equal(gen.get_instructions(), want)
+
+
+# ---------------------------------------------------------------- the lane-0 lock-step
+def _steps(ref):
+    """Steps of the longest function, as the forms' rules count them."""
+    return int(ref.bufs["cnt_fn_size"].max())
+
+
+def _far_operand(tree, n):
+    """tree with one literal operand of an addition replaced by 1 + (((1 + 1) + 1) + ...), n
+    additions in the parentheses: the first operand is read some 3n words later (a literal is
+    two words), and few symbols are alive meanwhile."""
+    import dataclasses
+    ADD, LIT, INT = 13, 35, 2
+    t, rt, par = (np.asarray(getattr(tree, k)) for k in ("type", "rtype", "parent"))
+    leaf = [k for k in range(tree.n) if t[k] == LIT and rt[k] == INT and t[par[k]] == ADD][-1]
+    more = 2 * n + 2  # before the leaf, whose place is the outer addition's: 1, then 1, (1, +) n times
+    at = lambda k: k if k < leaf else k + more
+    cols = {k: np.asarray(getattr(tree, k)) for k in ("type", "rtype", "parent", "depth", "child_idx", "data")}
+    new = {k: np.insert(c, leaf, np.zeros(more, c.dtype)) for k, c in cols.items()}
+    new["parent"] = np.array([at(p) if p >= 0 else p for p in new["parent"]], cols["parent"].dtype)
+    d = int(cols["depth"][leaf])
+
+    def put(i, kind, parent, depth, child):
+        new["type"][i], new["rtype"][i], new["data"][i] = kind, INT, 1 if kind == LIT else 0
+        new["parent"][i], new["depth"][i], new["child_idx"][i] = parent, depth, child
+
+    outer = leaf + more
+    new["type"][outer], new["rtype"][outer], new["data"][outer] = ADD, INT, 0
+    put(leaf, LIT, outer, d + 1, 0)
+    add = lambda k: leaf + 3 + 2 * k  # addition k, the innermost 0
+    put(leaf + 1, LIT, add(0), d + n + 1, 0)
+    for k in range(n):
+        depth = d + n - k
+        put(add(k) - 1, LIT, add(k), depth + 1, 1)
+        put(add(k), ADD, add(k + 1) if k + 1 < n else outer, depth, 0 if k + 1 < n else 1)
+    return dataclasses.replace(tree, max_depth=int(new["depth"].max()), **new)
+
+
+@pytest.mark.parametrize("rounds", [0, 1, 2])
+@pytest.mark.parametrize("ring", [4, 16, 1024])
+@pytest.mark.parametrize("n_functions", [1, 9, 40, 300])
+def test_hostmodel_lock_step(built, n_functions, ring, rounds):
+    """The lock-step's step functions on the CPU, several slots among them, with operands older
+    than the ring: from the start, and after chunks whose rounds have run out."""
+    from test_hostmodel import assert_stages_equal, hostmodel
+    L = hostmodel()
+    L.ptlhm_set_ring_words(ctypes.c_uint32(ring))
+    L.ptlhm_set_chunks(1 if rounds else 0)
+    L.ptlhm_set_chunk_rounds(ctypes.c_uint32(rounds))
+    try:
+        assert_stages_equal(tree_to_ast(_program(n_functions, 300.0, max_expr_depth=12, float_frac=0.5)))
+        assert L.ptlhm_last_lock_step()
+    finally:
+        L.ptlhm_set_ring_words(ctypes.c_uint32(16))
+        L.ptlhm_set_chunks(1)
+        L.ptlhm_set_chunk_rounds(ctypes.c_uint32(0))
+
+
+@pytest.mark.parametrize("n", [2000, 3000, 6000])
+def test_hostmodel_far_operand(built, n):
+    """A symbol that lives through fewer chunks than a symbol may, and through more (the
+    lock-step then does the program)."""
+    from test_hostmodel import assert_stages_equal, hostmodel
+    tree = _far_operand(_program(1, 900.0, float_frac=0.0), n)
+    assert_stages_equal(tree_to_ast(tree))
+    assert bool(hostmodel().ptlhm_last_locked()) == (3 * n > 256 * 32)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_functions", [1, 9, 257, 2048, 2049, 4100, 8193])
+def test_gpu_lock_step_short(built_cuda, n_functions):
+    """Programs too short for chunks: one slot, one warp (2 slots), a block (33 and 256), a
+    cluster of two CTAs (257), of three (513) and of five (1,025)."""
+    from oracle import portbind
+    from ptilopsis_gb300 import RvGenerator
+    tree = _program(n_functions, 100.0, sigma=0.4)
+    ref = portbind.compile_ast(tree_to_ast(tree), snapshots=True)
+    assert _steps(ref) < 768
+    with RvGenerator(tree) as gen:
+        gen.process()
+        np.testing.assert_array_equal(gen.get_instructions(), ref.words)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rounds", [1, 2])
+@pytest.mark.parametrize("n_functions", [1, 9, 140, 2049, 8200])
+def test_gpu_lock_step_after_chunks(built_cuda, n_functions, rounds):
+    """Programs long enough for chunks whose rounds have run out: operands older than the
+    lock-step's ring, on one warp, a block and a cluster."""
+    from oracle import portbind
+    from ptilopsis_gb300 import RvGenerator
+    more = {"max_expr_depth": 12, "max_nesting": 64}
+    tree = _program(n_functions, 6000.0 if n_functions < 100 else 300.0, float_frac=0.3, **more)
+    ref = portbind.compile_ast(tree_to_ast(tree), snapshots=True)
+    assert _steps(ref) >= 768
+    with RvGenerator(tree) as gen:
+        gen.set_chunk_limits(rounds=rounds)
+        gen.process()
+        np.testing.assert_array_equal(gen.get_instructions(), ref.words)
+
+
+@pytest.mark.gpu
+def test_gpu_batch_lock_step_after_chunks(built_cuda):
+    """A batch whose chunks' rounds run out, settled programs among them, beside one in
+    lock-step from the start and one on a cluster; then with the built-in limit."""
+    from oracle import portbind
+    from ptilopsis_gb300.batch import BatchCompiler
+    trees = [_program(n, m, float_frac=0.3) for n, m in ((1, 1500.0), (9, 4000.0), (140, 900.0), (3, 40.0))]
+    trees += [_program(5, 3000.0, seed=0x50544DA0, max_expr_depth=12, float_frac=0.5, max_nesting=64)]
+    trees += [_program(8200, 60.0, sigma=1.5, max_fn_nodes=4000)]
+    refs = [portbind.compile_ast(tree_to_ast(t)).words for t in trees]
+    with BatchCompiler(tiles=None) as b:
+        for rounds in (1, 2, 0):
+            b.set_chunk_limits(rounds=rounds)
+            b.compile(trees)
+            for k, want in enumerate(refs):
+                np.testing.assert_array_equal(b.words(k), want, err_msg=f"{rounds} rounds, program {k}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2000, 6000])
+def test_gpu_far_operand(built_cuda, n):
+    """A symbol that lives through fewer chunks than a symbol may, and through more."""
+    from oracle import portbind
+    from ptilopsis_gb300 import RvGenerator
+    tree = _far_operand(_program(9, 900.0, float_frac=0.0), n)
+    ref = portbind.compile_ast(tree_to_ast(tree))
+    with RvGenerator(tree) as gen:
+        gen.process()
+        np.testing.assert_array_equal(gen.get_instructions(), ref.words)
