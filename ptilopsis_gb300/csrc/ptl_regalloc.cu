@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(32) k_step_free(Src src, uint32_t per_warp) {
 
 // ---- the scalar generator's functions: one thread each, one warp a block.  The warp form
 // (k_s_ra_warp: every lane runs the same function) took 790 cycles a step and a warp per
-// function; this one takes half as long and a lane.
+// function; this one takes 560 (a function a warp) to 720 (32 side by side) and a lane.
 constexpr uint32_t kScalarRing = 256, kScalarStride = 36;
 template <class Src>
 __global__ void __launch_bounds__(32) k_step_scalar(Src src, unsigned long long* preserve, uint32_t per_warp) {
